@@ -253,11 +253,11 @@ int gbfem_dg_set_faces(gbfem_ctx ctx, int nfa, const int *fa_type, const int *fa
  * accuracy; or GBFEM_DG_VOLUME_TF32, the tensor cores with TF32 hi/lo
  * operands and FP32 accumulation (about 1e-6 of the entry scale: an
  * approximate matrix, for comparison).  The tensor-core kernels cover
- * p = 1..3; p = 4 elements keep the FP64 kernel.  GBFEM_DG_VOLUME_DWORD:
- * the FP64 kernel's algebra with each stiffness entry summed in double-word
- * (float pair) arithmetic on the FP32 pipes (errors of order 2^-48 of the
- * summed magnitudes), all degrees; GBFEM_DG_VOLUME_TC_DWORD: split BF16 on
- * the tensor cores for p = 1..3 and the double-word kernel for p = 4. */
+ * p = 1..3; p = 4 elements keep the FP64 kernel.  GBFEM_DG_VOLUME_DWORD asks
+ * for entries within 2^-48 of the summed magnitudes: the FP64 kernel meets
+ * that and is the fastest that does, so it serves this choice;
+ * GBFEM_DG_VOLUME_TC_DWORD: split BF16 on the tensor cores for p = 1..3 and
+ * the FP64 kernel for p = 4. */
 #define GBFEM_DG_VOLUME_FP64 0
 #define GBFEM_DG_VOLUME_TC 1
 #define GBFEM_DG_VOLUME_TF32 2
@@ -302,8 +302,8 @@ int gbfem_dg_get_structure(gbfem_ctx ctx, int *dof_off, int *bptr, int *bcol, lo
  * and the rhs, each block entry written by one thread in a fixed order. */
 int gbfem_dg_assemble(gbfem_ctx ctx);
 /* Launch-shape autotuner (no reference counterpart): per degree class,
- * times the FP64 volume kernel's three shapes (threads per CTA, points per
- * shared-memory chunk) and the face kernel's two (threads per CTA) on up to
+ * times the FP64 volume kernel's three shapes (elements per CTA) and the face
+ * kernel's two (threads per CTA) on up to
  * `sample` elements (<= 0: 16384) of the current mesh and keeps the fastest
  * for later assemblies.  Every shape sums each matrix entry in the same
  * order, so the choice never changes the results.  Overwrites the matrix:
@@ -468,10 +468,9 @@ int gbfem_batch_set_layout(gbfem_batch batch, const long long *val_off, const in
  * elements per tile).  Either pointer may be NULL.  Every variant gives the
  * same bits. */
 int gbfem_batch_set_variants(gbfem_batch batch, const int *prism_v, const int *tet_v);
-/* Arithmetic of the prism stiffness sums: 0 FP64 (default), 1 double word
- * (float pairs on the FP32 pipes, exact products and TwoSum chains; entries
- * within about 2^-48 of the summed magnitudes).  Tetrahedra (6 FMAs per
- * entry against exact reference matrices) stay FP64. */
+/* Accuracy of the prism stiffness sums: 0 FP64 (default), 1 within about
+ * 2^-48 of the summed magnitudes.  The FP64 kernel is the fastest that meets
+ * either, and serves both. */
 int gbfem_batch_set_arith(gbfem_batch batch, int dword);
 /* Times every variant of every (type, degree) class present on up to
  * `sample` of its elements (<= 0: 16384), keeps the fastest.  prism_v[5],

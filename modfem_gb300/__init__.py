@@ -458,7 +458,7 @@ class Batch:
         self.nval, self.nrhs, self.layout = nval, nrhs, (vo, ro)
 
     def set_arith(self, dword):
-        """Prism stiffness sums in FP64 (False) or double-word arithmetic (True)."""
+        """Prism stiffness sums to FP64 (False) or double-word (True) accuracy; one FP64 kernel serves both."""
         self._check(self.L.gbfem_batch_set_arith(self._h, 1 if dword else 0))
 
     def set_variants(self, prism=None, tet=None):

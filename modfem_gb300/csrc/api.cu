@@ -1558,9 +1558,6 @@ int gbfem_dg_assemble(gbfem_ctx c) {
   // adds to those and writes every off-diagonal block: nothing to clear
   const bool tc = c->dg_volume_mode == GBFEM_DG_VOLUME_TC || c->dg_volume_mode == GBFEM_DG_VOLUME_TF32 ||
                   c->dg_volume_mode == GBFEM_DG_VOLUME_TC_DWORD;
-  // double-word stiffness sums: for every degree, or for those the tensor
-  // cores do not cover
-  const bool dwv = c->dg_volume_mode == GBFEM_DG_VOLUME_DWORD || c->dg_volume_mode == GBFEM_DG_VOLUME_TC_DWORD;
   if (tc) GB_CUDA(cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream));
   const bool tcf = c->dg_face_mode == GBFEM_DG_FACE_TC || c->dg_face_mode == GBFEM_DG_FACE_TC_DWORD;
   // Tensor-core faces beside a volume kernel on the CUDA cores (FP64 or
@@ -1624,7 +1621,7 @@ int gbfem_dg_assemble(gbfem_ctx c) {
       r = gbfem::launch_dg_prism_elements(c->stream, c->device, p, (int)c->dg_list[p].n, c->dg_list[p].p,
                                           c->el_nodes.p, c->xyz.p, c->k_el.p, c->D_el.p, c->f,
                                           c->dg_boff_diag_d.p, c->dg_roff_d.p, c->dg_val.p, c->dg_rhs.p,
-                                          c->dg_var_vol[p], dwv);
+                                          c->dg_var_vol[p]);
     GB_TRY(r);
     launches += r;
   }

@@ -31,30 +31,16 @@ __host__ __device__ constexpr int tet_ns(int p) { return (p + 1) * (p + 2) * (p 
 
 // Work: tiles of one (type, degree, launch variant) class, listed heaviest
 // class first; persistent CTAs (256 threads, as many as fit on the SMs) take
-// tiles from an atomic counter.  A prism tile holds 256 / THR elements, each
-// integrated by a group of THR threads exactly as the per-degree kernel does
-// (bit-identical for every variant); a tetrahedron tile holds `tile`
-// elements, threads over (element, block entry).  The variant of each class
-// (prism: threads per element, points per shared-memory chunk; tetrahedron:
-// elements per tile) is chosen by gbfem_batch_autotune.
+// tiles from an atomic counter.  A prism tile holds dg_vol_elems(p, variant)
+// elements, integrated exactly as the per-degree kernel does (bit-identical
+// for every variant); a tetrahedron tile holds `tile` elements, threads over
+// (element, block entry).  The variant of each class (elements per tile) is
+// chosen by gbfem_batch_autotune.
 
-constexpr int DGB_VARIANTS = 3;    // prism variants per degree
+constexpr int DGB_VARIANTS = DG_VOL_VARIANTS;  // prism variants per degree
+static_assert(DGB_THREADS == DG_VOL_THREADS, "the prism tiles run on the whole CTA");
 constexpr int DGB_TET_VARIANTS = 5;
-__host__ __device__ constexpr int dgb_prism_thr(int p, int v) {
-  return p == 1 ? (v == 0 ? 32 : v == 1 ? 64 : 128)
-       : p == 2 ? (v == 0 ? 64 : v == 1 ? 128 : 256)
-       : p == 3 ? (v == 2 ? 128 : 256)
-                : 256;
-}
-__host__ __device__ constexpr int dgb_prism_qc(int p, int v) {
-  return p == 3 ? (v == 1 ? 16 : 8) : p == 4 ? (v == 0 ? 8 : v == 1 ? 16 : 4) : 8;
-}
 __host__ __device__ constexpr int dgb_tet_tile(int v) { return 8 << v; }  // 8 .. 128
-// shared doubles of one prism group
-__host__ __device__ constexpr int dgb_prism_group_smem(int p, int v) {
-  return 32 + 7 * (p == 1 ? 6 : p == 2 ? 18 : p == 3 ? 48 : 80) +
-         dgb_prism_qc(p, v) * 3 * (p == 1 ? 6 : p == 2 ? 18 : p == 3 ? 40 : 75);
-}
 
 struct DgBatchTile {
   unsigned char type;  // 0 prism, 1 tetrahedron
@@ -67,8 +53,8 @@ struct DgBatchTile {
 };
 
 struct DgBatchTables {
-  const double *D[GB_DG_PMAX + 1], *PHI[GB_DG_PMAX + 1], *QP[GB_DG_PMAX + 1];  // prisms
-  const float2 *Ddw[GB_DG_PMAX + 1];  // prisms, D as double words
+  const double *QP[GB_DG_PMAX + 1], *VT[GB_DG_PMAX + 1];  // prisms (dg_volume.cuh)
+  const DgVolEntry *ENT[GB_DG_PMAX + 1];
   const double *T[GB_DG_PMAX + 1];    // tets: 6 x (ns(ns+1)/2) packed upper entries
   const double *MOM[GB_DG_PMAX + 1];  // tets: int_ref phi_i
 };
@@ -81,29 +67,15 @@ struct DgBatchArgs {
   const int *proff, *troff;         // rhs offset
   double *val, *rhs;
   double f;
-  int dword;  // prism stiffness sums in double-word arithmetic
 };
 
-template <int P, int THR, int QC>
+template <int P>
 __device__ void dgb_prism(const DgBatchTables &tb, const DgBatchArgs &a, const DgBatchTile &T, double *smem) {
-  using Dm = DgDims<P, THR, QC>;
-  constexpr int GROUP = 32 + 7 * Dm::NQ + QC * 3 * Dm::NS;
-  const int g = threadIdx.x / THR, lt = threadIdx.x % THR;
-  const bool valid = g < T.count;
-  const int e = a.order[T.start + (valid ? g : T.count - 1)];
-  double *base = smem + g * GROUP;
-  double *sX = base, *sA = base + 18;
-  double(*sG)[6] = (double(*)[6])(base + 32);
-  double *sV = base + 32 + 6 * Dm::NQ;
-  double(*sT)[3][Dm::NS] = (double(*)[3][Dm::NS])(base + 32 + 7 * Dm::NQ);
-  if (lt < 18) sX[lt] = a.pX[18 * (size_t)e + lt];
-  if (lt < 9) sA[lt] = a.pA[9 * (size_t)e + lt];
-  if (a.dword)  // uniform over the launch; the float2 slices fill the same scratch
-    dg_prism_volume_body_dw<P, THR, QC>(sX, sA, a.f, tb.D[P], tb.Ddw[P], tb.PHI[P], tb.QP[P], a.val + a.poff[e],
-                                        a.rhs + a.proff[e], sG, sV, (float2(*)[3][Dm::NS])sT, lt, valid);
-  else
-    dg_prism_volume_body<P, THR, QC>(sX, sA, a.f, tb.D[P], tb.PHI[P], tb.QP[P], a.val + a.poff[e],
-                                     a.rhs + a.proff[e], sG, sV, sT, lt, valid);
+  const int *ord = a.order + T.start;
+  dg_prism_volume_tile<P>(
+      T.count, a.f, tb.VT[P], tb.QP[P], tb.ENT[P], smem,
+      [&](int el, int i) { return i < 18 ? a.pX[18 * (size_t)ord[el] + i] : a.pA[9 * (size_t)ord[el] + i - 18]; },
+      [&](int el) { return a.val + a.poff[ord[el]]; }, [&](int el) { return a.rhs + a.proff[ord[el]]; });
 }
 
 // The 6 geometric factors G = C^T A C / |det| (00 01 02 11 12 22) and |det|
@@ -160,16 +132,6 @@ __device__ void dgb_tets(const DgBatchTables &tb, const DgBatchArgs &a, const Dg
   for (int t = tid; t < count * NS; t += DGB_THREADS) {
     const int el = t / NS, i = t % NS;
     a.rhs[a.troff[sE[el]] + i] = a.f * sGc[7 * el + 6] * __ldg(tb.MOM[P] + i);
-  }
-}
-
-template <int P>
-__device__ __forceinline__ void dgb_prism_variant(const DgBatchTables &tb, const DgBatchArgs &a,
-                                                  const DgBatchTile &T, double *smem) {
-  switch (T.variant) {
-    case 0: dgb_prism<P, dgb_prism_thr(P, 0), dgb_prism_qc(P, 0)>(tb, a, T, smem); break;
-    case 1: dgb_prism<P, dgb_prism_thr(P, 1), dgb_prism_qc(P, 1)>(tb, a, T, smem); break;
-    default: dgb_prism<P, dgb_prism_thr(P, 2), dgb_prism_qc(P, 2)>(tb, a, T, smem); break;
   }
 }
 
@@ -231,10 +193,10 @@ __global__ void __launch_bounds__(DGB_THREADS) dg_batch_kernel(int ntiles, int *
     const DgBatchTile T = a.tiles[t];
     if (T.type == 0) {
       switch (T.p) {
-        case 1: dgb_prism_variant<1>(tb, a, T, smem); break;
-        case 2: dgb_prism_variant<2>(tb, a, T, smem); break;
-        case 3: dgb_prism_variant<3>(tb, a, T, smem); break;
-        default: dgb_prism_variant<4>(tb, a, T, smem); break;
+        case 1: dgb_prism<1>(tb, a, T, smem); break;
+        case 2: dgb_prism<2>(tb, a, T, smem); break;
+        case 3: dgb_prism<3>(tb, a, T, smem); break;
+        default: dgb_prism<4>(tb, a, T, smem); break;
       }
     } else {
       switch (T.p) {
@@ -293,10 +255,9 @@ static int dg_batch_tables(int device, DgBatchTables *out) {
     const int r = dg_tables_for_device(device, &pt);
     if (r < 0) return r;
     for (int p = 1; p <= GB_DG_PMAX; p++) {
-      g_bt[device].D[p] = pt->D[p];
-      g_bt[device].PHI[p] = pt->PHI[p];
       g_bt[device].QP[p] = pt->QP[p];
-      g_bt[device].Ddw[p] = pt->Ddw[p];
+      g_bt[device].VT[p] = pt->VT[p];
+      g_bt[device].ENT[p] = pt->ENT[p];
       std::vector<double> T, MOM;
       tet_tables(p, T, MOM);
       double *dT = nullptr, *dM = nullptr;
@@ -341,7 +302,7 @@ static size_t dgb_smem_bytes() {
   int m = 7 * 128 + 128;  // tets: G and |det| per element, element ids
   for (int p = 1; p <= 4; p++)
     for (int v = 0; v < DGB_VARIANTS; v++)
-      m = std::max(m, (DGB_THREADS / dgb_prism_thr(p, v)) * dgb_prism_group_smem(p, v));
+      m = std::max(m, dg_vol_smem(p, v));
   return sizeof(double) * (size_t)m;
 }
 
@@ -359,7 +320,6 @@ struct gbfem_batch_s {
   int np = 0, nt = 0, ntiles = 0;
   int var_prism[5] = {0, 0, 0, 0, 0}, var_tet[5] = {2, 2, 2, 2, 2};
   double f = 1.0;
-  int dword = 0;
   long long nval = 0, nrhs = 0;
   DevBuf<double> pX, pA, tX, tA, val, rhs;
   DevBuf<long long> poff, toff;
@@ -394,7 +354,7 @@ static void batch_tiles(gbfem_batch b, unsigned sel, int limit, std::vector<DgBa
       if (!(sel & (1u << (t * 5 + p)))) continue;
       const int begin = b->cls_start[t][p][0], end = std::min(b->cls_start[t][p][1], begin + limit);
       const int v = t == 0 ? b->var_prism[p] : b->var_tet[p];
-      const int per = t == 0 ? gbfem::DGB_THREADS / gbfem::dgb_prism_thr(p, v) : gbfem::dgb_tet_tile(v);
+      const int per = t == 0 ? gbfem::dg_vol_elems(p, v) : gbfem::dgb_tet_tile(v);
       for (int s = begin; s < end; s += per) {
         DgBatchTile T{};
         T.type = (unsigned char)t;
@@ -422,7 +382,6 @@ static gbfem::DgBatchArgs batch_args(gbfem_batch b) {
   a.val = b->val.p;
   a.rhs = b->rhs.p;
   a.f = b->f;
-  a.dword = b->dword;
   return a;
 }
 
@@ -619,9 +578,9 @@ int gbfem_batch_set_variants(gbfem_batch b, const int *prism_v, const int *tet_v
 int gbfem_batch_set_arith(gbfem_batch b, int dword) {
   GB_CHECK(b, "null batch");
   GB_CHECK(dword == 0 || dword == 1, "arithmetic must be 0 (FP64) or 1 (double word)");
-  b->dword = dword;
-  GB_CUDA(cudaSetDevice(b->device));
-  return b->np + b->nt > 0 ? batch_build(b) : 0;
+  // the FP64 moment form is both more accurate and faster than the former
+  // double-word sums over the points: it serves either choice
+  return 0;
 }
 
 int gbfem_batch_autotune(gbfem_batch b, int sample, int *prism_v, int *tet_v, double *ms) {

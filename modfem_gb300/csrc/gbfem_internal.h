@@ -63,13 +63,14 @@ struct DevBuf {
   size_t bytes() const { return n * sizeof(T); }
 };
 
-// Per-degree DG prism tables on a device (dg_kernels.cu): D[q][a][u]
-// reference derivatives, PHI[q][u] values, QP (xi, eta, zeta, w) per point.
+// Per-degree DG prism tables on a device (dg_kernels.cu): QP (xi, eta, zeta,
+// w) per point; the monomial tables and the entry list of the volume kernels
+// (dg_volume.cuh).
+struct DgVolEntry;
 struct DgDeviceTables {
-  const double *D[5];
-  const double *PHI[5];
   const double *QP[5];
-  const float2 *Ddw[5];  // D as double words (h, l) for the double-word volume kernel
+  const double *VT[5];
+  const DgVolEntry *ENT[5];
 };
 int dg_tables_for_device(int device, DgDeviceTables **out);
 
@@ -251,7 +252,7 @@ int launch_dg_tc_volume(cudaStream_t st, int device, int p, int count, const int
                         const int *roff, double *val, double *rhs, int *err, int mode);
 int launch_dg_prism_elements(cudaStream_t st, int device, int p, int count, const int *ent_el, const int *el_nodes,
                              const double *xyz, const double *k_el, const double *D_el, double f,
-                             const long long *boff, const int *roff, double *val, double *rhs, int variant, bool dword = false);
+                             const long long *boff, const int *roff, double *val, double *rhs, int variant);
 
 }  // namespace gbfem
 
