@@ -269,12 +269,14 @@ int gbfem_dg_set_volume_kernel(gbfem_ctx ctx, int mode);
  * slices per operand, exact FP32 slice sums, recombination rounded once to
  * FP64: the reference's face matrices to FP64 accuracy) for owners of degree
  * <= 3 whose neighbours all have degree <= 3; other owners keep the FP64
- * kernel; or GBFEM_DG_FACE_DWORD, the FP64 kernel's algebra with the point
- * tables in double-word (float pair) form and every entry summed on the
- * FP32 pipes by exact products and sums (errors of order 2^-48 of the summed
- * magnitudes), all degrees, prisms and tetrahedra; or
- * GBFEM_DG_FACE_TC_DWORD: the tensor cores where they apply (prisms) and the
- * double-word kernel for the other owners. */
+ * sums over the face points.  GBFEM_DG_FACE_DWORD asks for entries within
+ * 2^-48 of the summed magnitudes, GBFEM_DG_FACE_TC_DWORD for the tensor cores
+ * where they apply (prisms) and that accuracy elsewhere: between prisms the
+ * FP64 kernel (moments of the face geometry) meets both and is the fastest,
+ * so it serves them; tetrahedra, and prism meshes in which a quadrilateral is
+ * turned by 90 degrees between its neighbours (the moment form does not cover
+ * those), take the point sums in double-word (float pair) arithmetic on the
+ * FP32 pipes (or the tensor cores). */
 #define GBFEM_DG_FACE_FP64 0
 #define GBFEM_DG_FACE_TC 1
 #define GBFEM_DG_FACE_DWORD 2

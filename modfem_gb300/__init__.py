@@ -290,8 +290,8 @@ class Context:
         self._check(self.L.gbfem_dg_set_volume_kernel(self._h, mode))
 
     def dg_set_face_kernel(self, mode):
-        """DG_FACE_FP64, DG_FACE_TC (tensor cores, split BF16, FP64-equivalent), DG_FACE_DWORD (double-word
-        sums on the FP32 pipes) or DG_FACE_TC_DWORD (tensor cores where they apply, double word elsewhere)."""
+        """DG_FACE_FP64, DG_FACE_TC (tensor cores, split BF16, FP64-equivalent), DG_FACE_DWORD (entries to
+        double-word accuracy) or DG_FACE_TC_DWORD (the fastest of at least that accuracy)."""
         self._check(self.L.gbfem_dg_set_face_kernel(self._h, mode))
 
     def dg_build_structure(self):

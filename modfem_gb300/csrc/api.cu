@@ -8,6 +8,7 @@
 #include <functional>
 #include <mutex>
 
+#include "dg_tables.h"
 #include "gbfem_internal.h"
 
 namespace gbfem {
@@ -236,6 +237,9 @@ int gbfem_destroy(gbfem_ctx c) {
   }
   c->dg_mhf_ptr.release();
   c->dg_mhf.release();
+  c->dg_frec.release();
+  c->dg_hrec.release();
+  c->dg_ffield.release();
   c->el_nodes4.release();
   c->dg_boff_diag_d.release();
   c->dg_val.release();
@@ -287,6 +291,7 @@ long long gbfem_device_bytes(gbfem_ctx c) {
   for (int cls = 0; cls < 9; cls++) s += c->dg_list[cls].bytes() + c->dg_mlist[cls].bytes();
   for (int p = 0; p < 5; p++) s += c->dg_flist_tc[p].bytes() + c->dg_flist_64[p].bytes();
   s += c->dg_mhf_ptr.bytes() + c->dg_mhf.bytes() + c->el_nodes4.bytes();
+  s += c->dg_frec.bytes() + c->dg_hrec.bytes() + c->dg_ffield.bytes();
   return s;
 }
 
@@ -1384,15 +1389,25 @@ int gbfem_dg_build_structure(gbfem_ctx c, int *ndof, long long *nval) {
   // face-point configurations (vertex count, local vertex order) of the
   // tensor-core face kernel's basis tables (faces between prisms)
   std::vector<unsigned char> cfgs;
+  std::vector<short> cfg_at(2 * 4096, -1);  // by (vertex count, local vertices of 3 bits)
   auto cfg_of = [&](int nfv, const unsigned char *loc) -> int {
+    short &at = cfg_at[4096 * (nfv == 4) + (loc[0] | loc[1] << 3 | loc[2] << 6 | (nfv == 4 ? loc[3] << 9 : 0))];
+    if (at >= 0) return at;
     const int ncfg = (int)cfgs.size() / 5;
-    for (int k = 0; k < ncfg; k++)
-      if (cfgs[5 * k] == nfv && memcmp(&cfgs[5 * k + 1], loc, nfv) == 0) return k;
     if (ncfg >= gbfem::DG_TF_MAXCFG) return 255;
     cfgs.push_back((unsigned char)nfv);
     for (int i = 0; i < 4; i++) cfgs.push_back(i < nfv ? loc[i] : 0);
+    at = (short)ncfg;
     return ncfg;
   };
+  // records of the moment form of the faces between prisms and of their
+  // Dirichlet faces, sorted below
+  std::vector<gbfem::DgFaceRec> frec;
+  std::vector<int> frec_face;
+  frec.reserve(nfa);
+  frec_face.reserve(nfa);
+  bool mom_ok = true;
+  int fb_count[8][2] = {};
   std::vector<int> face_rep(nfa, -1);  // the first neighbour's record of each face between prisms
   for (int f = 0; f < nfa; f++) {
     gbfem::DgHalfFace h;
@@ -1424,12 +1439,76 @@ int gbfem_dg_build_structure(gbfem_ctx c, int *ndof, long long *nval) {
       mhf[mfill[h.el2]++] = h;
       continue;
     }
-    if (!el_is_tet(c, h.el1)) face_rep[f] = hfill[h.el1];
+    const bool prism = !el_is_tet(c, h.el1);
+    if (prism) face_rep[f] = hfill[h.el1];
     hf[hfill[h.el1]++] = h;
+    const long long blk1 = h.blk;
     if (h.el2 >= 0) {
       h.owner_is_2 = 1;
       h.blk = block_of(h.el2, h.el1);
       hf[hfill[h.el2]++] = h;
+    }
+    if (prism) {
+      gbfem::DgFaceRec r;
+      memset(&r, 0, sizeof(r));
+      r.el1 = h.el1;
+      r.el2 = h.el2;
+      r.blk1 = blk1;
+      r.blk2 = h.blk;
+      memcpy(r.loc1, h.loc1, 4);
+      memcpy(r.loc2, h.loc2, 4);
+      r.side1 = (unsigned char)h.side1;
+      r.nfv = (unsigned char)h.nfv;
+      r.p1 = (unsigned char)c->dg_p[h.el1];
+      r.p2 = h.el2 >= 0 ? (unsigned char)c->dg_p[h.el2] : 0;
+      mom_ok = mom_ok && gbfem::dg_face_moments_cover(r);
+      fb_count[4 * (r.nfv == 4) + std::max(r.p1, r.p2) - 1][r.el2 < 0]++;
+      frec.push_back(r);
+      frec_face.push_back(f);
+    }
+  }
+  // the records by bucket 4 (triangles 0, quadrilaterals 1) + larger degree
+  // - 1, interior faces before boundary faces, table order within; not used
+  // when a face does not suit the form or an element has more faces than sides
+  {
+    int at[8][2], n = 0;
+    long long geo_at[8][2], geo = 0;
+    for (int b = 0; b < 8; b++) {
+      c->dg_fb_start[b] = n;
+      c->dg_fb_inner[b] = fb_count[b][0];
+      for (int k = 0; k < 2; k++) {
+        at[b][k] = n;
+        geo_at[b][k] = geo;
+        n += fb_count[b][k];
+        geo += 7ll * GB_DG_NQF[b % 4 + 1][b / 4] * fb_count[b][k];
+      }
+    }
+    c->dg_fb_start[8] = n;
+    std::vector<gbfem::DgFaceRec> all(n);
+    std::vector<int> rec_of(nfa, -1), hrec(hf.size());
+    for (size_t i = 0; i < frec.size(); i++) {
+      gbfem::DgFaceRec &r = frec[i];
+      const int b = 4 * (r.nfv == 4) + std::max(r.p1, r.p2) - 1, k = r.el2 < 0;
+      r.geo = geo_at[b][k];
+      geo_at[b][k] += 7 * GB_DG_NQF[b % 4 + 1][b / 4];
+      rec_of[frec_face[i]] = at[b][k];
+      all[at[b][k]++] = r;
+    }
+    for (int e = 0; e < nel; e++) {
+      if (el_is_tet(c, e)) continue;
+      int quads = 0, tris = 0;
+      for (int h = hptr[e]; h < hptr[e + 1]; h++) {
+        hrec[h] = 2 * rec_of[hf[h].face] + hf[h].owner_is_2;
+        (hf[h].nfv == 4 ? quads : tris)++;
+      }
+      mom_ok = mom_ok && quads <= 3 && tris <= 2;
+    }
+    c->dg_mom_ok = mom_ok && n > 0;
+    c->dg_ffield_n = geo;
+    if (c->dg_mom_ok) {
+      GB_TRY(upload(c, c->dg_frec, all.data(), all.size()));
+      GB_TRY(upload(c, c->dg_hrec, hrec.data(), hrec.size()));
+      GB_CUDA(cudaStreamSynchronize(c->stream));  // the host arrays end here
     }
   }
   // tables and face list for the tensor-core face kernel (faces between
@@ -1473,13 +1552,14 @@ int gbfem_dg_build_structure(gbfem_ctx c, int *ndof, long long *nval) {
   // ordered by their row's column count so that the rows a warp multiplies
   // together take the same number of steps; the owners of faces between a
   // prism and a tetrahedron per class
+  std::vector<int> lsts[9], mlsts[9];
+  for (int e = 0; e < nel; e++) {
+    const int cls = dg_cls(c, e);
+    lsts[cls].push_back(e);
+    if (mcnt[e]) mlsts[cls].push_back(e);
+  }
   for (int cls = 1; cls <= 8; cls++) {
-    std::vector<int> lst, mlst;
-    for (int e = 0; e < nel; e++)
-      if (dg_cls(c, e) == cls) {
-        lst.push_back(e);
-        if (mcnt[e]) mlst.push_back(e);
-      }
+    std::vector<int> &lst = lsts[cls], &mlst = mlsts[cls];
     c->dg_list[cls].release();
     c->dg_mlist[cls].release();
     if (lst.empty()) continue;
@@ -1492,17 +1572,19 @@ int gbfem_dg_build_structure(gbfem_ctx c, int *ndof, long long *nval) {
   // prism face owners of degree <= 3 whose neighbours across faces between
   // prisms all have degree <= 3 suit the tensor-core face kernel; the others
   // keep the FP64 one
-  for (int p = 1; p <= 4; p++) {
-    std::vector<int> tcl, fpl;
-    for (int e = 0; e < nel; e++) {
-      if (c->dg_p[e] != p || el_is_tet(c, e)) continue;
-      bool ok = p <= 3;
-      for (int h = hptr[e]; ok && h < hptr[e + 1]; h++) {
-        const int nb = hf[h].owner_is_2 ? hf[h].el1 : hf[h].el2;
-        if (nb >= 0 && c->dg_p[nb] > 3) ok = false;
-      }
-      (ok ? tcl : fpl).push_back(e);
+  std::vector<int> tcls[5], fpls[5];
+  for (int e = 0; e < nel; e++) {
+    if (el_is_tet(c, e)) continue;
+    const int p = c->dg_p[e];
+    bool ok = p <= 3;
+    for (int h = hptr[e]; ok && h < hptr[e + 1]; h++) {
+      const int nb = hf[h].owner_is_2 ? hf[h].el1 : hf[h].el2;
+      if (nb >= 0 && c->dg_p[nb] > 3) ok = false;
     }
+    (ok ? tcls : fpls)[p].push_back(e);
+  }
+  for (int p = 1; p <= 4; p++) {
+    const std::vector<int> &tcl = tcls[p], &fpl = fpls[p];
     c->dg_flist_tc[p].release();
     c->dg_flist_64[p].release();
     if (!tcl.empty()) GB_TRY(upload(c, c->dg_flist_tc[p], tcl.data(), tcl.size()));
@@ -1549,6 +1631,19 @@ int gbfem_dg_get_structure(gbfem_ctx c, int *dof_off, int *bptr, int *bcol, long
   return (int)c->dg_bcol.size();
 }
 
+// Point fields of every face of the moment form; returns the launches.
+static int launch_mom_fields(gbfem_ctx c) {
+  int n = 0;
+  for (int b = 0; b < 8; b++) {
+    const int r = gbfem::launch_dg_face_fields(c->stream, b % 4 + 1, b / 4, c->dg_fb_start[b + 1] - c->dg_fb_start[b],
+                                               c->dg_frec.p + c->dg_fb_start[b], c->el_nodes.p, c->xyz.p, c->k_el.p,
+                                               c->D_el.p, c->dg_pen, c->dg_ffield.p);
+    GB_TRY(r);
+    n += r;
+  }
+  return n;
+}
+
 int gbfem_dg_assemble(gbfem_ctx c) {
   GB_CHECK(c && c->dg_ready, "DG structure not built (gbfem_dg_build_structure)");
   GB_TRY(settle_uploads(c));
@@ -1559,7 +1654,11 @@ int gbfem_dg_assemble(gbfem_ctx c) {
   const bool tc = c->dg_volume_mode == GBFEM_DG_VOLUME_TC || c->dg_volume_mode == GBFEM_DG_VOLUME_TF32 ||
                   c->dg_volume_mode == GBFEM_DG_VOLUME_TC_DWORD;
   if (tc) GB_CUDA(cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream));
-  const bool tcf = c->dg_face_mode == GBFEM_DG_FACE_TC || c->dg_face_mode == GBFEM_DG_FACE_TC_DWORD;
+  // faces between prisms from moments: the FP64 form, and the fastest that
+  // meets the double-word accuracy (p = 3, 54,000 prisms: 5.9 ms; sums
+  // over the points 48 ms, in double words 22 ms, on the tensor cores 14 ms)
+  const bool mom = c->dg_mom_ok && c->dg_face_mode != GBFEM_DG_FACE_TC;
+  const bool tcf = !mom && (c->dg_face_mode == GBFEM_DG_FACE_TC || c->dg_face_mode == GBFEM_DG_FACE_TC_DWORD);
   // Tensor-core faces beside a volume kernel on the CUDA cores (FP64 or
   // double word): the face kernel runs on the side stream from the start,
   // its diagonal-block and rhs shares go to scratch and are added once both
@@ -1654,7 +1753,28 @@ int gbfem_dg_assemble(gbfem_ctx c) {
       GB_TRY(r);
       launches += r;
     }
-    for (int p = 1; p <= 4; p++) {
+    if (mom) {
+      GB_TRY(c->dg_ffield.alloc((size_t)c->dg_ffield_n));
+      const int rf = launch_mom_fields(c);
+      GB_TRY(rf);
+      launches += rf;
+      for (int p = 1; p <= 4; p++) {
+        if (!c->dg_list[p].p) continue;
+        const int r = gbfem::launch_dg_face_diag(c->stream, c->device, p, (int)c->dg_list[p].n, c->dg_list[p].p,
+                                                 c->dg_hf_ptr.p, c->dg_hrec.p, c->dg_frec.p, c->dg_ffield.p, c->g,
+                                                 c->dg_boff_diag_d.p, c->dg_roff_d.p, c->dg_val.p, c->dg_rhs.p,
+                                                 c->dg_var_face[p]);
+        GB_TRY(r);
+        launches += r;
+      }
+      for (int b = 7; b >= 0; b--) {
+        const int r = gbfem::launch_dg_face_blocks(c->stream, c->device, b % 4 + 1, b / 4, c->dg_fb_inner[b],
+                                                   c->dg_frec.p + c->dg_fb_start[b], c->dg_ffield.p, c->dg_val.p);
+        GB_TRY(r);
+        launches += r;
+      }
+    }
+    for (int p = 1; !mom && p <= 4; p++) {
       if (!c->dg_list[p].p) continue;
       if (tcf && c->dg_ftab_ok) {
         // tensor-core eligible owners (done above when overlapped), then the
@@ -1770,6 +1890,10 @@ int gbfem_dg_autotune(gbfem_ctx c, int sample, int *vol_out, int *face_out, doub
     }
     return 0;
   };
+  if (c->dg_hf.p && c->dg_mom_ok) {
+    GB_TRY(c->dg_ffield.alloc((size_t)c->dg_ffield_n));
+    GB_TRY(launch_mom_fields(c));
+  }
   for (int p = 1; p <= 4; p++) {
     if (!c->dg_list[p].p) continue;
     const int cnt = (int)std::min<size_t>(c->dg_list[p].n, (size_t)sample);
@@ -1791,6 +1915,10 @@ int gbfem_dg_autotune(gbfem_ctx c, int sample, int *vol_out, int *face_out, doub
       for (int v = 0; v < 2; v++) {
         float ms;
         GB_TRY(time_it([&] {
+          if (c->dg_mom_ok)
+            return gbfem::launch_dg_face_diag(st, c->device, p, cnt, c->dg_list[p].p, c->dg_hf_ptr.p, c->dg_hrec.p,
+                                              c->dg_frec.p, c->dg_ffield.p, c->g, c->dg_boff_diag_d.p, c->dg_roff_d.p,
+                                              c->dg_val.p, c->dg_rhs.p, v);
           return gbfem::launch_dg_prism_faces(st, p, cnt, c->dg_list[p].p, c->dg_hf_ptr.p, c->dg_hf.p, c->dg_p_d.p,
                                               c->el_nodes.p, c->xyz.p, c->k_el.p, c->D_el.p, c->dg_pen, c->g,
                                               c->dg_boff_diag_d.p, c->dg_roff_d.p, c->dg_val.p, c->dg_rhs.p, v);

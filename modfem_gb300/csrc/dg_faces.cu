@@ -1,5 +1,7 @@
-// DG prism face integrals on the device, one CTA per element (the owner of a
-// block row), FP64.
+// DG prism face integrals on the device as sums over the face points, one CTA
+// per element (the owner of a block row), FP64 or double words: the form for
+// meshes that the moment form (dg_face_moments.cu, 6 to 8 times fewer FP64
+// operations) does not cover, and for the owners that the tensor-core faces leave.
 //
 // Reference: pdr_conv_diff_comp_fa_stiff_mat_app of the DG weak form
 // (pds_conv_diff_weakform_dg.c:232-1140), assembled by lar_assemble_SM_and_LV_

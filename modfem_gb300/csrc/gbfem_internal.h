@@ -169,6 +169,35 @@ struct DgHalfFace {
 };
 static_assert(sizeof(DgHalfFace) == 40, "half-face record layout");
 
+// One face of a prism mesh for the moment form of the face integrals
+// (dg_face_moments.cu): its neighbours (el2 = -1 on a Dirichlet face) and their
+// degrees, the value offsets of blocks (el1, el2) and (el2, el1), the local vertex
+// index in each neighbour of the face vertices, the side of el1, and the
+// offset of its point fields.  Records are sorted by (triangles /
+// quadrilaterals, larger degree), interior faces first.
+struct DgFaceRec {
+  int el1, el2;
+  long long blk1, blk2, geo;
+  unsigned char loc1[4], loc2[4];
+  unsigned char side1, nfv, p1, p2;
+};
+// Whether the moment form covers the face: the edge direction of a
+// quadrilateral is the same in both neighbours, a triangle is a bottom or top
+bool dg_face_moments_cover(const DgFaceRec &r);
+// Point fields of `count` faces of one rule (degree pm, ti 0 triangles, 1
+// quadrilaterals): 7 x nq doubles a face at geo + rec.geo
+int launch_dg_face_fields(cudaStream_t st, int pm, int ti, int count, const DgFaceRec *rec, const int *el_nodes,
+                          const double *xyz, const double *k_el, const double *D_el, double pen, double *geo);
+// Diagonal shares and boundary loads of the owners of degree p; hrec[h] = 2
+// record + (1 if the owner is its second neighbour) of half-face h.  variant:
+// threads per CTA (same results).
+int launch_dg_face_diag(cudaStream_t st, int device, int p, int count, const int *ent_el, const int *hf_ptr,
+                        const int *hrec, const DgFaceRec *rec, const double *geo, double g, const long long *boff_diag,
+                        const int *roff, double *val, double *rhs, int variant);
+// Both off-diagonal blocks of `count` interior faces of one rule
+int launch_dg_face_blocks(cudaStream_t st, int device, int pm, int ti, int count, const DgFaceRec *rec,
+                          const double *geo, double *val);
+
 int launch_dg_tet_elements(cudaStream_t st, int device, int p, int count, const int *ent_el, const int *el_nodes,
                            const double *xyz, const double *k_el, const double *D_el, double f,
                            const long long *boff, const int *roff, double *val, double *rhs);
@@ -386,6 +415,15 @@ struct gbfem_ctx_s {
   int dg_var_vol[5] = {0, 0, 0, 0, 0}, dg_var_face[5] = {0, 0, 0, 0, 0};  // launch-shape variants per degree
   gbfem::DevBuf<int> dg_hf_ptr, dg_p_d;
   gbfem::DevBuf<gbfem::DgHalfFace> dg_hf;
+  // faces of the prisms for the moment form: sorted records, the record of
+  // each half-face, records before each (ti, degree) bucket and its interior
+  // count, point fields; dg_mom_ok: every face between prisms is covered
+  gbfem::DevBuf<gbfem::DgFaceRec> dg_frec;
+  gbfem::DevBuf<int> dg_hrec;
+  gbfem::DevBuf<double> dg_ffield;
+  int dg_fb_start[9] = {}, dg_fb_inner[8] = {};
+  long long dg_ffield_n = 0;
+  bool dg_mom_ok = false;
   // tensor-core faces: face-point configurations, basis tables at the face
   // points, faces between degree <= 3 elements (a record of each) and their
   // per-point geometry
