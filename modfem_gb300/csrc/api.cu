@@ -205,6 +205,7 @@ int gbfem_destroy(gbfem_ctx c) {
   }
   c->row_last.release();
   if (c->gm_graph) cudaGraphExecDestroy(c->gm_graph);
+  if (c->gm_host) cudaFreeHost(c->gm_host);
   c->sell_off.release();
   c->sell_col.release();
   c->sell_col16.release();
@@ -213,7 +214,7 @@ int gbfem_destroy(gbfem_ctx c) {
   c->gm_xdw.release();
   c->gm_small.release();
   c->gm_npart.release();
-  c->gm_cnt.release();
+  c->gm_alive.release();
   if (c->side_stream) {
     cudaStreamSynchronize(c->side_stream);
     cudaStreamDestroy(c->side_stream);

@@ -380,13 +380,14 @@ struct gbfem_ctx_s {
   // matrix, small arrays and state, the captured restart cycle
   gbfem::DevBuf<int> sell_off, sell_col;
   gbfem::DevBuf<double> sell_val, gm_small, gm_npart;
-  gbfem::DevBuf<unsigned> gm_cnt;
+  gbfem::DevBuf<int> gm_alive;
   gbfem::DevBuf<float2> sell_valdw, gm_xdw;
   gbfem::DevBuf<short> sell_col16;  // columns relative to the row, where they fit in 16 bits
   bool sell_ready = false, std_spmv_dword = false, sell_cols16 = false;
   int sell_n = 0;
   long long sell_nnz = 0, sell_total = 0;
   cudaGraphExec_t gm_graph = nullptr;
+  void *gm_host = nullptr;  // page-locked copy of the solver's state
   int gm_key_n = 0, gm_key_m = 0, gm_kernels = 0;
   bool gm_key_dw = false;
   unsigned char gm_key_args[256] = {};

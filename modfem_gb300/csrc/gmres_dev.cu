@@ -10,16 +10,22 @@
 // the rotations, the convergence test and the small triangular solve run on
 // the device, and every kernel of a restart cycle (restart residual, m
 // Arnoldi steps, update of x) reads a state word and returns at once when the
-// cycle has already ended.  An Arnoldi step is three kernels: the SpMV, the
-// Gram-Schmidt dot products (the last block of each column entry to finish
-// sums its block partials) and the orthogonalisation, one row a thread (its
-// last block to finish runs the step's logic: norm, Givens rotations, test).
-// Krylov vectors after the first are stored unnormalised with a scale each
-// (V_k = sc_k W_k), applied by their readers, so no normalisation pass runs;
-// the cycle's triangular solve runs in the update of x.  "Last block" is an
-// atomic count after a memory fence: nothing waits.  One cycle is captured
+// cycle has already ended.  An Arnoldi step is the SpMV, the Gram-Schmidt dot
+// products and the orthogonalisation; small systems, where the step is a chain
+// of latencies, form the dots in the SpMV kernel.  No kernel has a serial
+// tail: the block partials of the dots are summed at the start of the
+// orthogonalisation (by every block, in the same order), and the step's logic
+// (norm, rotations, test, at the end of a cycle the triangular solve) runs in
+// one extra block of the next step's SpMV, which therefore starts before the
+// test of the step before it is known; a step that turns out not to be wanted
+// leaves nothing behind (alive[], below).  Krylov vectors after the first are
+// stored unnormalised with a scale each (V_k = sc_k W_k), applied by their
+// readers, so no normalisation pass runs.  Every dependence is a kernel
+// boundary: no atomics, no fences.  One cycle is captured
 // as a CUDA graph (per context, matrix size and Krylov dimension) and
-// replayed; the host reads the state once per cycle.
+// replayed; the host reads the state once per cycle.  Large systems are bound
+// by the FP64 pipe (SpMV 21, dots and orthogonalisation j + 1 FMA a row each at
+// 0.63 T/s) with HBM close behind.
 //
 // The SpMV runs on a sliced-ELL copy of the CRS matrix (SELL-32 in natural
 // row order: slice s = rows 32 s .. 32 s + 31, padded to the slice's longest
@@ -49,7 +55,6 @@ namespace gbfem {
 
 constexpr int GM_T = 256;
 constexpr int GM_MMAX = 256;  // largest Krylov dimension (gbfem_solve's check)
-constexpr int GM_RSTAGE = 64;  // Krylov dimensions up to which the triangular solve runs on a shared copy of R
 constexpr int SELL_C = 32;
 
 // ---------------------------------------------------------------- SELL-32
@@ -170,22 +175,30 @@ __device__ __forceinline__ double sell_row_dw(const float2 *__restrict__ v, cons
   return dw_to_double(dw(acc0.h, acc0.l) + dw(acc1.h, acc1.l));
 }
 
-template <typename VT, typename CT>
+// GUARDED: the last batch is guarded (w is the same for the whole warp)
+// instead of finished entry by entry: a prism row's 21 entries are three
+// rounds of memory latency, not seven, at more registers (74 against 40):
+// better where few warps run, worse where occupancy hides the latency
+// (1,030,301 rows: 58 us against 46).
+template <bool GUARDED = false, typename VT, typename CT>
 __device__ __forceinline__ double sell_row(const VT *__restrict__ v, const CT *__restrict__ col, int w, int base,
                                            const double *__restrict__ x) {
   using AT = typename std::conditional<sizeof(VT) == 8 && std::is_same<VT, double>::value, double, dw>::type;
   constexpr int U = 8;  // entries whose loads are in flight together
   AT acc = AT(0.0);
   int j = 0;
-  for (; j + U <= w; j += U) {
+  for (; GUARDED ? j < w : j + U <= w; j += U) {
     VT a[U];
     double xv[U];
 #pragma unroll
-    for (int u = 0; u < U; u++) a[u] = sell_ld(v + u * SELL_C);
+    for (int u = 0; u < U; u++)
+      if (!GUARDED || j + u < w) a[u] = sell_ld(v + u * SELL_C);
 #pragma unroll
-    for (int u = 0; u < U; u++) xv[u] = __ldg(x + sell_col(col + u * SELL_C, base));
+    for (int u = 0; u < U; u++)
+      if (!GUARDED || j + u < w) xv[u] = __ldg(x + sell_col(col + u * SELL_C, base));
 #pragma unroll
-    for (int u = 0; u < U; u++) sell_acc(acc, a[u], xv[u]);
+    for (int u = 0; u < U; u++)
+      if (!GUARDED || j + u < w) sell_acc(acc, a[u], xv[u]);
     v += U * SELL_C;
     col += U * SELL_C;
   }
@@ -217,9 +230,11 @@ struct GmArgs {
   double *sc;  // scale of each Krylov vector: V_k = sc_k W_k, W_k stored
   float2 *xdw;  // double-word copy of the current Arnoldi vector (double-word SpMV only)
   GmState *st;
-  int ng;          // blocks of the row-parallel kernels
+  int m;           // Krylov dimension
+  int nd;          // blocks of the dots
+  int ng;          // blocks of the orthogonalisation
   double *npart;   // [ng] their norm partials
-  unsigned *cnt;   // [m + 2] finished-block counts (dot products 0..m-1, orthogonalisation m + 1)
+  int *alive;      // [m + 1] alive[j]: step j of the cycle is wanted (set by the restart test and the logic of j - 1)
 };
 
 // sum of nb partials in a fixed order (one block of GM_T threads); valid in thread 0
@@ -297,6 +312,7 @@ __global__ void __launch_bounds__(GM_T) gm_logic_restart(GmArgs a) {
   const double tot = gm_block_total(a.partial, a.nb);
   if (threadIdx.x != 0) return;
   S.done_cols = 0;
+  for (int i = 0; i <= S.m; i++) a.alive[i] = 0;  // nothing of the last cycle is left standing
   if (S.final_flag) {
     S.phase = GM_DONE;
     return;
@@ -310,6 +326,7 @@ __global__ void __launch_bounds__(GM_T) gm_logic_restart(GmArgs a) {
   }
   a.s[0] = rn;
   for (int i = 1; i <= S.m; i++) a.s[i] = 0.0;
+  a.alive[0] = 1;
   a.sc[0] = 1.0;  // V_0 is stored normalised
   S.beta = rn;
   S.j = 0;
@@ -327,181 +344,341 @@ __global__ void __launch_bounds__(GM_T) gm_start_cycle(GmArgs a) {
   }
 }
 
-// V[j+1] = dinv A V[j]
-template <typename VT, typename CT>
-__global__ void __launch_bounds__(GM_T) gm_arnoldi_spmv(GmArgs a, const VT *__restrict__ sv,
-                                                        const CT *__restrict__ scol, int j) {
-  const GmState &S = *a.st;
-  if (S.phase != GM_ARNOLDI || S.j != j) return;
-  const int s = blockIdx.x * (GM_T / 32) + threadIdx.x / 32, l = threadIdx.x & 31;
-  if (s >= a.nslices) return;
-  const int r = s * SELL_C + l;
-  const int o = a.sell_off[s], w = (a.sell_off[s + 1] - o) / SELL_C;
-  double acc;
-  if constexpr (std::is_same<VT, float2>::value)
-    acc = sell_row_dw(sv + o + l, scol + o + l, w, sell_base(r, a.n), a.xdw);
-  else
-    acc = sell_row(sv + o + l, scol + o + l, w, sell_base(r, a.n), a.V + (size_t)j * a.n);
-  // the copy holds D^-1 A; W_j is stored unnormalised: V_j = sc_j W_j
-  if (r < a.n) a.V[(size_t)(j + 1) * a.n + r] = a.sc[j] * acc;
-}
-
-// Gram-Schmidt dot products <W_k, w>, k = blockIdx.y <= j (w = W_{j+1}),
-// block partials; the last block of each
-// k to finish (an atomic count after a fence, no waiting) sums the partials
-// in block order (one warp, lane-strided then a shuffle tree) and stores the
-// column entry h_k = <V_k, w> = sc_k total.  Partials of other blocks are
-// read through L2 (__ldcg).
-__global__ void __launch_bounds__(GM_T) gm_dot_partial(GmArgs a, int j) {
-  const GmState &S = *a.st;
-  if (S.phase != GM_ARNOLDI || S.j != j) return;
-  __shared__ bool last;
-  const int k = blockIdx.y;
-  const double *v = a.V + (size_t)k * a.n, *w = a.V + (size_t)(j + 1) * a.n;
-  double s0 = 0.0;
-  for (long long i = (long long)blockIdx.x * GM_T + threadIdx.x; i < a.n; i += (long long)gridDim.x * GM_T)
-    s0 = fma(__ldg(v + i), __ldg(w + i), s0);
-  const double s = gm_block_sum(s0);
-  if (threadIdx.x == 0) {
-    a.partial[(size_t)k * a.nb + blockIdx.x] = s;
-    __threadfence();
-    last = atomicAdd(a.cnt + k, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last || threadIdx.x >= 32) return;
-  __threadfence();
-  double t = 0.0;
-  for (int b = threadIdx.x; b < a.nb; b += 32) t += __ldcg(a.partial + (size_t)k * a.nb + b);
+// Sums of eight values over a warp: afterwards lane l holds the sum of value
+// l / 4.  Each exchange halves the values a lane keeps: 9 adds instead of 40.
+__device__ __forceinline__ double gm_warp_sums(double (&t)[8], int lane) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (threadIdx.x == 0) {
-    a.hcol[k] = a.sc[k] * t;
-    a.cnt[k] = 0;  // for the next step
+  for (int h = 4, o = 16; h >= 1; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int u = 0; u < h; u++) {
+      const double send = up ? t[u] : t[u + h], keep = up ? t[u + h] : t[u];
+      t[u] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
   }
+  double v = t[0];
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v;
 }
 
-// The step's logic, by the last block of gm_orthogonalize: |w| from the
-// norm partials, the Hessenberg column j with the earlier rotations applied
-// (column and rotations staged in shared memory: thread 0's chain of
-// dependent operations then waits on no global memory), the new rotation,
-// the residual estimate and the decision (next step, or end of the cycle).
-__device__ void gm_step_logic(const GmArgs &a, int j, GmState &S) {
-  __shared__ double col[GM_MMAX + 2], rc[GM_MMAX + 1], rs[GM_MMAX + 1];
-  const int tid = threadIdx.x;
+// pairwise sum of N shared values at stride `st` (short chain of dependent adds)
+template <int N>
+__device__ __forceinline__ double gm_pairs(const double *p, int st) {
+  if constexpr (N == 1)
+    return p[0];
+  else
+    return gm_pairs<N / 2>(p, st) + gm_pairs<N - N / 2>(p + (N / 2) * st, st);
+}
+
+// The step's logic for step j (one block of T threads): |w| from the norm
+// partials, the earlier rotations applied to the Hessenberg column (the chain
+// c_{k+1} = rc_k h_{k+1} - rs_k c_k composes affine maps by a warp scan, 5 steps
+// per 32 rotations: an FP64 operation takes tens of cycles), the new rotation,
+// the residual estimate and the decision (next step, or end of the cycle,
+// where the block also solves R y = s by columns).
+template <int T>
+__device__ void gm_step_logic(const GmArgs &a, int j) {
+  __shared__ double col[GM_MMAX + 2];
+  __shared__ double sh[T / 32];
+  __shared__ int s_done;
+  GmState &S = *a.st;
+  const int tid = threadIdx.x, m = a.m, ld = m + 1;
   double v = 0.0;
-  for (int b = tid; b < a.ng; b += GM_T) v += __ldcg(a.npart + b);
-  __shared__ double sh[GM_T];
-  sh[tid] = v;
-  for (int k = tid; k <= j; k += GM_T) col[k] = __ldcg(a.hcol + k);
-  for (int k = tid; k < j; k += GM_T) {
-    rc[k] = a.cs[k];
-    rs[k] = a.sn[k];
+  for (int b = tid; b < a.ng; b += 4 * T) {
+    double x[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) x[u] = b + u * T < a.ng ? a.npart[b + u * T] : 0.0;
+    v += (x[0] + x[1]) + (x[2] + x[3]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((tid & 31) == 0) sh[tid >> 5] = v;
+  __syncthreads();
+  if (tid < 32) {
+    double *H = a.H + (size_t)j * ld;
+    double c = a.hcol[0];
+    for (int k0 = 0; k0 < j; k0 += 32) {
+      const int k = k0 + tid;
+      const double rc = k < j ? a.cs[k] : 1.0, rs = k < j ? a.sn[k] : 0.0, hk = k < j ? a.hcol[k + 1] : 0.0;
+      double A = k < j ? -rs : 1.0, B = rc * hk;  // (identity beyond the last rotation)
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double A1 = __shfl_up_sync(0xffffffffu, A, o), B1 = __shfl_up_sync(0xffffffffu, B, o);
+        if (tid >= o) {
+          B = fma(A, B1, B);
+          A *= A1;
+        }
+      }
+      const double next = fma(A, c, B);  // c_{k+1}
+      double prev = __shfl_up_sync(0xffffffffu, next, 1);
+      if (tid == 0) prev = c;
+      if (k < j) H[k] = fma(rc, prev, rs * hk);
+      c = __shfl_sync(0xffffffffu, next, 31);
+    }
+    if (tid == 0) {
+      const double h2 = gm_pairs<T / 32>(sh, 1), hn = sqrt(h2);
+      const double rr = hypot(c, hn), cj = c / rr, sj = hn / rr;
+      H[j] = rr;
+      H[j + 1] = 0.0;
+      a.cs[j] = cj;
+      a.sn[j] = sj;
+      const double s0 = a.s[j], s1 = -sj * s0, resid = fabs(s1);
+      a.s[j] = cj * s0;
+      a.s[j + 1] = s1;
+      const int it = S.it + 1;
+      S.it = it;
+      S.resid = resid;
+      S.hn = hn;
+      a.sc[j + 1] = 1.0 / hn;
+      const bool conv = resid < S.tol_abs || resid / S.beta0 < S.tol_rel;
+      const bool end = j == m - 1 || it >= S.max_iter || conv;
+      s_done = end;
+      if (end) {
+        S.done_cols = j + 1;
+        S.final_flag = (conv || it >= S.max_iter) ? 1 : 0;
+        S.phase = GM_RESTART;
+      } else {
+        S.j = j + 1;
+        a.alive[j + 1] = 1;
+      }
+    }
   }
   __syncthreads();
-  for (int o = GM_T / 2; o > 0; o >>= 1) {
-    if (tid < o) sh[tid] += sh[tid + o];
+  if (!s_done) return;
+  // y = R^-1 s by columns, then scaled to the stored W_k
+  if (j < 32) {
+    // one warp, lane i holds row i: R's columns and the reciprocals of its
+    // diagonal loaded at once, then a product, a shuffle and an FMA a column
+    if (tid >= 32) return;
+    double R[32], y = tid <= j ? a.s[tid] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 32; k++) R[k] = k <= j && tid <= k ? a.H[(size_t)k * ld + tid] : 0.0;
+    const double rd = tid <= j ? 1.0 / a.H[(size_t)tid * ld + tid] : 0.0;
+#pragma unroll
+    for (int k = 31; k >= 0; k--) {
+      if (k > j) continue;
+      const double yk = __shfl_sync(0xffffffffu, y * rd, k);
+      y = tid == k ? yk : fma(-R[k], yk, y);
+    }
+    if (tid <= j) a.y[tid] = y * a.sc[tid];
+    return;
+  }
+  for (int k = tid; k <= j; k += T) col[k] = a.s[k];
+  __syncthreads();
+  for (int k = j; k >= 0; k--) {
+    const double *Hk = a.H + (size_t)k * ld;
+    if (tid == 0) col[k] = col[k] / Hk[k];
+    __syncthreads();
+    const double yk = col[k];
+    for (int i = tid; i < k; i += T) col[i] -= Hk[i] * yk;
     __syncthreads();
   }
-  if (tid != 0) return;
-  const int m = S.m, ld = m + 1;
-  const double hn = sqrt(sh[0]);
-  col[j + 1] = hn;
-  for (int k = 0; k < j; k++) {
-    const double x0 = col[k], x1 = col[k + 1];
-    col[k] = rc[k] * x0 + rs[k] * x1;
-    col[k + 1] = rc[k] * x1 - rs[k] * x0;
+  for (int k = tid; k <= j; k += T) a.y[k] = col[k] * a.sc[k];
+}
+
+// after the last step of a cycle (no further SpMV carries its logic)
+__global__ void __launch_bounds__(GM_T) gm_last_logic(GmArgs a, int j) {
+  if (a.alive[j]) gm_step_logic<GM_T>(a, j);
+}
+
+// W_{j+1} = D^-1 A W_j (the copy holds D^-1 A; the scale sc_j of V_j = sc_j W_j
+// is applied by the orthogonalisation), a slice per warp.  DOTS: and the
+// block partials of <W_k, W_{j+1}>, k <= j, from the rows in registers.  The
+// first block runs the logic of step j - 1 (the register bound keeps the
+// row blocks of the plain form at eight per SM; the logic may spill).
+template <int WARPS, bool DOTS, typename VT, typename CT>
+__global__ void __launch_bounds__(32 * WARPS, DOTS ? 1 : 8) gm_arnoldi_spmv(GmArgs a, const VT *__restrict__ sv,
+                                                                           const CT *__restrict__ scol, int j) {
+  if (!a.alive[j > 0 ? j - 1 : 0]) return;
+  int blk = blockIdx.x;
+  if (j > 0) {
+    if (blk == 0) {
+      gm_step_logic<32 * WARPS>(a, j - 1);
+      return;
+    }
+    blk--;
   }
-  const double x0 = col[j], x1 = col[j + 1];
-  const double rr = hypot(x0, x1), cj = x0 / rr, sj = x1 / rr;
-  col[j] = rr;
-  col[j + 1] = 0.0;
-  double *H = a.H + (size_t)j * ld;
-  for (int k = 0; k <= j + 1; k++) H[k] = col[k];
-  a.cs[j] = cj;
-  a.sn[j] = sj;
-  const double s0 = a.s[j];
-  a.s[j] = cj * s0;
-  const double s1 = -sj * s0;
-  a.s[j + 1] = s1;
-  const int it = S.it + 1;
-  const double resid = fabs(s1);
-  S.it = it;
-  S.resid = resid;
-  S.hn = hn;
-  a.sc[j + 1] = 1.0 / hn;
-  const bool conv = resid < S.tol_abs || resid / S.beta0 < S.tol_rel;
-  if (j == m - 1 || it >= S.max_iter || conv) {
-    S.done_cols = j + 1;  // the triangular solve runs in gm_update_x
-    S.final_flag = (conv || it >= S.max_iter) ? 1 : 0;
-    S.phase = GM_RESTART;
-  } else {
-    S.j = j + 1;
+  const int warp = threadIdx.x / 32, l = threadIdx.x & 31, s = blk * WARPS + warp, r = s * SELL_C + l;
+  if (!DOTS && s >= a.nslices) return;
+  double w = 0.0;
+  if (s < a.nslices) {
+    const int o = a.sell_off[s], wd = (a.sell_off[s + 1] - o) / SELL_C;
+    if constexpr (std::is_same<VT, float2>::value)
+      w = sell_row_dw(sv + o + l, scol + o + l, wd, sell_base(r, a.n), a.xdw);
+    else
+      w = sell_row<DOTS>(sv + o + l, scol + o + l, wd, sell_base(r, a.n), a.V + (size_t)j * a.n);
+    if (r < a.n) a.V[(size_t)(j + 1) * a.n + r] = w;
+    if (r >= a.n) w = 0.0;
+  }
+  if constexpr (DOTS) {
+    __shared__ double part[WARPS][GM_MMAX + 8];
+    const double *v = a.V + min(r, a.n - 1);
+    for (int k0 = 0; k0 <= j; k0 += 32) {
+      double x[32];  // all loads of up to 32 vectors in flight
+#pragma unroll
+      for (int u = 0; u < 32; u++)
+        if (k0 + u <= j) x[u] = __ldg(v + (size_t)(k0 + u) * a.n);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (k0 + 8 * q > j) break;
+        double t[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) t[u] = k0 + 8 * q + u <= j ? x[8 * q + u] * w : 0.0;
+        const double d = gm_warp_sums(t, l);
+        if ((l & 3) == 0) part[warp][k0 + 8 * q + (l >> 2)] = d;
+      }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k <= j; k += 32 * WARPS)
+      a.partial[(size_t)blk * (a.m + 1) + k] = gm_pairs<WARPS>(&part[0][k], GM_MMAX + 8);
   }
 }
 
-// w = W_{j+1} -= sum_k h_k sc_k W_k (one row a thread), the block partials
-// of its squared norm and its double-word copy for the next SpMV; the last
-// block to finish then runs the step's logic.
-__global__ void __launch_bounds__(GM_T) gm_orthogonalize(GmArgs a, int j) {
-  GmState &S = *a.st;
-  if (S.phase != GM_ARNOLDI || S.j != j) return;
-  __shared__ double coef[GM_MMAX + 1];
-  __shared__ bool last;
-  for (int k = threadIdx.x; k <= j; k += GM_T) coef[k] = a.hcol[k] * a.sc[k];
+// Block partials of <W_k, W_{j+1}>, k <= j: one block per SM takes an equal
+// share of the rows and all vectors, eight at a time (two rows' loads in
+// flight), so that a row costs one FMA a vector and the reductions are paid
+// once per thread and eight vectors.  W_{j+1} is read once per eight vectors
+// (L1 after the first).
+constexpr int GM_DOT_BLOCKS = 152, GM_DOT_T = 768;
+__global__ void __launch_bounds__(GM_DOT_T) gm_dots(GmArgs a, int j) {
+  if (!a.alive[j]) return;
+  constexpr int W = GM_DOT_T / 32, KP = 64;  // vectors between two barriers
+  __shared__ double part[W][KP];
+  const int lo = (int)((long long)a.n * blockIdx.x / gridDim.x), hi = (int)((long long)a.n * (blockIdx.x + 1) / gridDim.x);
+  const double *w = a.V + (size_t)(j + 1) * a.n;
+  for (int k0 = 0; k0 <= j; k0 += 8) {
+    const double *v = a.V + (size_t)k0 * a.n;
+    double t[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) t[u] = 0.0;
+    for (int i = lo + threadIdx.x; i < hi; i += 2 * GM_DOT_T) {
+      const bool two = i + GM_DOT_T < hi;
+      const double w0 = __ldg(w + i), w1 = two ? __ldg(w + i + GM_DOT_T) : 0.0;
+      double x[8], y[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        if (k0 + u <= j) {
+          x[u] = __ldg(v + (size_t)u * a.n + i);
+          y[u] = two ? __ldg(v + (size_t)u * a.n + i + GM_DOT_T) : 0.0;
+        }
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        if (k0 + u <= j) t[u] = fma(y[u], w1, fma(x[u], w0, t[u]));
+    }
+    const double d = gm_warp_sums(t, threadIdx.x & 31);
+    if ((threadIdx.x & 3) == 0) part[threadIdx.x / 32][k0 % KP + ((threadIdx.x & 31) >> 2)] = d;
+    if (k0 % KP == KP - 8 || k0 + 8 > j) {
+      const int kb = k0 / KP * KP;
+      __syncthreads();
+      if (threadIdx.x < KP && kb + threadIdx.x <= j)
+        a.partial[(size_t)blockIdx.x * (a.m + 1) + kb + threadIdx.x] = gm_pairs<W>(&part[0][threadIdx.x], KP);
+      __syncthreads();
+    }
+  }
+}
+
+// Sums of the dots' block partials: out[k] = sum over the nd blocks (in every
+// block of a small system's orthogonalisation, the same order in each).  Lanes take consecutive k of one
+// block's row, groups of lanes the rows in turn, eight rows in flight.
+template <int T>
+__device__ __forceinline__ void gm_sum_dots(const GmArgs &a, int j, double *out) {
+  __shared__ double red[T];
+  const int tid = threadIdx.x, ld = a.m + 1, rows = a.nd;
+  for (int kb = 0; kb <= j; kb += 32) {
+    const int nk = min(32, j + 1 - kb), kw = nk <= 8 ? 8 : nk <= 16 ? 16 : 32, G = T / kw, k = tid % kw, g = tid / kw;
+    const double *p = a.partial + kb + k;
+    double v = 0.0;
+    for (int r = g; r < rows; r += 8 * G) {
+      double x[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) x[u] = k < nk && r + u * G < rows ? __ldg(p + (size_t)(r + u * G) * ld) : 0.0;
+      v += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+    }
+    for (int o = kw; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((tid & 31) < kw) red[(tid >> 5) * 32 + (tid & 31)] = v;
+    __syncthreads();
+    if (tid < nk) out[kb + tid] = gm_pairs<T / 32>(red + tid, 32);
+    __syncthreads();
+  }
+}
+
+// sum_k c[k] V_k[i], U vectors' loads in flight, two accumulators (an FP64 FMA
+// waits long for the one before it)
+template <int U>
+__device__ __forceinline__ double gm_combine(const GmArgs &a, const double *c, int nk, long long i) {
+  double a0 = 0.0, a1 = 0.0;
+  const double *v = a.V + i;
+  for (int k = 0; k < nk; k += U) {
+    double x[U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (k + u < nk) x[u] = __ldg(v + (size_t)(k + u) * a.n);
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (k + u < nk) {
+        if (u & 1)
+          a1 = fma(c[k + u], x[u], a1);
+        else
+          a0 = fma(c[k + u], x[u], a0);
+      }
+  }
+  return a0 + a1;
+}
+
+// Large systems: the column entries h_k = <V_k, D^-1 A V_j> = sc_k sc_j <W_k,
+// W_{j+1}> by one block (summed by every block of the orthogonalisation, 760 of
+// them reading the same lines, they took 9 us more at 1,030,301 rows)
+constexpr int GM_SUM_T = 1024;
+__global__ void __launch_bounds__(GM_SUM_T) gm_column(GmArgs a, int j) {
+  if (!a.alive[j]) return;
+  __shared__ double t[GM_MMAX + 1];
+  gm_sum_dots<GM_SUM_T>(a, j, t);
+  for (int k = threadIdx.x; k <= j; k += GM_SUM_T) a.hcol[k] = a.sc[k] * (a.sc[j] * t[k]);
+}
+
+// W_{j+1} = sc_j W_{j+1} - sum_k h_k sc_k W_k, the block partials of its squared
+// norm and its double-word copy for the next SpMV.  SMALL: the column entries
+// first.  Otherwise (T = 256) five blocks fit an SM, and the grid is at most
+// that many (a second wave would leave most SMs idle).
+template <int T, bool SMALL>
+__global__ void __launch_bounds__(T, SMALL ? 1 : 5) gm_orthogonalize(GmArgs a, int j) {
+  if (!a.alive[j]) return;
+  __shared__ double coef[GM_MMAX + 1], sh[T / 32];
+  if constexpr (SMALL) gm_sum_dots<T>(a, j, coef);
+  const double scj = a.sc[j];
+  for (int k = threadIdx.x; k <= j; k += T) {
+    const double sk = a.sc[k], h = SMALL ? sk * (scj * coef[k]) : a.hcol[k];
+    if (SMALL && blockIdx.x == 0) a.hcol[k] = h;
+    coef[k] = h * sk;
+  }
   __syncthreads();
   double *w = a.V + (size_t)(j + 1) * a.n;
   double s = 0.0;
-  for (long long i = (long long)blockIdx.x * GM_T + threadIdx.x; i < a.n; i += (long long)gridDim.x * GM_T) {
-    double acc = 0.0;
-    for (int k = 0; k <= j; k++) acc = fma(coef[k], __ldg(a.V + (size_t)k * a.n + i), acc);
-    const double wi = w[i] - acc;
+  for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < a.n; i += (long long)gridDim.x * T) {
+    const double wi = fma(scj, w[i], -gm_combine<SMALL ? 32 : 8>(a, coef, j + 1, i));
     w[i] = wi;
     if (a.xdw) a.xdw[i] = dw_f2(wi);
     s = fma(wi, wi, s);
   }
-  s = gm_block_sum(s);
-  if (threadIdx.x == 0) {
-    a.npart[blockIdx.x] = s;
-    __threadfence();
-    last = atomicAdd(a.cnt + S.m + 1, 1u) == gridDim.x - 1;
-  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
   __syncthreads();
-  if (!last) return;
-  __threadfence();
-  if (threadIdx.x == 0) a.cnt[S.m + 1] = 0;  // for the next step
-  gm_step_logic(a, j, S);
+  if (threadIdx.x == 0) a.npart[blockIdx.x] = gm_pairs<T / 32>(sh, 1);
 }
 
-// At the end of a cycle: y from the triangular system R y = s (every block
-// solves it, the same arithmetic in each: thread 0 on a shared-memory copy
-// of R when the Krylov dimension is at most GM_RSTAGE, else on R in global
-// memory), then x += sum_k y_k V_k, one row a thread.
-__global__ void __launch_bounds__(GM_T) gm_update_x(GmArgs a) {
+// At the end of a cycle: x += sum_k y_k W_k (y from the last step's logic)
+template <int T>
+__global__ void __launch_bounds__(T, T == 256 ? 5 : 1) gm_update_x(GmArgs a) {
   const GmState &S = *a.st;
   if (S.phase != GM_RESTART || S.done_cols == 0) return;
-  __shared__ double R[GM_RSTAGE * GM_RSTAGE], yc[GM_MMAX + 1];
-  const int done = S.done_cols, ld = S.m + 1, tid = threadIdx.x;
-  const bool staged = done <= GM_RSTAGE;
-  if (staged)
-    for (int t = tid; t < done * done; t += GM_T) R[t] = a.H[(size_t)(t / done) * ld + t % done];  // column t / done
+  __shared__ double yc[GM_MMAX + 1];
+  const int done = S.done_cols;
+  for (int k = threadIdx.x; k < done; k += T) yc[k] = a.y[k];
   __syncthreads();
-  if (tid == 0) {
-    for (int k = done - 1; k >= 0; k--) {
-      double v = a.s[k];
-      if (staged)
-        for (int i = k + 1; i < done; i++) v -= R[i * done + k] * yc[i];
-      else
-        for (int i = k + 1; i < done; i++) v -= a.H[k + (size_t)i * ld] * yc[i];
-      yc[k] = v / (staged ? R[k * done + k] : a.H[k + (size_t)k * ld]);
-    }
-    for (int k = 0; k < done; k++) yc[k] *= a.sc[k];  // to the stored W_k
-  }
-  __syncthreads();
-  for (long long i = (long long)blockIdx.x * GM_T + tid; i < a.n; i += (long long)gridDim.x * GM_T) {
-    double acc = 0.0;
-    for (int k = 0; k < done; k++) acc = fma(yc[k], __ldg(a.V + (size_t)k * a.n + i), acc);
-    a.x[i] += acc;
-  }
+  for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < a.n; i += (long long)gridDim.x * T)
+    a.x[i] += gm_combine<T == 256 ? 8 : 32>(a, yc, done, i);
 }
 
 }  // namespace gbfem
@@ -513,6 +690,12 @@ using gbfem::GmState;
 namespace {
 
 unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
+
+// Up to here (slices of 32 rows; 38,912 rows) the dots run in the SpMV kernel:
+// below, an Arnoldi step is launches and memory latency (9,261 rows: 14 us a step
+// in two kernels; the three kernels with last-block tails before took 28).
+// 1,030,301 rows: 135 us a step on average over 30 (180 before).
+constexpr int GM_SMALL = 1216, GM_SMALL_WARPS = 4;
 
 // SELL-32 index arrays of the context's structure (once per structure)
 int build_sell(gbfem_ctx c) {
@@ -592,26 +775,41 @@ int capture_cycle(gbfem_ctx c, const GmArgs &a, int m, bool dword, int *kernels)
   gbfem::gm_logic_restart<<<1, gbfem::GM_T, 0, st>>>(a);
   gbfem::gm_start_cycle<<<gv, gbfem::GM_T, 0, st>>>(a);
   k += 4;
+  const bool small = ns <= GM_SMALL;
+  constexpr int W = gbfem::GM_T / 32, WS = GM_SMALL_WARPS;
+  auto spmv = [&](auto val, auto col, int j) {
+    if (small)
+      gbfem::gm_arnoldi_spmv<WS, true><<<nblk(ns, WS) + (j > 0), 32 * WS, 0, st>>>(a, val, col, j);
+    else
+      gbfem::gm_arnoldi_spmv<W, false><<<gs + (j > 0), gbfem::GM_T, 0, st>>>(a, val, col, j);
+  };
   for (int j = 0; j < m; j++) {
     if (j == 0) cudaEventRecordWithFlags(c->ev2, st, cudaEventRecordExternal);
-    if (dword) {
-      if (a.sell_col16)
-        gbfem::gm_arnoldi_spmv<<<gs, gbfem::GM_T, 0, st>>>(a, a.sell_valdw, a.sell_col16, j);
-      else
-        gbfem::gm_arnoldi_spmv<<<gs, gbfem::GM_T, 0, st>>>(a, a.sell_valdw, a.sell_col32, j);
-    } else {
-      if (a.sell_col16)
-        gbfem::gm_arnoldi_spmv<<<gs, gbfem::GM_T, 0, st>>>(a, a.sell_val64, a.sell_col16, j);
-      else
-        gbfem::gm_arnoldi_spmv<<<gs, gbfem::GM_T, 0, st>>>(a, a.sell_val64, a.sell_col32, j);
-    }
+    if (dword && a.sell_col16)
+      spmv(a.sell_valdw, a.sell_col16, j);
+    else if (dword)
+      spmv(a.sell_valdw, a.sell_col32, j);
+    else if (a.sell_col16)
+      spmv(a.sell_val64, a.sell_col16, j);
+    else
+      spmv(a.sell_val64, a.sell_col32, j);
     if (j == 0) cudaEventRecordWithFlags(c->ev3, st, cudaEventRecordExternal);
-    gbfem::gm_dot_partial<<<dim3(gv, j + 1), gbfem::GM_T, 0, st>>>(a, j);
-    gbfem::gm_orthogonalize<<<(unsigned)a.ng, gbfem::GM_T, 0, st>>>(a, j);
-    k += 3;
+    if (small) {
+      gbfem::gm_orthogonalize<32 * WS, true><<<(unsigned)a.ng, 32 * WS, 0, st>>>(a, j);
+      k += 2;
+    } else {
+      gbfem::gm_dots<<<gbfem::GM_DOT_BLOCKS, gbfem::GM_DOT_T, 0, st>>>(a, j);
+      gbfem::gm_column<<<1, gbfem::GM_SUM_T, 0, st>>>(a, j);
+      gbfem::gm_orthogonalize<gbfem::GM_T, false><<<(unsigned)a.ng, gbfem::GM_T, 0, st>>>(a, j);
+      k += 4;
+    }
   }
-  gbfem::gm_update_x<<<(unsigned)a.ng, gbfem::GM_T, 0, st>>>(a);
-  k += 1;
+  gbfem::gm_last_logic<<<1, gbfem::GM_T, 0, st>>>(a, m - 1);
+  if (small)
+    gbfem::gm_update_x<32 * WS><<<(unsigned)a.ng, 32 * WS, 0, st>>>(a);
+  else
+    gbfem::gm_update_x<gbfem::GM_T><<<(unsigned)a.ng, gbfem::GM_T, 0, st>>>(a);
+  k += 2;
   const cudaError_t e1 = cudaGetLastError();
   const cudaError_t e2 = cudaStreamEndCapture(st, &graph);
   GB_CUDA(e1);
@@ -639,17 +837,18 @@ int gmres_device_std(gbfem_ctx c, int krylov, int max_iter, double tol_rel, int 
   GB_TRY(launch_jacobi_diag(st, n, c->row_ptr.p, c->col_ind.p, c->val.p, c->dinv.p));
   GB_TRY(fill_sell_values(c));
   const int nb = reduction_blocks(n);
+  const bool small = (int)nblk(n, SELL_C) <= GM_SMALL;
+  const int dot_blocks = small ? (int)nblk(nblk(n, SELL_C), GM_SMALL_WARPS) : GM_DOT_BLOCKS;
   GB_TRY(c->V.alloc((size_t)n * (m + 1)));
   GB_TRY(c->x.alloc(n));
   GB_TRY(c->tmp.alloc(n));
-  GB_TRY(c->partial.alloc((size_t)nb * (m + 2)));
-  // row-parallel grid: one row a thread up to 8 blocks per SM (1,216 on
-  // GB300), beyond that a grid-stride loop (every block counts itself into
-  // one atomic word at the end of the step)
-  const int ng = (int)std::min<unsigned>(nblk(n, GM_T), 1216u);
+  GB_TRY(c->partial.alloc(std::max<size_t>((size_t)dot_blocks * (m + 1), nb)));
+  // blocks of the orthogonalisation: one row a thread, up to five blocks of 256
+  // threads per SM (all resident), beyond that a grid-stride loop
+  const int ng = (int)std::min<unsigned>(nblk(n, small ? 32 * GM_SMALL_WARPS : GM_T), 5u * 152u);
   GB_TRY(c->gm_npart.alloc((size_t)ng));
-  GB_TRY(c->gm_cnt.alloc((size_t)m + 2));
-  GB_CUDA(cudaMemsetAsync(c->gm_cnt.p, 0, ((size_t)m + 2) * sizeof(unsigned), st));
+  GB_TRY(c->gm_alive.alloc((size_t)m + 1));
+  GB_CUDA(cudaMemsetAsync(c->gm_alive.p, 0, ((size_t)m + 1) * sizeof(int), st));
   // H (m+1)^2, cs, sn, s (m+1 each), y (m), hcol (m+1), sc (m+1), state
   const size_t nsmall = (size_t)(m + 1) * (m + 1) + 3 * (size_t)(m + 1) + m + 2 * (size_t)(m + 1) + 16;
   GB_TRY(c->gm_small.alloc(nsmall));
@@ -684,7 +883,9 @@ int gmres_device_std(gbfem_ctx c, int krylov, int max_iter, double tol_rel, int 
   a.partial = c->partial.p;
   a.ng = ng;
   a.npart = c->gm_npart.p;
-  a.cnt = c->gm_cnt.p;
+  a.m = m;
+  a.nd = dot_blocks;
+  a.alive = c->gm_alive.p;
   if (c->std_spmv_dword) {
     GB_TRY(c->gm_xdw.alloc(n));
     a.xdw = c->gm_xdw.p;
@@ -715,8 +916,10 @@ int gmres_device_std(gbfem_ctx c, int krylov, int max_iter, double tol_rel, int 
     memcpy(c->gm_key_args, &a, sizeof(a));
     c->gm_kernels = kernels_per_cycle;
   }
-  GmState *hs = nullptr;
-  GB_CUDA(cudaMallocHost(&hs, sizeof(GmState)));
+  // the page-locked copy of the state lives with the context (allocating it
+  // here cost some 0.2 ms a solve)
+  if (!c->gm_host) GB_CUDA(cudaMallocHost(&c->gm_host, sizeof(GmState)));
+  GmState *hs = static_cast<GmState *>(c->gm_host);
   float spmv_ms = 0.f;
   int spmv_n = 0, cycles = 0, it_prev = 0;
   cudaEventRecord(c->ev0, st);
@@ -742,7 +945,6 @@ int gmres_device_std(gbfem_ctx c, int krylov, int max_iter, double tol_rel, int 
   }
   cudaEventRecord(c->ev1, st);
   const GmState fin = *hs;
-  cudaFreeHost(hs);
   GB_TRY(rc);
   GB_CUDA(cudaMemcpyAsync(x, c->x.p, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st));
   GB_CUDA(cudaStreamSynchronize(st));
