@@ -110,6 +110,20 @@ static int fetch_host_structure(gbfem_ctx c) {
   return 0;
 }
 
+// Inverts every diagonal block into c->dg_dinv on the context stream, one
+// launch per element class; returns the launches.
+int gbfem::dg_invert_diagonal(gbfem_ctx c) {
+  int n = 0;
+  for (int cls = 1; cls <= 8; cls++) {
+    if (!c->dg_list[cls].p) continue;
+    const int r = launch_dg_block_inverse(c->stream, cls, (int)c->dg_list[cls].n, c->dg_list[cls].p,
+                                          c->dg_boff_diag_d.p, c->dg_val.p, c->dg_dinv_off_d.p, c->dg_dinv.p, c->err.p);
+    if (r < 0) return r;
+    n += r;
+  }
+  return n;
+}
+
 // Block SpMV over all DG block rows, one launch per element class (1..4:
 // prisms of degree 1..4, 5..8: tetrahedra of degree 1..4).
 static int dg_spmv(gbfem_ctx c, int mode, const double *x, const double *b, double *out) {
@@ -2227,13 +2241,13 @@ int gbfem_dg_solve(gbfem_ctx c, int krylov, int max_iter, double tol_rel, int in
   cudaStream_t st = c->stream;
   GB_TRY(c->dg_dinv.alloc((size_t)c->dg_ninv));
   GB_CUDA(cudaMemsetAsync(c->err.p, 0, sizeof(int), st));
-  GB_TRY(gbfem::launch_dg_block_inverse(st, c->nel, c->dg_roff_d.p, c->dg_boff_diag_d.p, c->dg_val.p,
-                                        c->dg_dinv_off_d.p, c->dg_dinv.p, c->err.p));
+  const int ninv = gbfem::dg_invert_diagonal(c);
+  GB_TRY(ninv);
   int herr = 0;
   GB_CUDA(cudaMemcpyAsync(&herr, c->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   GB_CUDA(cudaStreamSynchronize(st));
   GB_CHECK(herr == 0, "singular diagonal block in the DG block Jacobi preconditioner");
-  c->last_solve_kernels = 1;
+  c->last_solve_kernels = ninv;
   if (c->dg_spmv_dword) {
     // double-word copies of the matrix and of the inverted diagonal blocks
     // for the Arnoldi products; the restart residuals stay FP64
@@ -2290,8 +2304,7 @@ int gbfem_dg_solve_ir(gbfem_ctx c, int krylov, int max_iter, double tol_rel, dou
   // preconditioner in FP64, then FP32 copies of it and of the matrix
   GB_TRY(c->dg_dinv.alloc((size_t)c->dg_ninv));
   GB_CUDA(cudaMemsetAsync(c->err.p, 0, sizeof(int), st));
-  GB_TRY(gbfem::launch_dg_block_inverse(st, c->nel, c->dg_roff_d.p, c->dg_boff_diag_d.p, c->dg_val.p,
-                                        c->dg_dinv_off_d.p, c->dg_dinv.p, c->err.p));
+  GB_TRY(gbfem::dg_invert_diagonal(c));
   GB_TRY(c->dg_val32.alloc((size_t)c->dg_nval));
   GB_TRY(c->dg_dinv32.alloc((size_t)c->dg_ninv));
   GB_TRY(gbfem::launch_to_float(st, c->dg_nval, c->dg_val.p, c->dg_val32.p));

@@ -39,6 +39,8 @@
 #include "dg_face.cuh"
 #include "gbfem_internal.h"
 
+#include <mutex>
+
 namespace gbfem {
 
 __device__ const double m_fq[GB_DG_PMAX][2][GB_DG_MAXNQF][3] = GB_DG_FQ_INIT;
@@ -71,6 +73,7 @@ struct DgFaceTables {
 
 static DgFaceTables g_fm[64];
 static bool g_fm_ready[64];
+static std::mutex g_fm_lock;  // contexts are made and used from several threads
 
 // moments of a diagonal block: M0 [T(2P)][2P+1], M1, M2 [T(2P-1)][2P+1], M3 [T(2P)][2P]
 template <int P>
@@ -83,6 +86,7 @@ struct FmDiag {
 
 static int fm_tables(int device, DgFaceTables *out) {
   GB_CHECK(device >= 0 && device < 64, "device index out of range");
+  std::lock_guard<std::mutex> hold(g_fm_lock);
   if (!g_fm_ready[device]) {
     static const double FQ[GB_DG_PMAX][2][GB_DG_MAXNQF][3] = GB_DG_FQ_INIT;
     std::vector<double> Z(4 * FM_Q1 * FM_ZP, 0.0), XE(4 * FM_MONO * FM_Q1, 0.0), XT(4 * 9 * FM_MONO * FM_QT, 0.0);

@@ -13,10 +13,13 @@
 #include "dg_volume.cuh"
 #include "prism_std.cuh"
 
+#include <mutex>
+
 namespace gbfem {
 
 static DgDeviceTables g_dg_tables[64];
 static bool g_dg_tables_ready[64] = {false};
+static std::mutex g_dg_tables_lock;  // contexts are made and used from several threads
 
 // The volume kernel's tables for degree p (layouts in dg_volume.cuh): point
 // rule QP, monomials and line-point powers VT, entries ENT (upper triangle row by
@@ -74,6 +77,7 @@ static void host_dg_tables(int p, std::vector<double> &QP, std::vector<double> &
 
 int dg_tables_for_device(int device, DgDeviceTables **out) {
   GB_CHECK(device >= 0 && device < 64, "device index out of range");
+  std::lock_guard<std::mutex> hold(g_dg_tables_lock);
   if (!g_dg_tables_ready[device]) {
     for (int p = 1; p <= GB_DG_PMAX; p++) {
       std::vector<double> QP, VT;

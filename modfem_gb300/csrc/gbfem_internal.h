@@ -246,8 +246,10 @@ int launch_dg_prism_faces(cudaStream_t st, int p, int count, const int *ent_el, 
                           const int *roff, double *val, double *rhs, int variant, bool dword = false, bool low = false);
 // Variable-block CRS (one block row per DG element, dense column-major
 // blocks with the row block's size as leading dimension) and block Jacobi.
-int launch_dg_block_inverse(cudaStream_t st, int nel, const int *roff, const long long *boff_diag,
+// (inverts the diagonal blocks of the count elements of one class)
+int launch_dg_block_inverse(cudaStream_t st, int cls, int count, const int *ent_el, const long long *boff_diag,
                             const double *val, const long long *dinv_off, double *dinv, int *err);
+int dg_invert_diagonal(gbfem_ctx c);  // every class of a context (api.cu)
 // mode 0: out = Minv (b - A x) (b may be NULL), 1: out = Minv A x,
 // 2: out = (b ? b : 0) - A x (Minv unused); rows of the count elements of
 // degree p listed in ent_el.  row_val[e]: value offset of block row e (its

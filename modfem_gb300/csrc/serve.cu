@@ -607,9 +607,7 @@ int prepare(gbfem_server s, SrvRequest &r) {
     r.n = nd;
     if ((rc = c->dg_dinv.alloc((size_t)c->dg_ninv)) < 0) return rc;
     cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream);
-    if ((rc = gbfem::launch_dg_block_inverse(c->stream, c->nel, c->dg_roff_d.p, c->dg_boff_diag_d.p, c->dg_val.p,
-                                             c->dg_dinv_off_d.p, c->dg_dinv.p, c->err.p)) < 0)
-      return rc;
+    if ((rc = gbfem::dg_invert_diagonal(c)) < 0) return rc;
     int herr = 0;
     cudaMemcpyAsync(&herr, c->err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess || herr != 0) {
