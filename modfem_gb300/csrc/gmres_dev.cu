@@ -50,6 +50,7 @@
 
 #include "dword.cuh"
 #include "gbfem_internal.h"
+#include "gmres_step.cuh"
 
 namespace gbfem {
 
@@ -344,142 +345,33 @@ __global__ void __launch_bounds__(GM_T) gm_start_cycle(GmArgs a) {
   }
 }
 
-// Sums of eight values over a warp: afterwards lane l holds the sum of value
-// l / 4.  Each exchange halves the values a lane keeps: 9 adds instead of 40.
-__device__ __forceinline__ double gm_warp_sums(double (&t)[8], int lane) {
-#pragma unroll
-  for (int h = 4, o = 16; h >= 1; h >>= 1, o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int u = 0; u < h; u++) {
-      const double send = up ? t[u] : t[u + h], keep = up ? t[u + h] : t[u];
-      t[u] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  double v = t[0];
-  v += __shfl_xor_sync(0xffffffffu, v, 2);
-  v += __shfl_xor_sync(0xffffffffu, v, 1);
-  return v;
-}
-
-// pairwise sum of N shared values at stride `st` (short chain of dependent adds)
-template <int N>
-__device__ __forceinline__ double gm_pairs(const double *p, int st) {
-  if constexpr (N == 1)
-    return p[0];
-  else
-    return gm_pairs<N / 2>(p, st) + gm_pairs<N - N / 2>(p + (N / 2) * st, st);
-}
-
-// The step's logic for step j (one block of T threads): |w| from the norm
-// partials, the earlier rotations applied to the Hessenberg column (the chain
-// c_{k+1} = rc_k h_{k+1} - rs_k c_k composes affine maps by a warp scan, 5 steps
-// per 32 rotations: an FP64 operation takes tens of cycles), the new rotation,
-// the residual estimate and the decision (next step, or end of the cycle,
-// where the block also solves R y = s by columns).
+// the logic of step j on the solver's state
 template <int T>
-__device__ void gm_step_logic(const GmArgs &a, int j) {
-  __shared__ double col[GM_MMAX + 2];
-  __shared__ double sh[T / 32];
-  __shared__ int s_done;
-  GmState &S = *a.st;
-  const int tid = threadIdx.x, m = a.m, ld = m + 1;
-  double v = 0.0;
-  for (int b = tid; b < a.ng; b += 4 * T) {
-    double x[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) x[u] = b + u * T < a.ng ? a.npart[b + u * T] : 0.0;
-    v += (x[0] + x[1]) + (x[2] + x[3]);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((tid & 31) == 0) sh[tid >> 5] = v;
-  __syncthreads();
-  if (tid < 32) {
-    double *H = a.H + (size_t)j * ld;
-    double c = a.hcol[0];
-    for (int k0 = 0; k0 < j; k0 += 32) {
-      const int k = k0 + tid;
-      const double rc = k < j ? a.cs[k] : 1.0, rs = k < j ? a.sn[k] : 0.0, hk = k < j ? a.hcol[k + 1] : 0.0;
-      double A = k < j ? -rs : 1.0, B = rc * hk;  // (identity beyond the last rotation)
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const double A1 = __shfl_up_sync(0xffffffffu, A, o), B1 = __shfl_up_sync(0xffffffffu, B, o);
-        if (tid >= o) {
-          B = fma(A, B1, B);
-          A *= A1;
-        }
-      }
-      const double next = fma(A, c, B);  // c_{k+1}
-      double prev = __shfl_up_sync(0xffffffffu, next, 1);
-      if (tid == 0) prev = c;
-      if (k < j) H[k] = fma(rc, prev, rs * hk);
-      c = __shfl_sync(0xffffffffu, next, 31);
+__device__ __forceinline__ void gm_logic(const GmArgs &a, int j) {
+  const GmStep g = {a.m, a.ng, 1, a.npart, a.H, a.cs, a.sn, a.s, a.y, a.hcol, a.sc};
+  gm_step_logic<T, GM_MMAX>(g, j, [&](double resid, double hn) -> int {
+    GmState &S = *a.st;
+    const int it = S.it + 1;
+    S.it = it;
+    S.resid = resid;
+    S.hn = hn;
+    const bool conv = resid < S.tol_abs || resid / S.beta0 < S.tol_rel;
+    const bool end = j == a.m - 1 || it >= S.max_iter || conv;
+    if (end) {
+      S.done_cols = j + 1;
+      S.final_flag = (conv || it >= S.max_iter) ? 1 : 0;
+      S.phase = GM_RESTART;
+    } else {
+      S.j = j + 1;
+      a.alive[j + 1] = 1;
     }
-    if (tid == 0) {
-      const double h2 = gm_pairs<T / 32>(sh, 1), hn = sqrt(h2);
-      const double rr = hypot(c, hn), cj = c / rr, sj = hn / rr;
-      H[j] = rr;
-      H[j + 1] = 0.0;
-      a.cs[j] = cj;
-      a.sn[j] = sj;
-      const double s0 = a.s[j], s1 = -sj * s0, resid = fabs(s1);
-      a.s[j] = cj * s0;
-      a.s[j + 1] = s1;
-      const int it = S.it + 1;
-      S.it = it;
-      S.resid = resid;
-      S.hn = hn;
-      a.sc[j + 1] = 1.0 / hn;
-      const bool conv = resid < S.tol_abs || resid / S.beta0 < S.tol_rel;
-      const bool end = j == m - 1 || it >= S.max_iter || conv;
-      s_done = end;
-      if (end) {
-        S.done_cols = j + 1;
-        S.final_flag = (conv || it >= S.max_iter) ? 1 : 0;
-        S.phase = GM_RESTART;
-      } else {
-        S.j = j + 1;
-        a.alive[j + 1] = 1;
-      }
-    }
-  }
-  __syncthreads();
-  if (!s_done) return;
-  // y = R^-1 s by columns, then scaled to the stored W_k
-  if (j < 32) {
-    // one warp, lane i holds row i: R's columns and the reciprocals of its
-    // diagonal loaded at once, then a product, a shuffle and an FMA a column
-    if (tid >= 32) return;
-    double R[32], y = tid <= j ? a.s[tid] : 0.0;
-#pragma unroll
-    for (int k = 0; k < 32; k++) R[k] = k <= j && tid <= k ? a.H[(size_t)k * ld + tid] : 0.0;
-    const double rd = tid <= j ? 1.0 / a.H[(size_t)tid * ld + tid] : 0.0;
-#pragma unroll
-    for (int k = 31; k >= 0; k--) {
-      if (k > j) continue;
-      const double yk = __shfl_sync(0xffffffffu, y * rd, k);
-      y = tid == k ? yk : fma(-R[k], yk, y);
-    }
-    if (tid <= j) a.y[tid] = y * a.sc[tid];
-    return;
-  }
-  for (int k = tid; k <= j; k += T) col[k] = a.s[k];
-  __syncthreads();
-  for (int k = j; k >= 0; k--) {
-    const double *Hk = a.H + (size_t)k * ld;
-    if (tid == 0) col[k] = col[k] / Hk[k];
-    __syncthreads();
-    const double yk = col[k];
-    for (int i = tid; i < k; i += T) col[i] -= Hk[i] * yk;
-    __syncthreads();
-  }
-  for (int k = tid; k <= j; k += T) a.y[k] = col[k] * a.sc[k];
+    return end;
+  });
 }
 
 // after the last step of a cycle (no further SpMV carries its logic)
 __global__ void __launch_bounds__(GM_T) gm_last_logic(GmArgs a, int j) {
-  if (a.alive[j]) gm_step_logic<GM_T>(a, j);
+  if (a.alive[j]) gm_logic<GM_T>(a, j);
 }
 
 // W_{j+1} = D^-1 A W_j (the copy holds D^-1 A; the scale sc_j of V_j = sc_j W_j
@@ -494,7 +386,7 @@ __global__ void __launch_bounds__(32 * WARPS, DOTS ? 1 : 8) gm_arnoldi_spmv(GmAr
   int blk = blockIdx.x;
   if (j > 0) {
     if (blk == 0) {
-      gm_step_logic<32 * WARPS>(a, j - 1);
+      gm_logic<32 * WARPS>(a, j - 1);
       return;
     }
     blk--;
@@ -578,54 +470,6 @@ __global__ void __launch_bounds__(GM_DOT_T) gm_dots(GmArgs a, int j) {
   }
 }
 
-// Sums of the dots' block partials: out[k] = sum over the nd blocks (in every
-// block of a small system's orthogonalisation, the same order in each).  Lanes take consecutive k of one
-// block's row, groups of lanes the rows in turn, eight rows in flight.
-template <int T>
-__device__ __forceinline__ void gm_sum_dots(const GmArgs &a, int j, double *out) {
-  __shared__ double red[T];
-  const int tid = threadIdx.x, ld = a.m + 1, rows = a.nd;
-  for (int kb = 0; kb <= j; kb += 32) {
-    const int nk = min(32, j + 1 - kb), kw = nk <= 8 ? 8 : nk <= 16 ? 16 : 32, G = T / kw, k = tid % kw, g = tid / kw;
-    const double *p = a.partial + kb + k;
-    double v = 0.0;
-    for (int r = g; r < rows; r += 8 * G) {
-      double x[8];
-#pragma unroll
-      for (int u = 0; u < 8; u++) x[u] = k < nk && r + u * G < rows ? __ldg(p + (size_t)(r + u * G) * ld) : 0.0;
-      v += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
-    }
-    for (int o = kw; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((tid & 31) < kw) red[(tid >> 5) * 32 + (tid & 31)] = v;
-    __syncthreads();
-    if (tid < nk) out[kb + tid] = gm_pairs<T / 32>(red + tid, 32);
-    __syncthreads();
-  }
-}
-
-// sum_k c[k] V_k[i], U vectors' loads in flight, two accumulators (an FP64 FMA
-// waits long for the one before it)
-template <int U>
-__device__ __forceinline__ double gm_combine(const GmArgs &a, const double *c, int nk, long long i) {
-  double a0 = 0.0, a1 = 0.0;
-  const double *v = a.V + i;
-  for (int k = 0; k < nk; k += U) {
-    double x[U];
-#pragma unroll
-    for (int u = 0; u < U; u++)
-      if (k + u < nk) x[u] = __ldg(v + (size_t)(k + u) * a.n);
-#pragma unroll
-    for (int u = 0; u < U; u++)
-      if (k + u < nk) {
-        if (u & 1)
-          a1 = fma(c[k + u], x[u], a1);
-        else
-          a0 = fma(c[k + u], x[u], a0);
-      }
-  }
-  return a0 + a1;
-}
-
 // Large systems: the column entries h_k = <V_k, D^-1 A V_j> = sc_k sc_j <W_k,
 // W_{j+1}> by one block (summed by every block of the orthogonalisation, 760 of
 // them reading the same lines, they took 9 us more at 1,030,301 rows)
@@ -633,7 +477,7 @@ constexpr int GM_SUM_T = 1024;
 __global__ void __launch_bounds__(GM_SUM_T) gm_column(GmArgs a, int j) {
   if (!a.alive[j]) return;
   __shared__ double t[GM_MMAX + 1];
-  gm_sum_dots<GM_SUM_T>(a, j, t);
+  gm_sum_dots<GM_SUM_T>(a.partial, a.nd, a.m + 1, j, t);
   for (int k = threadIdx.x; k <= j; k += GM_SUM_T) a.hcol[k] = a.sc[k] * (a.sc[j] * t[k]);
 }
 
@@ -645,7 +489,7 @@ template <int T, bool SMALL>
 __global__ void __launch_bounds__(T, SMALL ? 1 : 5) gm_orthogonalize(GmArgs a, int j) {
   if (!a.alive[j]) return;
   __shared__ double coef[GM_MMAX + 1], sh[T / 32];
-  if constexpr (SMALL) gm_sum_dots<T>(a, j, coef);
+  if constexpr (SMALL) gm_sum_dots<T>(a.partial, a.nd, a.m + 1, j, coef);
   const double scj = a.sc[j];
   for (int k = threadIdx.x; k <= j; k += T) {
     const double sk = a.sc[k], h = SMALL ? sk * (scj * coef[k]) : a.hcol[k];
@@ -656,7 +500,7 @@ __global__ void __launch_bounds__(T, SMALL ? 1 : 5) gm_orthogonalize(GmArgs a, i
   double *w = a.V + (size_t)(j + 1) * a.n;
   double s = 0.0;
   for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < a.n; i += (long long)gridDim.x * T) {
-    const double wi = fma(scj, w[i], -gm_combine<SMALL ? 32 : 8>(a, coef, j + 1, i));
+    const double wi = fma(scj, w[i], -gm_combine<SMALL ? 32 : 8>(a.V, a.n, coef, j + 1, i));
     w[i] = wi;
     if (a.xdw) a.xdw[i] = dw_f2(wi);
     s = fma(wi, wi, s);
@@ -678,7 +522,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 5 : 1) gm_update_x(GmArgs a) {
   for (int k = threadIdx.x; k < done; k += T) yc[k] = a.y[k];
   __syncthreads();
   for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < a.n; i += (long long)gridDim.x * T)
-    a.x[i] += gm_combine<T == 256 ? 8 : 32>(a, yc, done, i);
+    a.x[i] += gm_combine<T == 256 ? 8 : 32>(a.V, a.n, yc, done, i);
 }
 
 }  // namespace gbfem

@@ -28,11 +28,14 @@
 //    advances each of its active requests by one GMRES iteration with
 //    batched kernels over all of them - one CRS SpMV launch for all std
 //    requests, one launch per degree class for each DG request, and one
-//    launch each for the Gram-Schmidt dot products, updates and norms.  The scalar GMRES logic
-//    (Hessenberg column, Givens rotations, convergence test, restart and the
-//    small triangular solve) runs on the device per request, so a step needs
-//    no host round trip per request; the host reads the requests' phases once
-//    per step to retire finished ones and admit new ones between steps.
+//    launch each for the Gram-Schmidt dot products, the orthogonalisation and
+//    the scalar GMRES logic (Hessenberg column, Givens rotations, convergence
+//    test, restart and the small triangular solve, one block a request), so a
+//    step needs no host round trip per request; the host reads the requests'
+//    phases every few steps to retire finished ones and admit new ones
+//    between steps.  What a step does for a request depends on its phase:
+//    residual at a restart, Arnoldi step, or update of x at the end of a
+//    cycle (a cycle of m Arnoldi steps takes m + 2 engine steps).
 //
 // Assembly is deterministic (the gather scatter for std requests, one
 // owning thread per block entry for DG) and every request's reductions are
@@ -41,8 +44,10 @@
 // the same bits alone and in a mix.
 //
 // The kernel sequence of a lane's step depends only on its set of active
-// requests (their state lives on the device), so it is captured once per
-// change of that set as a CUDA graph and replayed every step.
+// requests (their state lives on the device): it is launched kernel by kernel
+// after a change of that set, and once the set has stood for some polls it is
+// captured as a CUDA graph and replayed every step (a capture costs as much as
+// dozens of steps' launches; in a burst the set changes every few steps).
 
 #include <algorithm>
 #include <atomic>
@@ -58,6 +63,7 @@
 
 #include "dg_spmv.cuh"
 #include "gbfem_internal.h"
+#include "gmres_step.cuh"
 
 namespace gbfem {
 
@@ -65,12 +71,16 @@ constexpr int SRV_MAXSLOTS = 64;
 constexpr int SRV_MMAX = 64;              // largest Krylov dimension of a served request
 constexpr int SRV_PART = SRV_MMAX + 2;    // per reduction block: dots 0..m, norm at SRV_MMAX + 1
 constexpr int SRV_T = 256;
-constexpr int SRV_PER = 8;
-constexpr int SRV_CHUNK = SRV_T * SRV_PER;  // vector entries per BLAS-1 block
-constexpr int SRV_SPMV_LANES = 4;
+constexpr int SRV_SPMV_LANES = 8;         // a prism row's 21 entries: three rounds
 constexpr int SRV_SPMV_ROWS = SRV_T / SRV_SPMV_LANES;
+constexpr int SRV_RED = 160;              // reduction blocks of a request at most
+// Entries per reduction block of a request of n unknowns: one a thread (the step
+// of a small request is memory latency) until the blocks are SRV_RED, since
+// every block of the orthogonalisation sums the partials of all.  By the
+// request's size only, so its sums are the same in every mix.
+constexpr int srv_chunk(int n) { return SRV_T * ((n + SRV_T * SRV_RED - 1) / (SRV_T * SRV_RED)); }
 
-enum { PH_RESTART = 0, PH_ARNOLDI = 1, PH_DONE = 2 };
+enum { PH_RESTART = 0, PH_ARNOLDI = 1, PH_DONE = 2, PH_UPDATE = 3 };
 
 // host-written description of an active request
 struct SrvDesc {
@@ -83,259 +93,200 @@ struct SrvDesc {
   const long long *row_val, *cx_off, *dinv_off;
   const double *dgval, *dgdinv;
   const double *b;
-  double *x, *V, *tmp, *H, *cs, *sn, *s, *y, *hcol;
-  int red_first, red_nb;
+  double *x, *V, *tmp, *H, *cs, *sn, *s, *y, *hcol, *sc;
+  int red_first, red_nb, chunk;
 };
 
 // device-written GMRES state of a request
 struct SrvState {
-  int phase, j, it, done_cols, final_flag, fresh, wscale, widx;
-  double beta0, resid, beta, hn;
+  int phase, j, it, done_cols, final_flag, pad[3];
+  double beta0, resid;
 };
 
-__device__ __forceinline__ double srv_block_sum(double s) {
-  __shared__ double sh[SRV_T / 32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-  __syncthreads();
-  s = 0.0;
-  if (threadIdx.x < 32) {
-    s = threadIdx.x < SRV_T / 32 ? sh[threadIdx.x] : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  }
-  return s;  // valid in thread 0
-}
-
-// x += V[:, :done] y at a restart
-__global__ void __launch_bounds__(SRV_T) srv_update_x(const int2 *map, const SrvDesc *dd, const SrvState *ss) {
-  const int2 mp = map[blockIdx.x];
-  const SrvDesc &D = dd[mp.x];
-  const SrvState &S = ss[mp.x];
-  if (S.phase != PH_RESTART || S.done_cols == 0) return;
-  for (int t = 0; t < SRV_PER; t++) {
-    const long long i = (long long)mp.y + t * SRV_T + threadIdx.x;
-    if (i >= D.n) break;
-    double a = 0.0;
-    for (int k = 0; k < S.done_cols; k++) a = fma(D.y[k], D.V[(size_t)k * D.n + i], a);
-    D.x[i] = fma(1.0, a, D.x[i]);
-  }
-}
-
-// CRS rows of the std requests: MODE 0 tmp = dinv (b - A x) for restarting
-// requests, MODE 1 V[j+1] = dinv A V[j] for requests in an Arnoldi step.
-template <int MODE>
+// CRS rows of the std requests: restart residual tmp = dinv (b - A x), or
+// W_{j+1} = dinv A W_j in an Arnoldi step.
 __global__ void __launch_bounds__(SRV_T) srv_crs_spmv(const int2 *map, const SrvDesc *dd, const SrvState *ss) {
   const int2 mp = map[blockIdx.x];
   const SrvDesc &D = dd[mp.x];
   const SrvState &S = ss[mp.x];
-  const bool act = MODE == 0 ? (S.phase == PH_RESTART && !S.final_flag) : S.phase == PH_ARNOLDI;
-  if (!act) return;  // uniform over the block
+  const bool restart = S.phase == PH_RESTART;
+  if (!restart && S.phase != PH_ARNOLDI) return;  // uniform over the block
   const int lane = threadIdx.x & (SRV_SPMV_LANES - 1);
   const long long r = (long long)mp.y + threadIdx.x / SRV_SPMV_LANES;
   const bool valid = r < D.n;
-  const double *x = MODE == 0 ? D.x : D.V + (size_t)S.j * D.n;
-  double *out = MODE == 0 ? D.tmp : D.V + (size_t)(S.j + 1) * D.n;
+  const double *x = restart ? D.x : D.V + (size_t)S.j * D.n;
+  double *out = restart ? D.tmp : D.V + (size_t)(S.j + 1) * D.n;
   const int lo = valid ? D.row_ptr[r] : 0, hi = valid ? D.row_ptr[r + 1] : 0;
   double s = 0.0;
-  for (int k = lo + lane; k < hi; k += SRV_SPMV_LANES) s = fma(D.val[k], x[D.col_ind[k]], s);
+  for (int k = lo + lane; k < hi; k += 4 * SRV_SPMV_LANES) {  // up to 32 entries of a row in flight
+    double a[4], xv[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int q = k + u * SRV_SPMV_LANES;
+      a[u] = q < hi ? D.val[q] : 0.0;
+      xv[u] = q < hi ? x[D.col_ind[q]] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (k + u * SRV_SPMV_LANES < hi) s = fma(a[u], xv[u], s);
+  }
 #pragma unroll
   for (int o = SRV_SPMV_LANES / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, SRV_SPMV_LANES);
-  if (valid && lane == 0) out[r] = MODE == 0 ? (D.b[r] - s) * D.dinv[r] : D.dinv[r] * s;
+  if (valid && lane == 0) out[r] = restart ? (D.b[r] - s) * D.dinv[r] : D.dinv[r] * s;
 }
 
-// the block rows of degree P of one DG request (same two modes)
-template <int P, int MODE>
+// the block rows of degree P of one DG request (the same two forms)
+template <int P>
 __global__ void __launch_bounds__(DGS_THREADS) srv_dg_spmv(int slot, int count, const int *ent_el,
                                                            const SrvDesc *dd, const SrvState *ss) {
-  __shared__ double sv[DGS_ROWS][DgSpmvDims<P>::NS];
   const SrvDesc &D = dd[slot];
   const SrvState &S = ss[slot];
-  const bool act = MODE == 0 ? (S.phase == PH_RESTART && !S.final_flag) : S.phase == PH_ARNOLDI;
-  if (!act) return;
-  const double *x = MODE == 0 ? D.x : D.V + (size_t)S.j * D.n;
-  double *out = MODE == 0 ? D.tmp : D.V + (size_t)(S.j + 1) * D.n;
-  dg_block_row_spmv<P>(MODE == 0 ? 0 : 1, count, ent_el, D.roff, D.row_val, D.cx_off, D.colx, D.dgval, D.dinv_off,
-                       D.dgdinv, x, MODE == 0 ? D.b : nullptr, out, sv);
+  const bool restart = S.phase == PH_RESTART;
+  if (!restart && S.phase != PH_ARNOLDI) return;
+  const double *x = restart ? D.x : D.V + (size_t)S.j * D.n, *b = restart ? D.b : nullptr;
+  double *out = restart ? D.tmp : D.V + (size_t)(S.j + 1) * D.n;
+  __shared__ double sv[DGS_ROWS][DgSpmvDims<P>::NS];
+  dg_block_row_spmv<P>(restart ? 0 : 1, count, ent_el, D.roff, D.row_val, D.cx_off, D.colx, D.dgval, D.dinv_off,
+                       D.dgdinv, x, b, out, sv);
 }
 
-// per-block sum of squares: WHICH 0 the restart residual tmp, 1 the new
-// Arnoldi vector V[j+1]
-template <int WHICH>
-__global__ void __launch_bounds__(SRV_T) srv_norm_partial(const int2 *map, const SrvDesc *dd, const SrvState *ss,
-                                                          double *partial) {
+// Block partials of <W_k, W_{j+1}>, k <= j, or of <tmp, tmp> at a restart:
+// sixteen vectors at a time, so that a small request (one row a thread) waits
+// for memory once per sixteen.
+__global__ void __launch_bounds__(SRV_T) srv_dots(const int2 *map, const SrvDesc *dd, const SrvState *ss,
+                                                  double *partial) {
+  constexpr int W = SRV_T / 32, KP = SRV_MMAX;
+  __shared__ double part[W][KP];
   const int2 mp = map[blockIdx.x];
   const SrvDesc &D = dd[mp.x];
   const SrvState &S = ss[mp.x];
-  const bool act = WHICH == 0 ? (S.phase == PH_RESTART && !S.final_flag) : S.phase == PH_ARNOLDI;
-  if (!act) return;
-  const double *v = WHICH == 0 ? D.tmp : D.V + (size_t)(S.j + 1) * D.n;
-  double s = 0.0;
-  for (int t = 0; t < SRV_PER; t++) {
-    const long long i = (long long)mp.y + t * SRV_T + threadIdx.x;
-    if (i < D.n) s = fma(v[i], v[i], s);
+  const bool restart = S.phase == PH_RESTART;
+  if (!restart && S.phase != PH_ARNOLDI) return;
+  const int j = restart ? 0 : S.j, l = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long n = D.n, end = min(n, (long long)mp.y + D.chunk);
+  const double *w = restart ? D.tmp : D.V + (size_t)(j + 1) * n, *V = restart ? D.tmp : D.V;
+  for (int k0 = 0; k0 <= j; k0 += 16) {
+    double t[2][8];
+#pragma unroll
+    for (int u = 0; u < 16; u++) t[u / 8][u % 8] = 0.0;
+    for (long long i = mp.y + threadIdx.x; i < end; i += SRV_T) {
+      const double wi = w[i];
+      double x[16];
+#pragma unroll
+      for (int u = 0; u < 16; u++)
+        if (k0 + u <= j) x[u] = V[(size_t)(k0 + u) * n + i];
+#pragma unroll
+      for (int u = 0; u < 16; u++)
+        if (k0 + u <= j) t[u / 8][u % 8] = fma(x[u], wi, t[u / 8][u % 8]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      if (k0 + 8 * h > j) break;
+      const double d = gm_warp_sums(t[h], l);
+      if ((l & 3) == 0) part[warp][k0 + 8 * h + (l >> 2)] = d;
+    }
   }
-  s = srv_block_sum(s);
-  if (threadIdx.x == 0) partial[(size_t)(D.red_first + mp.y / SRV_CHUNK) * SRV_PART + SRV_MMAX + 1] = s;
+  __syncthreads();
+  double *out = partial + (size_t)(D.red_first + mp.y / D.chunk) * SRV_PART;
+  for (int k = threadIdx.x; k <= j; k += SRV_T) out[k] = gm_pairs<W>(&part[0][k], KP);
 }
 
-// Gram-Schmidt dot products of V[k] (k = blockIdx.y <= j) with V[j+1]
-__global__ void __launch_bounds__(SRV_T) srv_dot_partial(const int2 *map, const SrvDesc *dd, const SrvState *ss,
-                                                         double *partial) {
+// Arnoldi step: h_k = sc_k sc_j <W_k, W_{j+1}>, W_{j+1} = sc_j W_{j+1} - sum_k h_k
+// sc_k W_k and the block partials of its squared norm.  Restart: V_0 = tmp /
+// |tmp|.  End of a cycle: x += sum_k y_k W_k.
+__global__ void __launch_bounds__(SRV_T) srv_orthogonalize(const int2 *map, const SrvDesc *dd, const SrvState *ss,
+                                                           double *partial) {
+  constexpr int W = SRV_T / 32;
+  __shared__ double coef[SRV_MMAX + 1], sh[W];
   const int2 mp = map[blockIdx.x];
-  const int k = blockIdx.y;
   const SrvDesc &D = dd[mp.x];
   const SrvState &S = ss[mp.x];
-  if (S.phase != PH_ARNOLDI || k > S.j) return;
-  const double *a = D.V + (size_t)k * D.n, *w = D.V + (size_t)(S.j + 1) * D.n;
-  double s = 0.0;
-  for (int t = 0; t < SRV_PER; t++) {
-    const long long i = (long long)mp.y + t * SRV_T + threadIdx.x;
-    if (i < D.n) s = fma(a[i], w[i], s);
+  const int phase = S.phase;
+  if (phase == PH_DONE) return;
+  const long long n = D.n, end = min(n, (long long)mp.y + D.chunk);
+  double *part = partial + (size_t)D.red_first * SRV_PART;
+  if (phase == PH_UPDATE) {
+    const int done = S.done_cols;
+    for (int k = threadIdx.x; k < done; k += SRV_T) coef[k] = D.y[k];
+    __syncthreads();
+    for (long long i = mp.y + threadIdx.x; i < end; i += SRV_T) D.x[i] += gm_combine<16>(D.V, n, coef, done, i);
+    return;
   }
-  s = srv_block_sum(s);
-  if (threadIdx.x == 0) partial[(size_t)(D.red_first + mp.y / SRV_CHUNK) * SRV_PART + k] = s;
+  const int j = phase == PH_RESTART ? 0 : S.j;
+  gm_sum_dots<SRV_T>(part, D.red_nb, SRV_PART, j, coef);
+  if (phase == PH_RESTART) {
+    const double inv = 1.0 / sqrt(coef[0]);
+    for (long long i = mp.y + threadIdx.x; i < end; i += SRV_T) D.V[i] = D.tmp[i] * inv;
+    return;
+  }
+  const double scj = D.sc[j];
+  for (int k = threadIdx.x; k <= j; k += SRV_T) {
+    const double sk = D.sc[k], h = sk * (scj * coef[k]);
+    if (mp.y == 0) D.hcol[k] = h;
+    coef[k] = h * sk;
+  }
+  __syncthreads();
+  double *w = D.V + (size_t)(j + 1) * n, s = 0.0;
+  for (long long i = mp.y + threadIdx.x; i < end; i += SRV_T) {
+    const double wi = fma(scj, w[i], -gm_combine<16>(D.V, n, coef, j + 1, i));
+    w[i] = wi;
+    s = fma(wi, wi, s);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) part[(size_t)(mp.y / D.chunk) * SRV_PART + SRV_MMAX + 1] = gm_pairs<W>(sh, 1);
 }
 
-// hcol[k] = sum over the request's blocks (fixed order), one CTA per request
-__global__ void srv_dot_sum(const int *act, const SrvDesc *dd, const SrvState *ss, const double *partial) {
+// The scalar logic, one block a request: the restart test
+// (lss_mkb_core.c:2377-2400, as gbfem_solve), the Arnoldi column, or the
+// end of a cycle's update.
+constexpr int SRV_LOGIC_T = 128;
+__global__ void __launch_bounds__(SRV_LOGIC_T) srv_logic(const int *act, const SrvDesc *dd, SrvState *ss,
+                                                         const double *partial) {
+  __shared__ double tot[1];
   const int slot = act[blockIdx.x];
   const SrvDesc &D = dd[slot];
-  const SrvState &S = ss[slot];
-  if (S.phase != PH_ARNOLDI) return;
-  for (int k = threadIdx.x; k <= S.j; k += blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < D.red_nb; b++) s += partial[(size_t)(D.red_first + b) * SRV_PART + k];
-    D.hcol[k] = s;
-  }
-}
-
-// V[j+1] -= V[:, :j+1] hcol
-__global__ void __launch_bounds__(SRV_T) srv_orthogonalize(const int2 *map, const SrvDesc *dd, const SrvState *ss) {
-  const int2 mp = map[blockIdx.x];
-  const SrvDesc &D = dd[mp.x];
-  const SrvState &S = ss[mp.x];
-  if (S.phase != PH_ARNOLDI) return;
-  double *w = D.V + (size_t)(S.j + 1) * D.n;
-  for (int t = 0; t < SRV_PER; t++) {
-    const long long i = (long long)mp.y + t * SRV_T + threadIdx.x;
-    if (i >= D.n) break;
-    double a = 0.0;
-    for (int k = 0; k <= S.j; k++) a = fma(D.hcol[k], D.V[(size_t)k * D.n + i], a);
-    w[i] = fma(-1.0, a, w[i]);
-  }
-}
-
-__device__ double srv_norm_from_partial(const SrvDesc &D, const double *partial) {
-  double s = 0.0;
-  for (int b = 0; b < D.red_nb; b++) s += partial[(size_t)(D.red_first + b) * SRV_PART + SRV_MMAX + 1];
-  return sqrt(s);
-}
-
-// restart: x is up to date, tmp = M^-1 (b - A x); start a new cycle or stop
-// (lss_mkb_core.c:2377-2400 tests, as gbfem_solve)
-__global__ void srv_logic_restart(int nact, const int *act, const SrvDesc *dd, SrvState *ss, const double *partial) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nact) return;
-  const int slot = act[t];
-  const SrvDesc &D = dd[slot];
   SrvState &S = ss[slot];
-  S.fresh = 0;
-  S.wscale = 0;
-  if (S.phase != PH_RESTART) return;
-  if (S.final_flag) {
-    S.phase = PH_DONE;
-    return;
-  }
-  const double rn = srv_norm_from_partial(D, partial);
-  if (S.beta0 < 0) S.beta0 = rn;
-  S.resid = rn;
-  if (rn < D.tol_abs || (S.beta0 > 0 && rn / S.beta0 < D.tol_rel) || S.it >= D.max_iter) {
-    S.phase = PH_DONE;
-    return;
-  }
-  D.s[0] = rn;
-  for (int i = 1; i <= D.m; i++) D.s[i] = 0.0;
-  S.beta = rn;
-  S.j = 0;
-  S.done_cols = 0;
-  S.fresh = 1;
-  S.phase = PH_ARNOLDI;
-}
-
-__global__ void __launch_bounds__(SRV_T) srv_start_cycle(const int2 *map, const SrvDesc *dd, const SrvState *ss) {
-  const int2 mp = map[blockIdx.x];
-  const SrvDesc &D = dd[mp.x];
-  const SrvState &S = ss[mp.x];
-  if (!S.fresh) return;
-  for (int t = 0; t < SRV_PER; t++) {
-    const long long i = (long long)mp.y + t * SRV_T + threadIdx.x;
-    if (i < D.n) D.V[i] = D.tmp[i] / S.beta;
-  }
-}
-
-// one Arnoldi column: Hessenberg entries, Givens rotations, residual
-// estimate, and at the end of a cycle the triangular solve for y
-__global__ void srv_logic_arnoldi(int nact, const int *act, const SrvDesc *dd, SrvState *ss,
-                                  const double *partial) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nact) return;
-  const int slot = act[t];
-  const SrvDesc &D = dd[slot];
-  SrvState &S = ss[slot];
-  if (S.phase != PH_ARNOLDI) return;
-  const int m = D.m, j = S.j, ld = m + 1;
-  const double hn = srv_norm_from_partial(D, partial);
-  double *H = D.H;
-  for (int k = 0; k <= j; k++) H[k + (size_t)j * ld] = D.hcol[k];
-  H[j + 1 + (size_t)j * ld] = hn;
-  for (int k = 0; k < j; k++) {
-    const double a = H[k + (size_t)j * ld], b = H[k + 1 + (size_t)j * ld];
-    H[k + (size_t)j * ld] = D.cs[k] * a + D.sn[k] * b;
-    H[k + 1 + (size_t)j * ld] = D.cs[k] * b - D.sn[k] * a;
-  }
-  {
-    const double a = H[j + (size_t)j * ld], b = H[j + 1 + (size_t)j * ld];
-    const double rr = hypot(a, b);
-    D.cs[j] = a / rr;
-    D.sn[j] = b / rr;
-    H[j + (size_t)j * ld] = rr;
-    H[j + 1 + (size_t)j * ld] = 0.0;
-    const double s0 = D.s[j];
-    D.s[j] = D.cs[j] * s0;
-    D.s[j + 1] = -D.sn[j] * s0;
-  }
-  S.it++;
-  S.resid = fabs(D.s[j + 1]);
-  S.hn = hn;
-  S.widx = j + 1;
-  S.wscale = 1;
-  const bool conv = S.resid < D.tol_abs || S.resid / S.beta0 < D.tol_rel;
-  if (j == m - 1 || S.it >= D.max_iter || conv) {
-    const int done = j + 1;
-    for (int k = done - 1; k >= 0; k--) {
-      double v = D.s[k];
-      for (int i = k + 1; i < done; i++) v -= H[k + (size_t)i * ld] * D.y[i];
-      D.y[k] = v / H[k + (size_t)k * ld];
+  const int phase = S.phase;
+  const double *part = partial + (size_t)D.red_first * SRV_PART;
+  if (phase == PH_ARNOLDI) {
+    const int j = S.j;
+    const GmStep g = {D.m, D.red_nb, SRV_PART, part + SRV_MMAX + 1, D.H, D.cs, D.sn, D.s, D.y, D.hcol, D.sc};
+    gm_step_logic<SRV_LOGIC_T, SRV_MMAX>(g, j, [&](double resid, double) -> int {
+      const int it = S.it + 1;
+      S.it = it;
+      S.resid = resid;
+      const bool conv = resid < D.tol_abs || resid / S.beta0 < D.tol_rel;
+      const bool end = j == D.m - 1 || it >= D.max_iter || conv;
+      if (end) {
+        S.done_cols = j + 1;
+        S.final_flag = (conv || it >= D.max_iter) ? 1 : 0;
+        S.phase = PH_UPDATE;
+      } else {
+        S.j = j + 1;
+      }
+      return end;
+    });
+  } else if (phase == PH_RESTART) {
+    gm_sum_dots<SRV_LOGIC_T>(part, D.red_nb, SRV_PART, 0, tot);
+    if (threadIdx.x != 0) return;
+    const double rn = sqrt(tot[0]);
+    if (S.beta0 < 0) S.beta0 = rn;
+    S.resid = rn;
+    if (rn < D.tol_abs || (S.beta0 > 0 && rn / S.beta0 < D.tol_rel) || S.it >= D.max_iter) {
+      S.phase = PH_DONE;
+      return;
     }
-    S.done_cols = done;
-    S.final_flag = (conv || S.it >= D.max_iter) ? 1 : 0;
-    S.phase = PH_RESTART;
-  } else {
-    S.j = j + 1;
-  }
-}
-
-__global__ void __launch_bounds__(SRV_T) srv_normalize(const int2 *map, const SrvDesc *dd, const SrvState *ss) {
-  const int2 mp = map[blockIdx.x];
-  const SrvDesc &D = dd[mp.x];
-  const SrvState &S = ss[mp.x];
-  if (!S.wscale) return;
-  double *w = D.V + (size_t)S.widx * D.n;
-  for (int t = 0; t < SRV_PER; t++) {
-    const long long i = (long long)mp.y + t * SRV_T + threadIdx.x;
-    if (i < D.n) w[i] = w[i] / S.hn;
+    D.s[0] = rn;
+    for (int i = 1; i <= D.m; i++) D.s[i] = 0.0;
+    D.sc[0] = 1.0;  // V_0 is stored normalised
+    S.j = 0;
+    S.done_cols = 0;
+    S.phase = PH_ARNOLDI;
+  } else if (phase == PH_UPDATE && threadIdx.x == 0) {
+    S.phase = S.final_flag ? PH_DONE : PH_RESTART;
   }
 }
 
@@ -408,9 +359,9 @@ struct SrvLane {
   DevBuf<int> d_act;
   DevBuf<double> d_partial;
   SrvState *h_state = nullptr;  // pinned readback of the last poll
-  int n_vec = 0, n_crs = 0, max_m1 = 1;
-  cudaGraphExec_t graph = nullptr;
-  int graph_kernels = 0;
+  int n_vec = 0, n_crs = 0;
+  cudaGraphExec_t graph = nullptr;  // of the current set, once it has stood
+  int graph_kernels = 0, polls = 0;  // polls since the set changed
 };
 
 struct gbfem_server_s {
@@ -430,9 +381,22 @@ struct gbfem_server_s {
   bool stop = false;
   std::vector<std::thread> workers;
   std::thread engine;
-  // contexts and Krylov spaces of finished requests, freed by the reaper
-  // thread: a cudaFree synchronises the device, which on the engine thread
-  // would hold every lane until all GPU work drained
+  // Contexts and Krylov spaces of finished requests wait here for the next
+  // request of their kind: a new context's stream, events and some thirty
+  // device allocations cost more than a small request's work, and each
+  // cudaFree synchronises the device.  At most SRV_IDLE of a kind and an
+  // eighth of the HBM budget; not charged to it, but freed as soon as an
+  // admission needs the room, and with the server.
+  struct Idle {
+    int key = 0, nno = 0, nel = 0;  // key: kind, or 2 for solo-sized std requests (another stream priority)
+    gbfem_ctx ctx = nullptr;
+    DevBuf<double> kry;
+    long long bytes = 0;
+  };
+  std::deque<Idle> idle;  // oldest first
+  long long idle_bytes = 0;
+  // the others are freed by the reaper thread (a cudaFree on the engine
+  // thread would hold every lane until all GPU work drained)
   std::deque<std::pair<gbfem_ctx, double *>> reapq;
   std::condition_variable cv_reap;
   bool reap_stop = false;
@@ -458,20 +422,77 @@ struct gbfem_server_s {
 
 namespace {
 
-// Hands a finished request's context and Krylov space to the reaper (no
-// device work of it may be in flight).
-void reap(gbfem_server s, SrvRequest &r) {
-  double *kry = r.kry.p;
-  r.kry.p = nullptr;  // ownership passes to the reaper
-  r.kry.n = 0;
-  gbfem_ctx c = r.ctx;
-  r.ctx = nullptr;
-  if (!c && !kry) return;
-  {
-    std::lock_guard<std::mutex> lk(s->mu);
-    s->reapq.emplace_back(c, kry);
-  }
+constexpr int SRV_IDLE = 8;
+constexpr int SRV_CAPTURE_POLLS = 16;  // polls of one set before its step is captured
+
+int idle_key(const SrvRequest &r) { return r.kind == 0 && r.solo_admit ? 2 : r.kind; }
+
+void drop_oldest_idle(gbfem_server s) {  // caller holds s->mu
+  gbfem_server_s::Idle &i = s->idle.front();
+  s->idle_bytes -= i.bytes;
+  s->reapq.emplace_back(i.ctx, i.kry.p);
+  s->idle.pop_front();
   s->cv_reap.notify_one();
+}
+
+// Whether `bytes` more fit in the HBM budget (idle contexts give way); a
+// request larger than the budget runs alone.
+bool fits(gbfem_server s, long long bytes) {  // caller holds s->mu
+  while (!s->idle.empty() && s->in_use + s->idle_bytes + bytes > s->budget) drop_oldest_idle(s);
+  return s->in_use + bytes <= s->budget || s->in_use == 0;
+}
+
+// A finished request's context and Krylov space (no device work of it may be
+// in flight) are kept for another request; a failed one's go to the reaper.
+void reap(gbfem_server s, SrvRequest &r, bool reusable = true) {
+  gbfem_server_s::Idle i;
+  i.key = idle_key(r);
+  i.nno = r.nno;
+  i.nel = r.nel;
+  i.ctx = r.ctx;
+  i.kry = r.kry;
+  r.ctx = nullptr;
+  r.kry = DevBuf<double>();  // ownership has passed
+  if (!i.ctx && !i.kry.p) return;
+  std::lock_guard<std::mutex> lk(s->mu);
+  if (i.ctx && reusable && !s->stop) {
+    i.bytes = gbfem_device_bytes(i.ctx) + (long long)i.kry.bytes();
+    int same = 0;
+    for (const auto &o : s->idle) same += o.key == i.key;
+    while (!s->idle.empty() && same >= SRV_IDLE) {
+      // the oldest of this kind makes room
+      auto o = std::find_if(s->idle.begin(), s->idle.end(), [&](const gbfem_server_s::Idle &q) { return q.key == i.key; });
+      std::swap(*o, s->idle.front());
+      drop_oldest_idle(s);
+      same--;
+    }
+    if (s->idle_bytes + i.bytes <= s->budget / 8 && s->in_use + s->idle_bytes + i.bytes <= s->budget) {
+      s->idle_bytes += i.bytes;
+      s->idle.push_back(i);
+      return;
+    }
+  }
+  s->reapq.emplace_back(i.ctx, i.kry.p);
+  s->cv_reap.notify_one();
+}
+
+// An idle context for the request, of its own mesh size if there is one (its
+// buffers then fit as they are)
+bool take_idle(gbfem_server s, SrvRequest &r) {
+  std::lock_guard<std::mutex> lk(s->mu);
+  const int key = idle_key(r);
+  auto best = s->idle.end();
+  for (auto it = s->idle.begin(); it != s->idle.end(); ++it) {
+    if (it->key != key) continue;
+    best = it;
+    if (it->nno == r.nno && it->nel == r.nel) break;
+  }
+  if (best == s->idle.end()) return false;
+  r.ctx = best->ctx;
+  r.kry = best->kry;
+  s->idle_bytes -= best->bytes;
+  s->idle.erase(best);
+  return true;
 }
 
 void reaper_loop(gbfem_server s) {
@@ -504,7 +525,7 @@ void try_admit(gbfem_server s) {  // caller holds s->mu
         ++it;
         continue;
       }
-      if (s->in_use + r->footprint > s->budget && s->in_use > 0) break;
+      if (!fits(s, r->footprint)) break;
       it = q.erase(it);
       r->solo_admit = true;
       s->n_solo++;
@@ -524,7 +545,7 @@ void try_admit(gbfem_server s) {  // caller holds s->mu
       ReqPtr r = ln.waitq.front();
       if (ln.held + other.held >= s->max_active) break;
       if (ln.held >= share && !other.waitq.empty()) break;
-      if (s->in_use + r->footprint > s->budget && s->in_use > 0) break;
+      if (!fits(s, r->footprint)) break;
       ln.waitq.pop_front();
       ln.held++;
       s->in_use += r->footprint;
@@ -550,12 +571,13 @@ int prepare(gbfem_server s, SrvRequest &r) {
       return -1;
     }
   }
-  gbfem_ctx c = nullptr;
   // std requests' preparation and solo solves at the std lane's priority:
   // the DG lane's long block SpMVs (lowest priority) do not hold them up
-  int rc = gbfem::create_context(&c, s->device, r.kind == 0 ? (r.solo_admit ? s->prio_solo : s->prio_std) : 0);
-  if (rc < 0) return rc;
-  r.ctx = c;
+  int rc = 0;
+  if (!take_idle(s, r) &&
+      (rc = gbfem::create_context(&r.ctx, s->device, r.kind == 0 ? (r.solo_admit ? s->prio_solo : s->prio_std) : 0)) < 0)
+    return rc;
+  gbfem_ctx c = r.ctx;
   std::vector<int> fid, fbc;
   if (r.kind == 0) {
     fbc.assign(r.nbf, 1);
@@ -615,9 +637,9 @@ int prepare(gbfem_server s, SrvRequest &r) {
       return -2;
     }
   }
-  // Krylov workspace: x, tmp, V (m+1 columns), H, cs, sn, s, y, hcol
+  // Krylov workspace: x, tmp, V (m+1 columns), H, cs, sn, s, y, hcol, sc
   const long long n = r.n, m1 = r.krylov + 1;
-  if ((rc = r.kry.alloc((size_t)(n * (m1 + 2) + m1 * m1 + 5 * (m1 + 1)))) < 0) return rc;
+  if ((rc = r.kry.alloc((size_t)(n * (m1 + 2) + m1 * m1 + 6 * (m1 + 1)))) < 0) return rc;
   if (cudaMemsetAsync(r.kry.p, 0, r.kry.bytes(), c->stream) != cudaSuccess) return -1;
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
     gbfem::set_error("preparation failed on the device");
@@ -653,7 +675,7 @@ void prep_worker(gbfem_server s) {
       r->status = rc < 0 ? -1 : -2;
       r->err = rc < 0 ? gbfem_last_error() : "cancelled";
       lk.unlock();
-      reap(s, *r);
+      reap(s, *r, rc >= 0);
       lk.lock();
       s->in_use -= r->charged;
       r->charged = 0;
@@ -708,7 +730,7 @@ void solo_worker(gbfem_server s) {
                         : gbfem::gmres_device_std(r->ctx, r->krylov, r->max_iter, r->tol, 1, r->x.data(), &res,
                                                        &rel);
     const std::string err = it < 0 ? std::string(gbfem_last_error()) : std::string();
-    reap(s, *r);
+    reap(s, *r, it >= 0);
     std::lock_guard<std::mutex> lk(s->mu);
     r->iters = it < 0 ? 0 : it;
     r->rel = rel;
@@ -762,6 +784,7 @@ void fill_desc(SrvDesc &d, SrvRequest &r) {
   d.s = d.sn + (m1 + 1);
   d.y = d.s + (m1 + 1);
   d.hcol = d.y + (m1 + 1);
+  d.sc = d.hcol + (m1 + 1);
 }
 
 // rebuild a lane's block maps and its requests' descriptors after its
@@ -770,20 +793,19 @@ int rebuild(gbfem_server s, SrvLane &ln, int L) {
   std::vector<int2> mv, mc;
   int red = 0;
   ln.act.clear();
-  ln.max_m1 = 1;
   for (int i = 0; i < gbfem::SRV_MAXSLOTS; i++) {
     if (!s->slots[i] || s->slots[i]->kind != L) continue;
     SrvRequest &r = *s->slots[i];
     ln.act.push_back(i);
     SrvDesc &d = s->h_desc[i];
-    const int nb = (r.n + gbfem::SRV_CHUNK - 1) / gbfem::SRV_CHUNK;
+    d.chunk = gbfem::srv_chunk(r.n);
+    const int nb = (r.n + d.chunk - 1) / d.chunk;
     d.red_first = red;
     d.red_nb = nb;
     red += nb;
-    for (int b = 0; b < nb; b++) mv.push_back(make_int2(i, b * gbfem::SRV_CHUNK));
+    for (int b = 0; b < nb; b++) mv.push_back(make_int2(i, b * d.chunk));
     if (r.kind == 0)
       for (int r0 = 0; r0 < r.n; r0 += gbfem::SRV_SPMV_ROWS) mc.push_back(make_int2(i, r0));
-    ln.max_m1 = std::max(ln.max_m1, r.krylov + 1);
   }
   ln.n_vec = (int)mv.size();
   ln.n_crs = (int)mc.size();
@@ -808,74 +830,56 @@ int rebuild(gbfem_server s, SrvLane &ln, int L) {
 int step(gbfem_server s, SrvLane &ln) {
   using namespace gbfem;
   cudaStream_t st = ln.stream;
-  const int nact = (int)ln.act.size();
-  const int lt = 128, lb = (nact + lt - 1) / lt;
-  int L = 0;
-  const int2 *mv = ln.d_map_vec.p, *mc = ln.d_map_crs.p;
+  const int2 *mv = ln.d_map_vec.p;
   SrvDesc *dd = s->d_desc.p;
   SrvState *ss = s->d_state.p;
   double *part = ln.d_partial.p;
-  auto dg_spmv = [&](int mode) {
-    for (int i : ln.act) {
-      SrvRequest &r = *s->slots[i];
-      if (r.kind != 1) continue;
-      for (int p = 1; p <= 4; p++) {
-        const int cnt = (int)r.ctx->dg_list[p].n;
-        if (!r.ctx->dg_list[p].p || cnt == 0) continue;
-        const int grid = (cnt + DGS_ROWS - 1) / DGS_ROWS;
-        const int *lst = r.ctx->dg_list[p].p;
-#define GB_SRV_DG(PP)                                                                          \
-  if (mode == 0)                                                                               \
-    srv_dg_spmv<PP, 0><<<grid, DGS_THREADS, 0, st>>>(i, cnt, lst, dd, ss);                    \
-  else                                                                                         \
-    srv_dg_spmv<PP, 1><<<grid, DGS_THREADS, 0, st>>>(i, cnt, lst, dd, ss)
-        switch (p) {
-          case 1: GB_SRV_DG(1); break;
-          case 2: GB_SRV_DG(2); break;
-          case 3: GB_SRV_DG(3); break;
-          default: GB_SRV_DG(4); break;
-        }
-#undef GB_SRV_DG
-        L++;
+  int L = 0;
+  if (ln.n_crs) {
+    srv_crs_spmv<<<ln.n_crs, SRV_T, 0, st>>>(ln.d_map_crs.p, dd, ss);
+    L++;
+  }
+  for (int i : ln.act) {
+    SrvRequest &r = *s->slots[i];
+    if (r.kind != 1) continue;
+    for (int p = 1; p <= 4; p++) {
+      const int cnt = (int)r.ctx->dg_list[p].n;
+      if (!r.ctx->dg_list[p].p || cnt == 0) continue;
+      const int grid = (cnt + DGS_ROWS - 1) / DGS_ROWS;
+      const int *lst = r.ctx->dg_list[p].p;
+#define GB_SRV_DG(PP) srv_dg_spmv<PP><<<grid, DGS_THREADS, 0, st>>>(i, cnt, lst, dd, ss)
+      switch (p) {
+        case 1: GB_SRV_DG(1); break;
+        case 2: GB_SRV_DG(2); break;
+        case 3: GB_SRV_DG(3); break;
+        default: GB_SRV_DG(4); break;
       }
+#undef GB_SRV_DG
+      L++;
     }
-  };
-  // restart: x += V y, residual, its norm, new cycle or stop
-  srv_update_x<<<ln.n_vec, SRV_T, 0, st>>>(mv, dd, ss);
-  if (ln.n_crs) srv_crs_spmv<0><<<ln.n_crs, SRV_T, 0, st>>>(mc, dd, ss);
-  dg_spmv(0);
-  srv_norm_partial<0><<<ln.n_vec, SRV_T, 0, st>>>(mv, dd, ss, part);
-  srv_logic_restart<<<lb, lt, 0, st>>>(nact, ln.d_act.p, dd, ss, part);
-  srv_start_cycle<<<ln.n_vec, SRV_T, 0, st>>>(mv, dd, ss);
-  // one Arnoldi step
-  if (ln.n_crs) srv_crs_spmv<1><<<ln.n_crs, SRV_T, 0, st>>>(mc, dd, ss);
-  dg_spmv(1);
-  srv_dot_partial<<<dim3(ln.n_vec, ln.max_m1), SRV_T, 0, st>>>(mv, dd, ss, part);
-  srv_dot_sum<<<nact, 64, 0, st>>>(ln.d_act.p, dd, ss, part);
-  srv_orthogonalize<<<ln.n_vec, SRV_T, 0, st>>>(mv, dd, ss);
-  srv_norm_partial<1><<<ln.n_vec, SRV_T, 0, st>>>(mv, dd, ss, part);
-  srv_logic_arnoldi<<<lb, lt, 0, st>>>(nact, ln.d_act.p, dd, ss, part);
-  srv_normalize<<<ln.n_vec, SRV_T, 0, st>>>(mv, dd, ss);
-  L += 11 + (ln.n_crs ? 2 : 0);
+  }
+  srv_dots<<<ln.n_vec, SRV_T, 0, st>>>(mv, dd, ss, part);
+  srv_orthogonalize<<<ln.n_vec, SRV_T, 0, st>>>(mv, dd, ss, part);
+  srv_logic<<<(int)ln.act.size(), SRV_LOGIC_T, 0, st>>>(ln.d_act.p, dd, ss, part);
+  L += 3;
   GB_CUDA(cudaGetLastError());
   return L;
 }
 
+void drop_graph(SrvLane &ln) {
+  if (ln.graph) cudaGraphExecDestroy(ln.graph);
+  ln.graph = nullptr;
+  ln.polls = 0;
+}
+
 // capture a lane's step for its current active set
 int capture(gbfem_server s, SrvLane &ln) {
-  if (ln.graph) {
-    cudaGraphExecDestroy(ln.graph);
-    ln.graph = nullptr;
-  }
-  if (ln.act.empty()) return 0;
-  cudaGraph_t g = nullptr;
   GB_CUDA(cudaStreamBeginCapture(ln.stream, cudaStreamCaptureModeThreadLocal));
   const int L = step(s, ln);
-  cudaGraph_t gg = nullptr;
-  const cudaError_t e = cudaStreamEndCapture(ln.stream, &gg);
+  cudaGraph_t g = nullptr;
+  const cudaError_t e = cudaStreamEndCapture(ln.stream, &g);
   if (L < 0) return L;
   GB_CUDA(e);
-  g = gg;
   const cudaError_t ei = cudaGraphInstantiate(&ln.graph, g, 0);
   cudaGraphDestroy(g);
   GB_CUDA(ei);
@@ -918,6 +922,7 @@ void engine_fail(gbfem_server s, const std::string &msg) {
 
 void engine_loop(gbfem_server s) {
   cudaSetDevice(s->device);
+  double last_progress = 0.0;
   for (;;) {
     {
       std::unique_lock<std::mutex> lk(s->mu);
@@ -976,7 +981,8 @@ void engine_loop(gbfem_server s) {
         }
       }
       if (ln.changed) {
-        if (rebuild(s, ln, L) < 0 || capture(s, ln) < 0) {
+        drop_graph(ln);
+        if (rebuild(s, ln, L) < 0) {
           engine_fail(s, gbfem_last_error());
           return;
         }
@@ -987,13 +993,21 @@ void engine_loop(gbfem_server s) {
       if (L == 1 && s->std_precedence && s->n_solo.load() > 0) continue;
       // several steps per poll: a finished request's kernels are no-ops until
       // it is retired, so the extra steps only cost their launch
-      cudaError_t ge = cudaSuccess;
-      for (int k = 0; k < s->steps_per_poll && ge == cudaSuccess; k++) {
-        ge = cudaGraphLaunch(ln.graph, ln.stream);
-        s->steps++;
-        s->launches += ln.graph_kernels;
+      if (!ln.graph && ++ln.polls > SRV_CAPTURE_POLLS && capture(s, ln) < 0) {
+        engine_fail(s, gbfem_last_error());
+        return;
       }
-      if (ge != cudaSuccess ||
+      bool ok = true;
+      for (int k = 0; k < s->steps_per_poll && ok; k++) {
+        int launched = ln.graph_kernels;
+        if (ln.graph)
+          ok = cudaGraphLaunch(ln.graph, ln.stream) == cudaSuccess;
+        else
+          ok = (launched = step(s, ln)) >= 0;
+        s->steps++;
+        s->launches += launched;
+      }
+      if (!ok ||
           cudaMemcpyAsync(ln.h_state, s->d_state.p, sizeof(SrvState) * gbfem::SRV_MAXSLOTS, cudaMemcpyDeviceToHost,
                           ln.stream) != cudaSuccess ||
           cudaEventRecord(ln.done, ln.stream) != cudaSuccess) {
@@ -1003,7 +1017,16 @@ void engine_loop(gbfem_server s) {
       ln.busy = true;
       progressed = true;
     }
-    if (!progressed) std::this_thread::sleep_for(std::chrono::microseconds(20));
+    // a poll's steps take some tens of microseconds for small requests: spin
+    // for the first 200 us without progress (a sleep of 20 us lasts 70 and
+    // more), then sleep between looks
+    const double t = now_s();
+    if (progressed)
+      last_progress = t;
+    else if (t - last_progress < 200e-6)
+      std::this_thread::yield();
+    else
+      std::this_thread::sleep_for(std::chrono::microseconds(20));
   }
 }
 
@@ -1092,6 +1115,7 @@ int gbfem_server_destroy(gbfem_server s) {
   if (s->engine.joinable()) s->engine.join();
   {
     std::lock_guard<std::mutex> lk(s->mu);
+    while (!s->idle.empty()) drop_oldest_idle(s);
     s->reap_stop = true;
   }
   s->cv_reap.notify_all();
