@@ -12,6 +12,8 @@
 // here as the explicit inverse of each diagonal block: applying it is then a
 // dense block product fused into the SpMV.
 
+#include <type_traits>
+
 #include "dg_spmv.cuh"
 #include "dg_tables.h"
 #include "gbfem_internal.h"
@@ -153,6 +155,16 @@ __global__ void __launch_bounds__(DGS_THREADS) dg_block_spmv_kernel(
   dg_block_row_spmv<P, VT>(mode, count, ent_el, roff, row_val, cx_off, colx, val, dinv_off, dinv, x, b, out, sv);
 }
 
+// one CTA a block row (small systems)
+template <int P>
+__global__ void __launch_bounds__(DGS_THREADS) dg_block_spmv_wide_kernel(
+    int mode, const int *__restrict__ ent_el, const int *__restrict__ roff, const long long *__restrict__ row_val,
+    const long long *__restrict__ cx_off, const int *__restrict__ colx, const double *__restrict__ val,
+    const long long *__restrict__ dinv_off, const double *__restrict__ dinv, const double *__restrict__ x,
+    const double *__restrict__ b, double *__restrict__ out) {
+  dg_block_row_wide<P>(mode, ent_el[blockIdx.x], roff, row_val, cx_off, colx, val, dinv_off, dinv, x, b, out);
+}
+
 // Residual out = b - A x with the products and sums carried in two FP64
 // words per row (error-free transformations: the exact product error from an
 // FMA, Knuth's TwoSum, the errors summed in a second word and added once at
@@ -265,6 +277,13 @@ static int launch_dg_block_spmv_t(cudaStream_t st, int mode, int p, int count, c
   GB_CHECK(mode == 2 || (dinv && dinv_off), "block SpMV needs the inverted diagonal blocks");
   const int grid = (count + DGS_ROWS - 1) / DGS_ROWS;
 #define GB_DGS_LAUNCH(PP)                                                                                      \
+  if constexpr (std::is_same<VT, double>::value) {                                                             \
+    if (count <= dgs_wide_max(PP)) {                                                                            \
+      dg_block_spmv_wide_kernel<PP><<<count, DGS_THREADS, 0, st>>>(mode, ent_el, roff, row_val, cx_off, colx,  \
+                                                                   val, dinv_off, dinv, x, b, out);            \
+      break;                                                                                                   \
+    }                                                                                                          \
+  }                                                                                                            \
   dg_block_spmv_kernel<PP, VT><<<grid, DGS_THREADS, 0, st>>>(mode, count, ent_el, roff, row_val, cx_off, colx, \
                                                              val, dinv_off, dinv, x, b, out)
   switch (p) {

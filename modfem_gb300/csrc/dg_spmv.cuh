@@ -3,6 +3,7 @@
 #pragma once
 
 #include "dword.cuh"
+#include "gmres_step.cuh"
 
 namespace gbfem {
 
@@ -134,6 +135,77 @@ __device__ __forceinline__ void dg_block_row_spmv(
     const int i = g + DGS_LANES * s;
     if (i < NS) out[r0 + i] = dgs_out(o[s]);
   }
+}
+
+// One block row by a whole CTA of DGS_THREADS threads, for systems too small to
+// fill the chip with eight-lane groups (250 prisms of degree 2 are 8 CTAs of
+// them, and a group walks a row's 104 columns alone): the columns are split
+// over C = 256 / NS groups of NS threads (a thread a row), four or eight loads
+// in flight, the partial sums added pairwise, then the same for the inverted
+// diagonal block.  The order depends on the class only.
+template <int P>
+struct DgWide {
+  static constexpr int NS = DgSpmvDims<P>::NS, C = DGS_THREADS / NS;
+  static constexpr int U = NS >= 35 ? 8 : 4;  // loads in flight
+};
+// Block rows of a class up to which the CTA form is the faster one (measured
+// crossovers; us a product, CTA form against groups of eight lanes):
+//   prisms  p = 1: 432 rows 10.7 / 11.1, 1,024 18 / 12;   p = 2: 2,000 23 / 37, 6,750 67 / 68
+//           p = 3: 2,000 63 / 200, 11,664 290 / 275;      p = 4: 2,000 183 / 863, 11,664 939 / 1,033
+//   tetrahedra p = 1: never;                              p = 2: 1,296 16 / 18, 2,058 21 / 18
+//           p = 3: 2,058 25 / 38, 6,000 61 / 64;          p = 4: 2,058 52 / 134, 10,368 211 / 197
+// (the groups' time stays flat until they fill the chip: they walk a row's
+// columns one or two at a time)
+__host__ __device__ constexpr int dgs_wide_max(int cls) {
+  return cls == 1 ? 512 : cls == 2 ? 6656 : cls == 3 ? 10000 : cls == 4 ? 13000
+       : cls == 6 ? 1536 : cls == 7 ? 6144 : cls == 8 ? 8192 : 0;
+}
+template <int P>
+__device__ __forceinline__ double dg_wide_product(const double *__restrict__ A, int nct, const int *__restrict__ cx,
+                                                  const double *x, double *red) {
+  constexpr int NS = DgWide<P>::NS, C = DgWide<P>::C, U = DgWide<P>::U;
+  const int i = threadIdx.x % NS, g = threadIdx.x / NS;
+  double acc = 0.0;
+  if (g < C)
+    for (int t = g; t < nct; t += U * C) {
+      double a[U], v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (t + u * C < nct) {
+          a[u] = A[(size_t)(t + u * C) * NS + i];
+          v[u] = x[cx ? cx[t + u * C] : t + u * C];
+        }
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (t + u * C < nct) acc = fma(a[u], v[u], acc);
+    }
+  if (g < C) red[g * NS + i] = acc;
+  __syncthreads();
+  return threadIdx.x < NS ? gm_pairs<C>(red + threadIdx.x, NS) : 0.0;
+}
+// (mode and arguments as dg_block_row_spmv; block row of element e)
+template <int P>
+__device__ __forceinline__ void dg_block_row_wide(int mode, int e, const int *__restrict__ roff,
+                                                  const long long *__restrict__ row_val,
+                                                  const long long *__restrict__ cx_off, const int *__restrict__ colx,
+                                                  const double *__restrict__ val,
+                                                  const long long *__restrict__ dinv_off,
+                                                  const double *__restrict__ dinv, const double *__restrict__ x,
+                                                  const double *__restrict__ b, double *__restrict__ out) {
+  constexpr int NS = DgWide<P>::NS;
+  __shared__ double red[DGS_THREADS], y[NS];
+  const int r0 = roff[e], tid = threadIdx.x;
+  const long long c0 = cx_off[e];
+  double s = dg_wide_product<P>(val + row_val[e], (int)(cx_off[e + 1] - c0), colx + c0, x, red);
+  if (tid < NS && mode != 1) s = (b ? b[r0 + tid] : 0.0) - s;
+  if (mode == 2) {
+    if (tid < NS) out[r0 + tid] = s;
+    return;
+  }
+  if (tid < NS) y[tid] = s;
+  __syncthreads();
+  s = dg_wide_product<P>(dinv + dinv_off[e], NS, nullptr, y, red);
+  if (tid < NS) out[r0 + tid] = s;
 }
 
 }  // namespace gbfem

@@ -135,8 +135,9 @@ __global__ void __launch_bounds__(SRV_T) srv_crs_spmv(const int2 *map, const Srv
   if (valid && lane == 0) out[r] = restart ? (D.b[r] - s) * D.dinv[r] : D.dinv[r] * s;
 }
 
-// the block rows of degree P of one DG request (the same two forms)
-template <int P>
+// the block rows of degree P of one DG request (the same two forms); WIDE:
+// one CTA a block row
+template <int P, bool WIDE>
 __global__ void __launch_bounds__(DGS_THREADS) srv_dg_spmv(int slot, int count, const int *ent_el,
                                                            const SrvDesc *dd, const SrvState *ss) {
   const SrvDesc &D = dd[slot];
@@ -145,9 +146,14 @@ __global__ void __launch_bounds__(DGS_THREADS) srv_dg_spmv(int slot, int count, 
   if (!restart && S.phase != PH_ARNOLDI) return;
   const double *x = restart ? D.x : D.V + (size_t)S.j * D.n, *b = restart ? D.b : nullptr;
   double *out = restart ? D.tmp : D.V + (size_t)(S.j + 1) * D.n;
-  __shared__ double sv[DGS_ROWS][DgSpmvDims<P>::NS];
-  dg_block_row_spmv<P>(restart ? 0 : 1, count, ent_el, D.roff, D.row_val, D.cx_off, D.colx, D.dgval, D.dinv_off,
-                       D.dgdinv, x, b, out, sv);
+  if constexpr (WIDE) {
+    dg_block_row_wide<P>(restart ? 0 : 1, ent_el[blockIdx.x], D.roff, D.row_val, D.cx_off, D.colx, D.dgval,
+                         D.dinv_off, D.dgdinv, x, b, out);
+  } else {
+    __shared__ double sv[DGS_ROWS][DgSpmvDims<P>::NS];
+    dg_block_row_spmv<P>(restart ? 0 : 1, count, ent_el, D.roff, D.row_val, D.cx_off, D.colx, D.dgval, D.dinv_off,
+                         D.dgdinv, x, b, out, sv);
+  }
 }
 
 // Block partials of <W_k, W_{j+1}>, k <= j, or of <tmp, tmp> at a restart:
@@ -847,7 +853,11 @@ int step(gbfem_server s, SrvLane &ln) {
       if (!r.ctx->dg_list[p].p || cnt == 0) continue;
       const int grid = (cnt + DGS_ROWS - 1) / DGS_ROWS;
       const int *lst = r.ctx->dg_list[p].p;
-#define GB_SRV_DG(PP) srv_dg_spmv<PP><<<grid, DGS_THREADS, 0, st>>>(i, cnt, lst, dd, ss)
+#define GB_SRV_DG(PP)                                                             \
+  if (cnt <= dgs_wide_max(PP))                                                    \
+    srv_dg_spmv<PP, true><<<cnt, DGS_THREADS, 0, st>>>(i, cnt, lst, dd, ss);      \
+  else                                                                            \
+    srv_dg_spmv<PP, false><<<grid, DGS_THREADS, 0, st>>>(i, cnt, lst, dd, ss)
       switch (p) {
         case 1: GB_SRV_DG(1); break;
         case 2: GB_SRV_DG(2); break;
