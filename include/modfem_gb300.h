@@ -39,8 +39,8 @@ typedef struct gbfem_ctx_s *gbfem_ctx;
 #define GBFEM_TETRA 4
 /* scatter modes of gbfem_assemble */
 #define GBFEM_SCATTER_ATOMIC 0 /* one launch, FP64 atomics (summation order varies) */
-#define GBFEM_SCATTER_COLOR 1  /* one launch per colour, plain adds (deterministic) */
-#define GBFEM_SCATTER_GATHER 2 /* local matrices stored, then one thread a row sums them over
+#define GBFEM_SCATTER_COLOR 1  /* one launch per colour, plain adds (deterministic); tetrahedra: as GATHER */
+#define GBFEM_SCATTER_GATHER 2 /* local matrices stored, then a group of lanes a row sums them over
                                   the incident elements in element order (deterministic, no
                                   colouring; std prisms, FP64 element arithmetic) */
 

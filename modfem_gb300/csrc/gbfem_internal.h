@@ -118,10 +118,15 @@ int launch_prism_faces(cudaStream_t st, bool atomic, int count, const int *ent_f
                        const double *xyz, double penalty, double g, const int *tab, double *val,
                        double *rhs, int do_sm, int do_rhs, int *err);
 // Prism elements by the deterministic gather scatter: local matrices stored
-// to ek (42 doubles an element), then one thread a row over the incidence
-int launch_std_gather(cudaStream_t st, bool aniso, int nel, int nd, const int *el_nodes, const double *xyz,
-                      const double *k_el, const double *D_el, double f, const int *inc_ptr, const int *inc,
-                      const int *tab, double *ek, double *val, double *rhs, int *err);
+// to ek (nv nv + nv doubles an element), then a group of lanes a row over the incidence
+// (and the penalty faces through the elements' face lists; nv 6 prisms, 4
+// tetrahedra, which have no faces); every entry is written
+int launch_std_gather(cudaStream_t st, int nv, bool aniso, int nel, int nd, const int *el_nodes, const double *xyz,
+                      const double *k_el, const double *D_el, double f, int nfa, const int *fa_el, const int *fa_side,
+                      double penalty, double g, const int *fa_head, const int *fa_next, const int *row_ptr,
+                      const int *inc_ptr, const int *inc, const int *tab, double *ek, double *fk, double *val,
+                      double *rhs);
+int launch_face_lists(cudaStream_t st, int nel, int nfa, const int *fa_el, int *head, int *next);
 // Elements (faces = false, 1-based element ids) or boundary faces (mesh face
 // ids through fa_map) whose element has constrained vertices: local matrices
 // rewritten for the constraints and scattered through n x n + n tables.
@@ -331,8 +336,8 @@ struct gbfem_ctx_s {
   // the device build leaves the element colouring to the first colour
   // scatter; the DOF -> element incidence (gather scatter) is built on demand
   bool el_colour_pending = false, have_inc = false;
-  gbfem::DevBuf<int> inc_ptr, inc;
-  gbfem::DevBuf<double> ek;  // local matrices of the gather scatter
+  gbfem::DevBuf<int> inc_ptr, inc, fa_head, fa_next;  // and the faces of each element
+  gbfem::DevBuf<double> ek, fk;  // local matrices of the gather scatter (elements, faces)
   std::vector<int> h_el_color_ptr, h_fa_color_ptr;
   gbfem::HostStructure hs;
   // the device build leaves the host copies in hs to be fetched on first use

@@ -66,23 +66,26 @@ constexpr int SELL_C = 32;
 // indices otherwise.
 __device__ __forceinline__ int sell_base(int r, int n) { return r < n ? r : n - 1; }
 
-// width[s]: the slice's longest row; fits[s]: every column within 16 bits of its base
+// width[s]: the slice's longest row; fits[s]: every column within 16 bits of its
+// base.  A lane a row, a warp a slice, four columns in flight (a thread a slice
+// walked its 32 rows one column after the other: 157,464 rows 86 us, 7.5 us so).
 __global__ void sell_width_kernel(int n, int nslices, const int *__restrict__ row_ptr, const int *__restrict__ col_ind,
                                   int *__restrict__ width, int *__restrict__ fits) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) / SELL_C, r = s * SELL_C + threadIdx.x % SELL_C;
   if (s >= nslices) return;
-  int w = 0, ok = 1;
-  for (int l = 0; l < SELL_C; l++) {
-    const int r = s * SELL_C + l;
-    if (r >= n) continue;
-    w = max(w, row_ptr[r + 1] - row_ptr[r]);
-    for (int k = row_ptr[r]; k < row_ptr[r + 1]; k++) {
-      const int d = col_ind[k] - r;
-      ok &= d >= -32768 && d <= 32767;
-    }
+  const int lo = r < n ? __ldg(row_ptr + r) : 0, hi = r < n ? __ldg(row_ptr + r + 1) : 0;
+  int ok = 1;
+#pragma unroll 4
+  for (int k = lo; k < hi; k++) {
+    const int d = __ldg(col_ind + k) - r;
+    ok &= d >= -32768 && d <= 32767;
   }
-  width[s] = w;
-  fits[s] = ok;
+  const int w = __reduce_max_sync(0xffffffffu, hi - lo);
+  ok = __all_sync(0xffffffffu, ok);
+  if (threadIdx.x % SELL_C == 0) {
+    width[s] = w;
+    fits[s] = ok;
+  }
 }
 
 // columns of slice s: entry j of lane l at off[s] + 32 j + l; padding entries
@@ -546,8 +549,8 @@ int build_sell(gbfem_ctx c) {
   const int n = c->ndof, ns = (n + gbfem::SELL_C - 1) / gbfem::SELL_C;
   if (c->sell_ready && c->sell_n == n && c->sell_nnz == c->nnz) return 0;
   GB_TRY(c->sell_off.alloc((size_t)2 * ns + 1));
-  gbfem::sell_width_kernel<<<nblk(ns, 256), 256, 0, c->stream>>>(n, ns, c->row_ptr.p, c->col_ind.p, c->sell_off.p,
-                                                                 c->sell_off.p + ns);
+  gbfem::sell_width_kernel<<<nblk((long long)ns * gbfem::SELL_C, 128), 128, 0, c->stream>>>(
+      n, ns, c->row_ptr.p, c->col_ind.p, c->sell_off.p, c->sell_off.p + ns);
   GB_CUDA(cudaGetLastError());
   std::vector<int> w(2 * (size_t)ns), off(ns + 1);
   GB_CUDA(cudaMemcpyAsync(w.data(), c->sell_off.p, 2 * (size_t)ns * sizeof(int), cudaMemcpyDeviceToHost,

@@ -16,6 +16,8 @@
 // aps_std_lin_intf.c:1537-2880 with apr_elem_calc_3D_prism, aps_std_util.c:
 // 520-820) up to rounding.
 
+#include <climits>
+
 #include "gbfem_internal.h"
 #include "prism_dw.cuh"
 #include "prism_std.cuh"
@@ -381,6 +383,42 @@ __global__ void __launch_bounds__(128) prism_faces_kernel(
 // Std linear tetrahedra (apr_elem_calc_3D_tetra, aps_std_util.c:869-1130):
 // constant Jacobian, volume |det|/6, 4-point order-2 rule with weights 1/4;
 // tables hold 20 ints (16 values + 4 rhs).
+// local matrix (upper entries row by row) and load vector of tetrahedron e
+__device__ __forceinline__ void tet_local(int e, const int *__restrict__ el_nodes, const double *__restrict__ xyz,
+                                          const double *__restrict__ k_el, double f, double (&K)[10], double (&R)[4]) {
+  const int4 n4 = __ldg(reinterpret_cast<const int4 *>(el_nodes + 4 * (size_t)e));
+  const d3 x0 = load_node(xyz, n4.x), x1 = load_node(xyz, n4.y), x2 = load_node(xyz, n4.z),
+           x3 = load_node(xyz, n4.w);
+  const d3 j1 = x1 - x0, j2 = x2 - x0, j3 = x3 - x0;
+  const d3 c1 = cross(j2, j3), c2 = cross(j3, j1), c3 = cross(j1, j2);
+  const double det = dot(j1, c1);
+  const double adet = fabs(det * 0.16666666666666666666666666666667);  // |det|/6
+  const double kk = k_el ? __ldg(k_el + e) : 1.0;
+  // k * vol / det^2 with vol = |det|/6 summed over the 4 weights 1/4
+  const double s = kk * adet / (det * det);
+  d3 g[4] = {-1.0 * (c1 + c2 + c3), c1, c2, c3};
+  int k = 0;
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    const d3 p = s * g[u];
+#pragma unroll
+    for (int w = u; w < 4; w++, k++) K[k] = dot(p, g[w]);
+  }
+  const double a = 0.585410196624969, b = 0.138196601125011;
+  // quadrature point order of apr_set_quadr_3D: (a,b,b), (b,b,a), (b,b,b), (b,a,b)
+  const double P[4][3] = {{a, b, b}, {b, b, a}, {b, b, b}, {b, a, b}};
+  const double fv = f * adet * 0.25;
+#pragma unroll
+  for (int w = 0; w < 4; w++) R[w] = 0.0;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    R[0] = fma(fv, 1.0 - P[q][0] - P[q][1] - P[q][2], R[0]);
+    R[1] = fma(fv, P[q][0], R[1]);
+    R[2] = fma(fv, P[q][1], R[2]);
+    R[3] = fma(fv, P[q][2], R[3]);
+  }
+}
+
 template <bool ATOMIC>
 __global__ void __launch_bounds__(128) tet_elements_kernel(
     int count, const int *__restrict__ ent_el, int el_base, const int *__restrict__ ent_pos, int nel,
@@ -395,53 +433,32 @@ __global__ void __launch_bounds__(128) tet_elements_kernel(
     return;
   }
   const int *tb = tab + (ent_pos ? (size_t)__ldg(ent_pos + i) : (size_t)20 * e);
-  const int4 n4 = __ldg(reinterpret_cast<const int4 *>(el_nodes + 4 * (size_t)e));
-  const d3 x0 = load_node(xyz, n4.x), x1 = load_node(xyz, n4.y), x2 = load_node(xyz, n4.z),
-           x3 = load_node(xyz, n4.w);
-  const d3 j1 = x1 - x0, j2 = x2 - x0, j3 = x3 - x0;
-  const d3 c1 = cross(j2, j3), c2 = cross(j3, j1), c3 = cross(j1, j2);
-  const double det = dot(j1, c1);
-  const double adet = fabs(det * 0.16666666666666666666666666666667);  // |det|/6
-  const double kk = k_el ? __ldg(k_el + e) : 1.0;
-  // k * vol / det^2 with vol = |det|/6 summed over the 4 weights 1/4
-  const double s = kk * adet / (det * det);
-  d3 g[4] = {-1.0 * (c1 + c2 + c3), c1, c2, c3};
+  double K[10], R[4];
+  tet_local(e, el_nodes, xyz, k_el, f, K, R);
   if (do_sm) {
+    int k = 0;
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const d3 p = s * g[u];
+    for (int u = 0; u < 4; u++)
 #pragma unroll
-      for (int w = u; w < 4; w++) {
-        const double v = dot(p, g[w]);
-        add_val<ATOMIC>(val, __ldg(tb + w + 4 * u), v);
-        if (w != u) add_val<ATOMIC>(val, __ldg(tb + u + 4 * w), v);
+      for (int w = u; w < 4; w++, k++) {
+        add_val<ATOMIC>(val, __ldg(tb + w + 4 * u), K[k]);
+        if (w != u) add_val<ATOMIC>(val, __ldg(tb + u + 4 * w), K[k]);
       }
-    }
   }
   if (do_rhs) {
-    const double a = 0.585410196624969, b = 0.138196601125011;
-    // quadrature point order of apr_set_quadr_3D: (a,b,b), (b,b,a), (b,b,b), (b,a,b)
-    const double P[4][3] = {{a, b, b}, {b, b, a}, {b, b, b}, {b, a, b}};
-    double R[4] = {0, 0, 0, 0};
-    const double fv = f * adet * 0.25;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      R[0] = fma(fv, 1.0 - P[q][0] - P[q][1] - P[q][2], R[0]);
-      R[1] = fma(fv, P[q][0], R[1]);
-      R[2] = fma(fv, P[q][1], R[2]);
-      R[3] = fma(fv, P[q][2], R[3]);
-    }
 #pragma unroll
     for (int w = 0; w < 4; w++) add_val<ATOMIC>(rhs, __ldg(tb + 16 + w), R[w]);
   }
 }
 
 // The deterministic gather scatter: each element's local matrix and load
-// vector are stored (ek[e*42 + a*6 + b] = row a, column b; ek[e*42 + 36 + a]
-// = load entry a), then one thread a row adds its row's entries over the
-// incident elements in element order, through the elements' tables.  Every
+// vector are stored (ek[e tl + a NV + b] = row a, column b; ek[e tl + NV NV + a] =
+// load entry a; tl = NV NV + NV), and each penalty face's (fk[f 14 ..]: the 10
+// upper entries over its vertices, 4 load entries); then a group of lanes a
+// row adds its row's entries over the incident elements in element order, each
+// element's faces after it in face order, through the elements' tables.  Every
 // CRS entry and rhs row has one writer and a fixed summation order, without
-// the colouring the colour scatter needs.
+// the colouring the colour scatter needs, and nothing is cleared first.
 template <bool ANISO>
 __global__ void __launch_bounds__(128) prism_elements_store_kernel(
     int nel, const int *__restrict__ el_nodes, const double *__restrict__ xyz, const double *__restrict__ k_el,
@@ -480,29 +497,141 @@ __global__ void __launch_bounds__(128) prism_elements_store_kernel(
   for (int a = 0; a < 6; a++) o[36 + a] = R[a];
 }
 
-__global__ void __launch_bounds__(128) std_gather_kernel(int nd, int nv, const int *__restrict__ inc_ptr,
-                                                         const int *__restrict__ inc, const int *__restrict__ tab,
-                                                         const double *__restrict__ ek, double *__restrict__ val,
-                                                         double *__restrict__ rhs, int *__restrict__ err) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nd) return;
-  const int tl = nv * nv + nv;
-  double racc = 0.0;
-  for (int k = __ldg(inc_ptr + r); k < __ldg(inc_ptr + r + 1); k++) {
-    const int e = __ldg(inc + k);
-    const int *tb = tab + (size_t)e * tl;
-    int a = -1;
-    for (int j = 0; j < nv; j++)
-      if (__ldg(tb + nv * nv + j) == r) a = j;
-    if (a < 0) {  // the incidence does not match the tables
-      atomicExch(err, 9);
-      return;
+__global__ void __launch_bounds__(128) tet_elements_store_kernel(
+    int nel, const int *__restrict__ el_nodes, const double *__restrict__ xyz, const double *__restrict__ k_el,
+    double f, double *__restrict__ ek) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nel) return;
+  double K[10], R[4];
+  tet_local(e, el_nodes, xyz, k_el, f, K, R);
+  double *o = ek + 20 * (size_t)e;
+  int k = 0;
+#pragma unroll
+  for (int u = 0; u < 4; u++)
+#pragma unroll
+    for (int w = u; w < 4; w++, k++) {
+      o[4 * u + w] = K[k];
+      if (w != u) o[4 * w + u] = K[k];
     }
-    const double *ke = ek + (size_t)e * tl + a * nv;
-    for (int b = 0; b < nv; b++) val[__ldg(tb + a + nv * b)] += __ldg(ke + b);
-    racc += __ldg(ek + (size_t)e * tl + nv * nv + a);
+#pragma unroll
+  for (int u = 0; u < 4; u++) o[16 + u] = R[u];
+}
+
+__global__ void __launch_bounds__(128) prism_faces_store_kernel(
+    int nfa, const int *__restrict__ fa_el, const int *__restrict__ fa_side, const int *__restrict__ el_nodes,
+    const double *__restrict__ xyz, double penalty, double g, double *__restrict__ fk) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= nfa) return;
+  const int *nd = el_nodes + 6 * (size_t)__ldg(fa_el + f);
+  d3 X[6];
+#pragma unroll
+  for (int j = 0; j < 6; j++) X[j] = load_node(xyz, __ldg(nd + j));
+  int loc[4], nloc;
+  double K[10], Rl[4];
+  prism_face_local(X, __ldg(fa_side + f), penalty, g, loc, nloc, K, Rl);
+#pragma unroll
+  for (int i = 0; i < 10; i++) fk[14 * (size_t)f + i] = K[i];
+#pragma unroll
+  for (int i = 0; i < 4; i++) fk[14 * (size_t)f + 10 + i] = g != 0.0 ? Rl[i] : 0.0;
+}
+
+// the face list of each element: head[e] (-1: none), next[f]
+__global__ void face_lists_kernel(int nfa, const int *__restrict__ fa_el, int *head, int *next) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f < nfa) next[f] = atomicExch(head + fa_el[f], f);
+}
+
+// place of local vertex v among the vertices of a prism side (prism_face_local's order), -1: not on it
+__device__ __forceinline__ int side_place(int side, int v) {
+  if (side <= 1) return v / 3 == side ? v % 3 : -1;
+  const int a = side - 2, b = (side - 1) % 3, t = v % 3;
+  return t == a ? 2 * (v / 3) : t == b ? 2 * (v / 3) + 1 : -1;
+}
+
+// GL lanes a row (lane b: column b of the incident elements), U elements'
+// loads in flight; the row is summed in shared memory (rows longer than
+// GATHER_ROW in place).  The rows of a warp take their turns together, so the
+// warp stays whole.  What is left is the latency of list -> table and matrix
+// -> sum: 157,464 rows of 315k prisms 278 us with a thread a row adding
+// through global memory, 96 us so (traffic 200 MB, 30 us; U = 4 103 us, 6 119 us).
+constexpr int GATHER_ROW = 40;
+template <int NV, int GL, int U>
+__global__ void __launch_bounds__(128) std_gather_kernel(
+    int nd, const int *__restrict__ row_ptr, const int *__restrict__ inc_ptr, const int *__restrict__ inc,
+    const int *__restrict__ tab, const double *__restrict__ ek, const int *__restrict__ fa_head,
+    const int *__restrict__ fa_next, const int *__restrict__ fa_side, const double *__restrict__ fk,
+    double *__restrict__ val, double *__restrict__ rhs) {
+  constexpr int TL = NV * NV + NV, ROWS = 128 / GL;
+  __shared__ double sacc[ROWS][GATHER_ROW];
+  const int grp = threadIdx.x / GL, b = threadIdx.x % GL, r = blockIdx.x * ROWS + grp;
+  const bool row = r < nd, twins = __ldg(inc_ptr + nd + 1) != 0;
+  const int lo = row ? __ldg(row_ptr + r) : 0, len = row ? __ldg(row_ptr + r + 1) - lo : 0;
+  const int k0 = row ? __ldg(inc_ptr + r) : 0, cnt = row ? __ldg(inc_ptr + r + 1) - k0 : 0;
+  double *acc = len <= GATHER_ROW ? sacc[grp] : val + lo;
+  for (int i = b; i < len; i += GL) acc[i] = 0.0;
+  __syncwarp();
+  double racc = 0.0;
+  const int most = __reduce_max_sync(0xffffffffu, cnt);
+  for (int t = 0; t < most; t += U) {
+    int i[U], fh[U], pos[U];
+    double ke[U], re[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) i[u] = t + u < cnt ? __ldg(inc + k0 + t + u) : -1;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      pos[u] = fh[u] = -1;
+      ke[u] = re[u] = 0.0;
+      if (i[u] < 0) continue;
+      const int e = i[u] / NV, a = i[u] - e * NV;
+      if (fa_head) fh[u] = __ldg(fa_head + e);
+      if (b < NV) {
+        pos[u] = __ldg(tab + (size_t)e * TL + a + NV * b) - lo;
+        ke[u] = __ldg(ek + (size_t)e * TL + a * NV + b);
+      }
+      if (b == 0) re[u] = __ldg(ek + (size_t)e * TL + NV * NV + a);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (t + u >= most) break;
+      if (!twins) {
+        if (pos[u] >= 0) acc[pos[u]] += ke[u];
+      } else {  // an element with a dof twice meets a column twice: one lane after the other
+        for (int v = 0; v < NV; v++) {
+          if (v == b && pos[u] >= 0) acc[pos[u]] += ke[u];
+          __syncwarp();
+        }
+      }
+      racc += re[u];
+      if (__any_sync(0xffffffffu, fh[u] >= 0)) {  // the element's faces in ascending order
+        const int a = i[u] % NV;
+        for (int last = -1; fh[u] >= 0;) {
+          int f = INT_MAX;
+          for (int q = fh[u]; q >= 0; q = __ldg(fa_next + q))
+            if (q > last && q < f) f = q;
+          if (f == INT_MAX) break;
+          last = f;
+          const int side = __ldg(fa_side + f), pa = side_place(side, a), pb = b < NV ? side_place(side, b) : -1;
+          if (pa < 0) continue;
+          const double *kf = fk + 14 * (size_t)f;
+          const int x = min(pa, pb), y = max(pa, pb);
+          const double kv = pb >= 0 ? __ldg(kf + 4 * x - x * (x - 1) / 2 + y - x) : 0.0;
+          if (!twins) {
+            if (pb >= 0) acc[pos[u]] += kv;
+          } else {
+            for (int v = 0; v < NV; v++) {
+              if (v == b && pb >= 0) acc[pos[u]] += kv;
+              __syncwarp(((1u << GL) - 1u) << ((threadIdx.x & 31) / GL * GL));
+            }
+          }
+          if (b == 0) racc += __ldg(kf + 10 + pa);
+        }
+      }
+      __syncwarp();
+    }
   }
-  rhs[r] += racc;
+  if (acc == sacc[grp])
+    for (int i = b; i < len; i += GL) val[lo + i] = acc[i];
+  if (row && b == 0) rhs[r] = racc;
 }
 
 // Elements and boundary faces whose element has constrained (hanging)
@@ -680,18 +809,38 @@ int launch_prism_faces(cudaStream_t st, bool atomic, int count, const int *ent_f
   return 1;
 }
 
-int launch_std_gather(cudaStream_t st, bool aniso, int nel, int nd, const int *el_nodes, const double *xyz,
-                      const double *k_el, const double *D_el, double f, const int *inc_ptr, const int *inc,
-                      const int *tab, double *ek, double *val, double *rhs, int *err) {
+int launch_face_lists(cudaStream_t st, int nel, int nfa, const int *fa_el, int *head, int *next) {
+  GB_CUDA(cudaMemsetAsync(head, 0xff, (size_t)nel * sizeof(int), st));
+  if (nfa > 0) face_lists_kernel<<<nblk(nfa, 128), 128, 0, st>>>(nfa, fa_el, head, next);
+  GB_CUDA(cudaGetLastError());
+  return 0;
+}
+
+int launch_std_gather(cudaStream_t st, int nv, bool aniso, int nel, int nd, const int *el_nodes, const double *xyz,
+                      const double *k_el, const double *D_el, double f, int nfa, const int *fa_el, const int *fa_side,
+                      double penalty, double g, const int *fa_head, const int *fa_next, const int *row_ptr,
+                      const int *inc_ptr, const int *inc, const int *tab, double *ek, double *fk, double *val,
+                      double *rhs) {
   if (nel <= 0) return 0;
   const int T = 128;
+  if (nv == 4) {
+    tet_elements_store_kernel<<<nblk(nel, T), T, 0, st>>>(nel, el_nodes, xyz, k_el, f, ek);
+    std_gather_kernel<4, 4, 2><<<nblk(nd, T / 4), T, 0, st>>>(nd, row_ptr, inc_ptr, inc, tab, ek, nullptr, nullptr,
+                                                           nullptr, nullptr, val, rhs);
+    GB_CUDA(cudaGetLastError());
+    return 2;
+  }
+  if (nfa > 0)
+    prism_faces_store_kernel<<<nblk(nfa, T), T, 0, st>>>(nfa, fa_el, fa_side, el_nodes, xyz, penalty, g, fk);
   if (aniso)
     prism_elements_store_kernel<true><<<nblk(nel, T), T, 0, st>>>(nel, el_nodes, xyz, k_el, D_el, f, ek);
   else
     prism_elements_store_kernel<false><<<nblk(nel, T), T, 0, st>>>(nel, el_nodes, xyz, k_el, D_el, f, ek);
-  std_gather_kernel<<<nblk(nd, T), T, 0, st>>>(nd, 6, inc_ptr, inc, tab, ek, val, rhs, err);
+  std_gather_kernel<6, 8, 2><<<nblk(nd, T / 8), T, 0, st>>>(nd, row_ptr, inc_ptr, inc, tab, ek,
+                                                         nfa > 0 ? fa_head : nullptr, fa_next, fa_side, fk, val,
+                                                              rhs);
   GB_CUDA(cudaGetLastError());
-  return 2;
+  return nfa > 0 ? 3 : 2;
 }
 
 int launch_prism_constrained(cudaStream_t st, bool faces, bool aniso, int count, const int *ent_id,

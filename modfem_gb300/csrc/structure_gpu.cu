@@ -8,8 +8,8 @@
 //     scan of a 0/1 mark at every first-appearance position
 //     (utr_get_list_dof_ent, utd_util/uts_ls_intf.c:182-300);
 //  2. DOF -> element incidence lists (count, scan, fill in any order);
-//  3. CRS rows: the DOFs of the incident elements of each row, sorted and
-//     deduplicated per row (two passes: lengths, scan, columns), diagonal
+//  3. CRS rows: the DOFs of the incident elements of each row, deduplicated
+//     and ordered by a warp a row (two passes: lengths, scan, columns), diagonal
 //     included (sis_mkb_intf.c:1128, lad_crs/las_crs_intf.c:72-300);
 //  4. element tables: for every (row dof j, column dof i) of an element the
 //     position found by binary search in row j, then the rhs rows
@@ -30,7 +30,9 @@ namespace gbfem {
 constexpr int SG_T = 256;
 constexpr int SG_PER = 8;
 constexpr int SG_CHUNK = SG_T * SG_PER;
-constexpr int SG_MAXROW = 256;  // candidate column slots per row (6 x incident elements)
+constexpr int SG_MAXROW = 256;  // columns a row may have
+constexpr int SG_ROWS = 4;      // rows (warps) a CTA of the row kernels
+constexpr int SG_HASH = 2 * SG_MAXROW;
 
 __device__ __forceinline__ int sg_block_exclusive(int v, int *total) {
   __shared__ int ws[SG_T / 32];
@@ -189,73 +191,105 @@ __global__ void sg_inc_fill(long long m, int nv, const int *__restrict__ el_dofs
     inc[atomicAdd(cursor + el_dofs[i], 1)] = (int)(i / nv);
 }
 
-// sorted unique columns of row r into buf (returns the count, or -1 if the
-// row has more candidates than SG_MAXROW)
-__device__ int sg_row(int r, int nv, const int *__restrict__ inc_ptr, const int *__restrict__ inc,
-                      const int *__restrict__ el_dofs, int *buf) {
+// The unique columns of row r, in no order, to list (shared, SG_MAXROW); returns
+// their count, -1 if there are more.  One warp: the lanes take the dofs of the
+// incident elements and enter them in a hash table in shared memory
+// (key + 1, 0 empty; the table is twice as large as the most a row may hold,
+// a smaller part of it is used where the row has few candidates).
+template <int nv>
+__device__ int sg_row(int r, const int *__restrict__ inc_ptr, const int *__restrict__ inc,
+                      const int *__restrict__ el_dofs, int *hash, int *list) {
+  const int lane = threadIdx.x & 31;
+  const int lo = __ldg(inc_ptr + r), m = (__ldg(inc_ptr + r + 1) - lo) * nv;
+  int size = 64;
+  while (size < SG_HASH && size < 2 * m) size <<= 1;
+  for (int i = lane; i < size; i += 32) hash[i] = 0;
+  __syncwarp();
   int n = 0;
-  for (int k = inc_ptr[r]; k < inc_ptr[r + 1]; k++) {
-    const int *ed = el_dofs + (size_t)inc[k] * nv;
-    for (int j = 0; j < nv; j++) {
-      if (n >= SG_MAXROW) return -1;
-      // insertion into the sorted prefix, skipping duplicates
-      const int v = ed[j];
-      int p = n;
-      while (p > 0 && buf[p - 1] > v) p--;
-      if (p > 0 && buf[p - 1] == v) continue;
-      for (int q = n; q > p; q--) buf[q] = buf[q - 1];
-      buf[p] = v;
-      n++;
+  for (int i0 = 0; i0 < m; i0 += 32) {
+    const int i = i0 + lane;
+    bool fresh = false;
+    int key = 0;
+    if (i < m) {
+      key = __ldg(el_dofs + (size_t)__ldg(inc + lo + i / nv) * nv + i % nv) + 1;
+      unsigned h = ((unsigned)key * 0x9E3779B1u) >> 16;
+      // at most SG_MAXROW + 32 of SG_HASH slots are ever taken: the walk meets a free one
+      for (int step = 0; step < SG_HASH; step++, h++) {
+        const int old = atomicCAS(hash + (h & (size - 1)), 0, key);
+        if (old == 0) fresh = true;
+        if (old == 0 || old == key) break;
+      }
     }
+    const unsigned got = __ballot_sync(0xffffffffu, fresh);
+    const int at = n + __popc(got & ((1u << lane) - 1u));
+    if (fresh && at < SG_MAXROW) list[at] = key - 1;
+    n += __popc(got);
+    if (n > SG_MAXROW) return -1;
+    __syncwarp();
   }
   return n;
 }
 
-__global__ void sg_row_len(int nd, int nv, const int *__restrict__ inc_ptr, const int *__restrict__ inc,
-                           const int *__restrict__ el_dofs, int *len, int *err) {
-  int buf[SG_MAXROW];
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// (315k prisms, 157,464 rows of 27 columns: lengths 150 us, columns 160 us with an
+// insertion sort by a thread a row in local memory; 49 and 63 us so)
+template <int nv>
+__global__ void __launch_bounds__(32 * SG_ROWS) sg_row_len(int nd, const int *__restrict__ inc_ptr,
+                                                           const int *__restrict__ inc,
+                                                           const int *__restrict__ el_dofs, int *len, int *err) {
+  __shared__ int hash[SG_ROWS][SG_HASH], list[SG_ROWS][SG_MAXROW];
+  const int w = threadIdx.x >> 5, r = blockIdx.x * SG_ROWS + w;
   if (r >= nd) return;
-  const int n = sg_row(r, nv, inc_ptr, inc, el_dofs, buf);
-  if (n < 0) {
-    atomicExch(err, 7);
-    len[r] = 0;
-  } else {
-    len[r] = n;
+  const int n = sg_row<nv>(r, inc_ptr, inc, el_dofs, hash[w], list[w]);
+  if ((threadIdx.x & 31) == 0) {
+    if (n < 0) atomicExch(err, 7);
+    len[r] = max(n, 0);
   }
 }
 
-__global__ void sg_row_fill(int nd, int nv, const int *__restrict__ inc_ptr, const int *__restrict__ inc,
-                            const int *__restrict__ el_dofs, const int *__restrict__ row_ptr, int *col_ind) {
-  int buf[SG_MAXROW];
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// every column to its rank among the row's
+template <int nv>
+__global__ void __launch_bounds__(32 * SG_ROWS) sg_row_fill(int nd, const int *__restrict__ inc_ptr,
+                                                            const int *__restrict__ inc,
+                                                            const int *__restrict__ el_dofs,
+                                                            const int *__restrict__ row_ptr, int *col_ind) {
+  __shared__ int hash[SG_ROWS][SG_HASH], list[SG_ROWS][SG_MAXROW];
+  const int w = threadIdx.x >> 5, r = blockIdx.x * SG_ROWS + w;
   if (r >= nd) return;
-  const int n = sg_row(r, nv, inc_ptr, inc, el_dofs, buf);
-  for (int i = 0; i < n && row_ptr[r] + i < row_ptr[r + 1]; i++) col_ind[row_ptr[r] + i] = buf[i];
+  const int n = sg_row<nv>(r, inc_ptr, inc, el_dofs, hash[w], list[w]), lo = __ldg(row_ptr + r);
+  for (int i = threadIdx.x & 31; i < n; i += 32) {
+    const int v = list[w][i];
+    int rank = 0;
+    for (int j = 0; j < n; j++) rank += list[w][j] < v;
+    if (lo + rank < __ldg(row_ptr + r + 1)) col_ind[lo + rank] = v;
+  }
 }
 
-__global__ void sg_tables(int nel, int nv, const int *__restrict__ el_dofs, const int *__restrict__ row_ptr,
-                          const int *__restrict__ col_ind, int *table) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nel) return;
-  const int tl = nv * nv + nv;
+// a thread an entry (a thread an element searched its nv nv pairs one after the
+// other: 315k prisms 128 us, 95 us so)
+template <int nv>
+__global__ void __launch_bounds__(256) sg_tables(long long entries, const int *__restrict__ el_dofs,
+                                                 const int *__restrict__ row_ptr, const int *__restrict__ col_ind,
+                                                 int *__restrict__ table) {
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= entries) return;
+  constexpr int tl = nv * nv + nv;
+  const int e = (int)(k / tl), q = (int)(k - (long long)e * tl);
   const int *ed = el_dofs + (size_t)e * nv;
-  int *t = table + (size_t)e * tl;
-  for (int j = 0; j < nv; j++) {
-    const int r = ed[j];
-    for (int i = 0; i < nv; i++) {
-      int lo = row_ptr[r], hi = row_ptr[r + 1];  // first position with col >= ed[i]
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (col_ind[mid] < ed[i])
-          lo = mid + 1;
-        else
-          hi = mid;
-      }
-      t[j + i * nv] = lo;
+  const int r = __ldg(ed + q % nv);
+  int at = r;
+  if (q < nv * nv) {  // first position of row r (dof j = q % nv) with a column >= dof i
+    const int c = __ldg(ed + q / nv);
+    int hi = __ldg(row_ptr + r + 1);
+    at = __ldg(row_ptr + r);
+    while (at < hi) {
+      const int mid = (at + hi) >> 1;
+      if (__ldg(col_ind + mid) < c)
+        at = mid + 1;
+      else
+        hi = mid;
     }
-    t[nv * nv + j] = r;
   }
+  table[k] = at;
 }
 
 // Element colouring for the deterministic colour-batched scatter: elements
@@ -284,7 +318,7 @@ __global__ void sg_jp_round(int nel, int nv, int rnd, const int *__restrict__ el
   for (int j = 0; j < nv && wins; j++) {
     const int d = el_dofs[(size_t)e * stride + j];
     for (int k = inc_ptr[d]; k < inc_ptr[d + 1]; k++) {
-      const int f = inc[k];
+      const int f = inc[k] / nv;
       if (f == e) continue;
       const int sf = ((volatile int *)state)[f];
       if (sf >= 0 && (sf >> 8) < rnd) {
@@ -353,7 +387,8 @@ int build_device_structure(cudaStream_t st, int nno, int nel, int nv, const int 
   sg_inc_fill<<<g1, 256, 0, st>>>(m, nv, el_dofs.p, inc_cnt.p, inc.p);
   // 3. rows
   if (len.alloc((size_t)nd + 1) < 0 || row_ptr.alloc((size_t)nd + 1) < 0) return fail(-1);
-  sg_row_len<<<(nd + 127) / 128, 128, 0, st>>>(nd, nv, inc_ptr.p, inc.p, el_dofs.p, len.p, err);
+  auto row_len = nv == 6 ? sg_row_len<6> : sg_row_len<4>;
+  row_len<<<(nd + SG_ROWS - 1) / SG_ROWS, 32 * SG_ROWS, 0, st>>>(nd, inc_ptr.p, inc.p, el_dofs.p, len.p, err);
   if (sg_scan(st, nd, len.p, row_ptr.p, tmp) < 0) return fail(-1);
   int nnz = 0, herr = 0;
   GB_CUDA(cudaMemcpyAsync(&nnz, row_ptr.p + nd, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -364,10 +399,15 @@ int build_device_structure(cudaStream_t st, int nno, int nel, int nv, const int 
     GB_CHECK(false, "a vertex has more neighbours than the device structure build supports");
   }
   if (col_ind.alloc((size_t)nnz) < 0) return fail(-1);
-  sg_row_fill<<<(nd + 127) / 128, 128, 0, st>>>(nd, nv, inc_ptr.p, inc.p, el_dofs.p, row_ptr.p, col_ind.p);
+  auto row_fill = nv == 6 ? sg_row_fill<6> : sg_row_fill<4>;
+  row_fill<<<(nd + SG_ROWS - 1) / SG_ROWS, 32 * SG_ROWS, 0, st>>>(nd, inc_ptr.p, inc.p, el_dofs.p, row_ptr.p,
+                                                                 col_ind.p);
   // 4. element tables
   if (el_table.alloc((size_t)nel * (nv * nv + nv)) < 0) return fail(-1);
-  sg_tables<<<(nel + 127) / 128, 128, 0, st>>>(nel, nv, el_dofs.p, row_ptr.p, col_ind.p, el_table.p);
+  const long long entries = (long long)nel * (nv * nv + nv);
+  auto tables = nv == 6 ? sg_tables<6> : sg_tables<4>;
+  tables<<<(unsigned)((entries + 255) / 256), 256, 0, st>>>(entries, el_dofs.p, row_ptr.p, col_ind.p,
+                                                            el_table.p);
   GB_CUDA(cudaGetLastError());
   GB_CUDA(cudaStreamSynchronize(st));
   cleanup();
@@ -378,24 +418,44 @@ int build_device_structure(cudaStream_t st, int nno, int nel, int nv, const int 
 
 
 // Incidence from the element tables (the rhs rows t[nv*nv + j] are the
-// element's dofs): count, scan, fill, then each list sorted by element.
-__global__ void sg_inc_count_tab(int nel, int nv, const int *__restrict__ table, int *cnt) {
-  const long long m = (long long)nel * nv, tl = nv * nv + nv;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < m; i += (long long)gridDim.x * blockDim.x)
-    atomicAdd(cnt + table[(i / nv) * tl + nv * nv + i % nv], 1);
+// element's dofs): count, scan, fill, then each list sorted.  An entry is
+// e nv + a, a the local vertex; *twins is set if an element has a dof twice.
+template <int nv>
+__global__ void sg_inc_count_tab(long long m, const int *__restrict__ table, int *cnt, int *twins) {
+  constexpr int tl = nv * nv + nv;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < m; i += (long long)gridDim.x * blockDim.x) {
+    const int *d = table + (i / nv) * tl + nv * nv;
+    const int j = (int)(i % nv), v = __ldg(d + j);
+    atomicAdd(cnt + v, 1);
+    bool again = false;
+    for (int k = 0; k < j; k++) again |= __ldg(d + k) == v;
+    if (again) *twins = 1;
+  }
 }
 
-__global__ void sg_inc_fill_tab(int nel, int nv, const int *__restrict__ table, int *cursor, int *inc) {
-  const long long m = (long long)nel * nv, tl = nv * nv + nv;
+template <int nv>
+__global__ void sg_inc_fill_tab(long long m, const int *__restrict__ table, int *cursor, int *inc) {
+  constexpr int tl = nv * nv + nv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < m; i += (long long)gridDim.x * blockDim.x)
-    inc[atomicAdd(cursor + table[(i / nv) * tl + nv * nv + i % nv], 1)] = (int)(i / nv);
+    inc[atomicAdd(cursor + table[(i / nv) * tl + nv * nv + i % nv], 1)] = (int)i;
 }
 
+// A warp a list: up to 32 entries go to their ranks, longer ones are sorted by
+// one lane (157,464 lists of 12: 53 us by a thread a list, 27 us so).
 __global__ void sg_inc_sort(int nd, const int *__restrict__ inc_ptr, int *inc) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= nd) return;
   int *a = inc + inc_ptr[r];
   const int n = inc_ptr[r + 1] - inc_ptr[r];
+  if (n <= 32) {
+    const int v = lane < n ? a[lane] : 0;
+    int rank = 0;
+    for (int j = 0; j < n; j++) rank += __shfl_sync(0xffffffffu, v, j) < v;
+    __syncwarp();
+    if (lane < n) a[rank] = v;
+    return;
+  }
+  if (lane) return;
   for (int i = 1; i < n; i++) {
     const int v = a[i];
     int j = i;
@@ -411,15 +471,19 @@ int build_device_incidence(cudaStream_t st, int nel, int nv, const int *el_table
                            DevBuf<int> &inc) {
   const long long m = (long long)nel * nv;
   SgTemp<int> cnt(st), tmp(st);
-  if (cnt.alloc((size_t)nd + 1) < 0 || inc_ptr.alloc((size_t)nd + 1) < 0 || inc.alloc((size_t)std::max(m, 1LL)) < 0)
+  // (inc_ptr[nd + 1]: the flag of elements with a dof twice)
+  if (cnt.alloc((size_t)nd + 1) < 0 || inc_ptr.alloc((size_t)nd + 2) < 0 || inc.alloc((size_t)std::max(m, 1LL)) < 0)
     return -1;
   const int g1 = 152 * 8;
   GB_CUDA(cudaMemsetAsync(cnt.p, 0, ((size_t)nd + 1) * sizeof(int), st));
-  sg_inc_count_tab<<<g1, 256, 0, st>>>(nel, nv, el_table, cnt.p);
+  GB_CUDA(cudaMemsetAsync(inc_ptr.p + nd + 1, 0, sizeof(int), st));
+  auto count = nv == 6 ? sg_inc_count_tab<6> : sg_inc_count_tab<4>;
+  count<<<g1, 256, 0, st>>>(m, el_table, cnt.p, inc_ptr.p + nd + 1);
   if (sg_scan(st, nd, cnt.p, inc_ptr.p, tmp) < 0) return -1;
   GB_CUDA(cudaMemcpyAsync(cnt.p, inc_ptr.p, (size_t)nd * sizeof(int), cudaMemcpyDeviceToDevice, st));
-  sg_inc_fill_tab<<<g1, 256, 0, st>>>(nel, nv, el_table, cnt.p, inc.p);
-  sg_inc_sort<<<(nd + 127) / 128, 128, 0, st>>>(nd, inc_ptr.p, inc.p);
+  auto fill = nv == 6 ? sg_inc_fill_tab<6> : sg_inc_fill_tab<4>;
+  fill<<<g1, 256, 0, st>>>(m, el_table, cnt.p, inc.p);
+  sg_inc_sort<<<(unsigned)(((long long)nd * 32 + 255) / 256), 256, 0, st>>>(nd, inc_ptr.p, inc.p);
   GB_CUDA(cudaGetLastError());
   // the scratch is released in stream order: nothing here waits for the device
   return 0;
