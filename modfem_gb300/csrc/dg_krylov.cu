@@ -21,114 +21,153 @@
 namespace gbfem {
 
 // Gauss-Jordan inversion with partial pivoting (largest magnitude, first
-// index on ties) of the diagonal blocks of one class, each block held in
-// shared memory by a group of G threads: a warp up to 40 functions (p = 3: 17
-// blocks per SM, no CTA barriers), four warps for 75.  n^3 FMA a block bound
-// it by the FP64 pipe (p = 3: 2,000 of 2,400 FP64 warp instructions); the
-// pivot search compares bit patterns on the integer pipe.  54,000 blocks of
-// 40: 16.1 ms with 256 threads and five barriers a step, 13.8 ms so.
+// row on ties) of the diagonal blocks of one class, each block in the registers
+// of a group of GA x GB lanes (lane (a, b): rows a + GA s, columns b + GB u).
+// Rows are not exchanged: step k takes its pivot from row r_k of those left
+// and exchanges unknown k with right hand side r_k, so that in the end
+// inverse[k][r_j] = entry (r_k, j).  The pivot column (f) and row (p) pass
+// through shared memory and leave zeros behind; with g_i = f_i / pivot,
+// g_r = -1 / pivot and p_k = 1 the whole step is entry (i, j) -= g_i p_j.  n^3 FMA
+// a block bound it by the FP64 pipe (p = 3: 2,000 of 2,500 FP64 warp
+// instructions, 54,000 blocks 6.9 ms); held in shared memory, three loads and a store an
+// FMA, the pipe stood half idle: 13.8 ms, 6.7 ms so.  (21,296 prisms of p = 1..4
+// 52, 504, 2,695, 19,765 us, 20,250 tetrahedra 33, 106, 530, 2,042 us; one CTA a
+// block in shared memory 581, 1,886, 6,317, 25,931 and 384, 919, 2,030, 4,798 us.)
 template <int P>
 struct DgInv {
   static constexpr int NS = DgSpmvDims<P>::NS;
-  static constexpr int G = NS > 40 ? 128 : 32;            // threads per block
-  static constexpr int CTA = 128, PER = CTA / G;          // blocks per CTA
-  static constexpr int SZ = NS * NS + 2 * NS + (NS + 1) / 2 + 1;  // doubles per block
-  static constexpr int BYTES = 8 * SZ * PER;
+  static constexpr int GA = NS > 40 ? 16 : NS > 10 ? 8 : NS > 6 ? 4 : 2;
+  static constexpr int GB = NS > 40 ? 8 : NS > 6 ? 4 : 2;
+  static constexpr int G = GA * GB, W = G < 32 ? G : 32;    // lanes a block; of those that search the pivot
+  static constexpr int R = (NS + GA - 1) / GA, C = (NS + GB - 1) / GB, Q = (NS + W - 1) / W;
+  static constexpr int CTA = 128, PER = CTA / G;            // blocks per CTA
 };
 
 template <int P>
-__global__ void __launch_bounds__(DgInv<P>::CTA) dg_block_inverse_kernel(
+__global__ void __launch_bounds__(DgInv<P>::CTA, 3) dg_block_inverse_kernel(
     int count, const int *__restrict__ ent_el, const long long *__restrict__ boff_diag, const double *__restrict__ val,
     const long long *__restrict__ dinv_off, double *__restrict__ dinv, int *err) {
   using D = DgInv<P>;
-  constexpr int n = D::NS, G = D::G;
-  extern __shared__ double smem[];
-  const int grp = threadIdx.x / G, l = threadIdx.x % G, lane = threadIdx.x % 32;
+  constexpr int n = D::NS, GA = D::GA, GB = D::GB, G = D::G, W = D::W, R = D::R, C = D::C, Q = D::Q;
+  __shared__ double sf[D::PER][n], sg[D::PER][R * GA], sp[D::PER][C * GB];
+  __shared__ int srow[D::PER][n], sstep[D::PER][n];
+  const int grp = threadIdx.x / G, l = threadIdx.x % G, a = l % GA, b = l / GA, lw = threadIdx.x % W;
+  const unsigned mask = W == 32 ? ~0u : ((1u << (W & 31)) - 1u) << ((threadIdx.x & 31) / W * W);
   const int idx = blockIdx.x * D::PER + grp;
-  if (idx >= count) return;  // whole warps (or the whole CTA)
-  const int e = ent_el[idx];
-  double *a = smem + (size_t)grp * D::SZ, *fcol = a + n * n, *prow = fcol + n;
-  int *piv = reinterpret_cast<int *>(prow + n);
+  const int e = ent_el[min(idx, count - 1)];  // a group beyond the last block computes along and writes nothing
+  double *f = sf[grp], *g = sg[grp], *p = sp[grp];
   auto sync = [] {
-    if (G == 32)
+    if (G <= 32)
       __syncwarp();
     else
       __syncthreads();
   };
   const double *src = val + boff_diag[e];
-  for (int t = l; t < n * n; t += G) a[t] = src[t];
-  sync();
+  double A[R][C];
+#pragma unroll
+  for (int s = 0; s < R; s++)
+#pragma unroll
+    for (int u = 0; u < C; u++) {
+      const int i = a + GA * s, j = b + GB * u;
+      A[s][u] = i < n && j < n ? src[i + n * j] : 0.0;
+    }
+  for (int i = l; i < R * GA; i += G) g[i] = 0.0;
+  for (int j = l; j < C * GB; j += G) p[j] = 0.0;
+  unsigned used = 0;  // bit q: row lw + W q has been a pivot row
+  bool singular = false;
+#pragma unroll 1
   for (int k = 0; k < n; k++) {
+    const int ku = b == k % GB ? k / GB : -1;
+#pragma unroll
+    for (int s = 0; s < R; s++) {
+#pragma unroll
+      for (int u = 0; u < C; u++)
+        if (u == ku) {
+          if (a + GA * s < n) f[a + GA * s] = A[s][u];
+          A[s][u] = 0.0;
+        }
+    }
+    sync();
     // every warp of the group finds the same pivot row: magnitudes as
     // integers (a NaN is never chosen), a zero column has none
-    long long best = 0;
+    double fv[Q];
+    unsigned long long best = 0;
     int r = n;
-    for (int i = k + lane; i < n; i += 32) {
-      const long long v = __double_as_longlong(a[i + n * k]) & 0x7fffffffffffffffll;
-      if (v > best && v <= 0x7ff0000000000000ll) {
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      const int i = lw + W * q;
+      fv[q] = i < n ? f[i] : 0.0;
+      const unsigned long long v = (unsigned long long)__double_as_longlong(fv[q]) & 0x7fffffffffffffffull;
+      if (!(used >> q & 1u) && v > best && v <= 0x7ff0000000000000ull) {
         best = v;
         r = i;
       }
     }
+    const unsigned hi = __reduce_max_sync(mask, (unsigned)(best >> 32));
+    const unsigned lo = __reduce_max_sync(mask, (unsigned)(best >> 32) == hi ? (unsigned)best : 0u);
+    r = __reduce_min_sync(mask, best == ((unsigned long long)hi << 32 | lo) ? r : n);
+    if (r >= n) {  // singular diagonal block (the same for the whole group)
+      singular = true;
+      r = 0;
+    }
+    if (r % W == lw) used |= 1u << (r / W);
+    const double pinv = 1.0 / f[r];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const long long ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, r, o);
-      if (ov > best || (ov == best && oi < r)) {
-        best = ov;
-        r = oi;
-      }
+    for (int q = 0; q < Q; q++) {
+      const int i = lw + W * q;
+      if (i < n && l < W) g[i] = i == r ? -pinv : fv[q] * pinv;
     }
-    if (r >= n) {  // singular diagonal block (uniform across the group)
-      if (l == 0) atomicExch(err, 3);
-      return;
+    const int rs = a == r % GA ? r / GA : -1;
+#pragma unroll
+    for (int s = 0; s < R; s++) {
+#pragma unroll
+      for (int u = 0; u < C; u++)
+        if (s == rs) {
+          const int j = b + GB * u;
+          if (j < n) p[j] = j == k ? 1.0 : A[s][u];
+          A[s][u] = 0.0;
+        }
     }
-    if (l == 0) piv[k] = r;
-    const double pinv = 1.0 / a[r + n * k];
-    // column k with rows k and r exchanged
-    for (int i = l; i < n; i += G) fcol[i] = a[(i == r ? k : i) + n * k];
-    sync();
-    for (int j = l; j < n; j += G) {
-      const double x = j == k ? pinv : a[r + n * j] * pinv;
-      a[r + n * j] = a[k + n * j];
-      a[k + n * j] = x;
-      prow[j] = x;
+    if (l == 0) {
+      srow[grp][k] = r;
+      sstep[grp][r] = k;
     }
     sync();
-    for (int t = l; t < n * n; t += G) {
-      const int j = t / n, i = t - j * n;
-      if (i == k) continue;
-      a[t] = j == k ? -fcol[i] * pinv : fma(-fcol[i], prow[j], a[t]);
-    }
-    sync();
+    double gi[R], pj[C];
+#pragma unroll
+    for (int s = 0; s < R; s++) gi[s] = -g[a + GA * s];
+#pragma unroll
+    for (int u = 0; u < C; u++) pj[u] = p[b + GB * u];
+#pragma unroll
+    for (int s = 0; s < R; s++)
+#pragma unroll
+      for (int u = 0; u < C; u++) A[s][u] = fma(gi[s], pj[u], A[s][u]);
   }
-  // undo the row interchanges as column interchanges, last first
-  for (int k = n - 1; k >= 0; k--) {
-    const int r = piv[k];
-    if (r != k)
-      for (int i = l; i < n; i += G) {
-        const double t = a[i + n * k];
-        a[i + n * k] = a[i + n * r];
-        a[i + n * r] = t;
-      }
-    sync();
+  if (idx >= count) return;
+  if (singular) {
+    if (l == 0) atomicExch(err, 3);
+    return;
   }
   double *dst = dinv + dinv_off[e];
-  for (int t = l; t < n * n; t += G) dst[t] = a[t];
+#pragma unroll
+  for (int s = 0; s < R; s++) {
+    const int i = a + GA * s;
+    if (i >= n) continue;
+    const int row = sstep[grp][i];
+#pragma unroll
+    for (int u = 0; u < C; u++) {
+      const int j = b + GB * u;
+      if (j < n) dst[row + n * srow[grp][j]] = A[s][u];
+    }
+  }
 }
 
 int launch_dg_block_inverse(cudaStream_t st, int cls, int count, const int *ent_el, const long long *boff_diag,
                             const double *val, const long long *dinv_off, double *dinv, int *err) {
   if (count <= 0) return 0;
-#define GB_INV(PP)                                                                                              \
-  {                                                                                                             \
-    using D = DgInv<PP>;                                                                                        \
-    GB_CUDA(cudaFuncSetAttribute(dg_block_inverse_kernel<PP>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                                 D::BYTES));                                                                    \
-    dg_block_inverse_kernel<PP><<<(count + D::PER - 1) / D::PER, D::CTA, D::BYTES, st>>>(count, ent_el,         \
-                                                                                         boff_diag, val,        \
-                                                                                         dinv_off, dinv, err);  \
-  }
+#define GB_INV(PP)                                                                                             \
+  dg_block_inverse_kernel<PP><<<(count + DgInv<PP>::PER - 1) / DgInv<PP>::PER, DgInv<PP>::CTA, 0, st>>>(       \
+      count, ent_el, boff_diag, val, dinv_off, dinv, err);
   switch (cls) {
     case 1: GB_INV(1) break;
     case 2: GB_INV(2) break;
