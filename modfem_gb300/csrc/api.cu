@@ -2139,7 +2139,7 @@ static int gmres_run(gbfem_ctx c, int n, int krylov, int max_iter, double tol_re
   GB_TRY(c->tmp.alloc(n));
   GB_TRY(c->hcol.alloc(m + 2));
   const int nb = gbfem::reduction_blocks(n);
-  GB_TRY(c->partial.alloc((size_t)nb * (m + 2)));
+  GB_TRY(c->partial.alloc(std::max((size_t)nb * (m + 2), (size_t)n / 1024 + 1)));
   cudaStream_t st = c->stream;
   // x == NULL: the solution stays in c->x (zeroed when ini_zero)
   if (ini_zero)
@@ -2164,7 +2164,7 @@ static int gmres_run(gbfem_ctx c, int n, int krylov, int max_iter, double tol_re
     if (beta0 < 0) beta0 = rn;
     resid = rn;
     if (rn < tol_abs || (beta0 > 0 && rn / beta0 < tol_rel) || it >= max_iter) break;
-    GB_COUNT(gbfem::launch_scale(st, n, c->hcol.p, 1, c->tmp.p, c->V.p));
+    GB_COUNT(gbfem::launch_normalize(st, n, c->hcol.p, c->tmp.p, c->V.p));
     s[0] = rn;
     for (int i = 1; i <= m; i++) s[i] = 0.0;
     int done = 0;
@@ -2177,10 +2177,9 @@ static int gmres_run(gbfem_ctx c, int n, int krylov, int max_iter, double tol_re
       cudaEventRecord(c->ev3, st);
       // classical Gram-Schmidt: h = V^T w, w -= V h, h_{j+1} = |w|
       GB_COUNT(gbfem::launch_multidot(st, n, j + 1, c->V.p, ld, w, c->partial.p, c->hcol.p, 0));
-      GB_COUNT(gbfem::launch_multiaxpy(st, n, j + 1, c->hcol.p, -1.0, c->V.p, ld, w));
-      GB_COUNT(gbfem::launch_multidot(st, n, 1, w, ld, w, c->partial.p, c->hcol.p + j + 1, 1));
+      GB_COUNT(gbfem::launch_orthogonalize(st, n, j + 1, c->hcol.p, c->V.p, ld, w, c->partial.p, c->hcol.p + j + 1));
       GB_CUDA(cudaMemcpyAsync(hh.data(), c->hcol.p, (j + 2) * sizeof(double), cudaMemcpyDeviceToHost, st));
-      GB_COUNT(gbfem::launch_scale(st, n, c->hcol.p + j + 1, 1, w, w));
+      GB_COUNT(gbfem::launch_normalize(st, n, c->hcol.p + j + 1, w, w));
       GB_CUDA(cudaStreamSynchronize(st));
       {
         float ms = 0.f;

@@ -10,6 +10,7 @@
 // tree order), so GMRES is bit-reproducible run to run.
 
 #include "gbfem_internal.h"
+#include "gmres_step.cuh"
 
 namespace gbfem {
 
@@ -53,27 +54,51 @@ __global__ void jacobi_diag_kernel(int n, const int *__restrict__ row_ptr, const
   dinv[r] = d;
 }
 
-// partial[k*nb + blockIdx.x] = sum over this block's rows of A_k[i] * w[i],
-// A_k = base + k*ld, for k = blockIdx.y.
-__global__ void __launch_bounds__(RED_THREADS) multidot_stage1(int n, const double *__restrict__ base,
-                                                               long long ld, const double *__restrict__ w,
-                                                               double *__restrict__ partial) {
-  const int k = blockIdx.y, nb = gridDim.x;
-  const double *a = base + (size_t)k * ld;
-  double s = 0.0;
-  for (long long i = (long long)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (long long)nb * RED_THREADS)
-    s = fma(__ldg(a + i), __ldg(w + i), s);
-  __shared__ double sh[RED_THREADS / 32];
+// t[u] = this thread's share of <A_u, w>, u < K (exactly K: a predicated FMA
+// costs the FP64 pipe as much as a needed one)
+template <int K>
+__device__ __forceinline__ void dots_rows(long long n, const double *__restrict__ a, long long ld,
+                                          const double *__restrict__ w, double (&t)[8]) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    s = threadIdx.x < RED_THREADS / 32 ? sh[threadIdx.x] : 0.0;
+  for (int u = 0; u < 8; u++) t[u] = 0.0;
+  for (long long i = (long long)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (long long)gridDim.x * RED_THREADS) {
+    const double wi = __ldg(w + i);
+    double x[K];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) partial[(size_t)k * nb + blockIdx.x] = s;
+    for (int u = 0; u < K; u++) x[u] = __ldg(a + u * ld + i);
+#pragma unroll
+    for (int u = 0; u < K; u++) t[u] = fma(x[u], wi, t[u]);
   }
+}
+
+// partial[k*nb + blockIdx.x] = sum over this block's rows of A_k[i] * w[i],
+// A_k = base + k*ld, for the (up to eight) vectors of chunk blockIdx.y, which
+// read w once.  Bound by HBM and, with one FMA a value, nearly as much by the
+// FP64 pipe.  2.16M rows, 1 to 20 vectors: 72 us a call on average with a block
+// row a vector, 51 us so.
+__global__ void __launch_bounds__(RED_THREADS, 5) multidot_stage1(int n, int m, const double *__restrict__ base,
+                                                                  long long ld, const double *__restrict__ w,
+                                                                  double *__restrict__ partial) {
+  constexpr int W = RED_THREADS / 32;
+  __shared__ double sh[W][8];
+  const int k0 = blockIdx.y * 8, nb = gridDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double *a = base + (size_t)k0 * ld;
+  double t[8];
+  switch (m - k0) {
+    case 1: dots_rows<1>(n, a, ld, w, t); break;
+    case 2: dots_rows<2>(n, a, ld, w, t); break;
+    case 3: dots_rows<3>(n, a, ld, w, t); break;
+    case 4: dots_rows<4>(n, a, ld, w, t); break;
+    case 5: dots_rows<5>(n, a, ld, w, t); break;
+    case 6: dots_rows<6>(n, a, ld, w, t); break;
+    case 7: dots_rows<7>(n, a, ld, w, t); break;
+    default: dots_rows<8>(n, a, ld, w, t); break;
+  }
+  const double d = gm_warp_sums(t, lane);  // lane 4 u: vector u
+  if ((lane & 3) == 0) sh[warp][lane >> 2] = d;
+  __syncthreads();
+  if (threadIdx.x < 8 && k0 + threadIdx.x < m)
+    partial[(size_t)(k0 + threadIdx.x) * nb + blockIdx.x] = gm_pairs<W>(&sh[0][threadIdx.x], 8);
 }
 
 // out[k] = sum_b partial[k*nb + b]; if sqrt_out, out[k] = sqrt(sum).
@@ -95,24 +120,61 @@ __global__ void __launch_bounds__(RED_THREADS) multidot_stage2(int nb, const dou
   }
 }
 
-// y[i] += sign * sum_{k<m} c[k] * A_k[i]   (c on the device)
-__global__ void __launch_bounds__(256) multiaxpy_kernel(int n, int m, const double *__restrict__ c, double sign,
-                                                        const double *__restrict__ base, long long ld,
-                                                        double *__restrict__ y) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double s = 0.0;
-  for (int k = 0; k < m; k++) s = fma(__ldg(c + k), __ldg(base + (size_t)k * ld + i), s);
-  y[i] = fma(sign, s, y[i]);
+// y[i] += sign * sum_{k<m} c[k] * A_k[i]   (c on the device); NORM: and
+// partial[blockIdx.x] = sum of this block's y[i]^2 (a pass over y less).  Four
+// rows a thread: a warp sum is six FP64 instructions, as many as six vectors of
+// one row.  2.16M rows, 1 to 20 vectors, update and norm: 58 us on average in
+// two passes, 57 us so.
+constexpr int AXPY_ROWS = 4;
+template <bool NORM>
+__global__ void __launch_bounds__(RED_THREADS) multiaxpy_kernel(int n, int m, const double *__restrict__ c,
+                                                                double sign, const double *__restrict__ base,
+                                                                long long ld, double *__restrict__ y,
+                                                                double *__restrict__ partial) {
+  constexpr int W = RED_THREADS / 32, R = AXPY_ROWS;
+  const long long i0 = (long long)blockIdx.x * (R * RED_THREADS) + threadIdx.x;
+  double s[R], sq = 0.0;
+#pragma unroll
+  for (int q = 0; q < R; q++) s[q] = 0.0;
+  if (i0 + (R - 1) * RED_THREADS < n) {
+#pragma unroll 2
+    for (int k = 0; k < m; k++) {
+      const double ck = __ldg(c + k), *a = base + (size_t)k * ld + i0;
+#pragma unroll
+      for (int q = 0; q < R; q++) s[q] = fma(ck, __ldg(a + q * RED_THREADS), s[q]);
+    }
+  } else {
+    for (int k = 0; k < m; k++)
+#pragma unroll
+      for (int q = 0; q < R; q++)
+        if (i0 + q * RED_THREADS < n)
+          s[q] = fma(__ldg(c + k), __ldg(base + (size_t)k * ld + i0 + q * RED_THREADS), s[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < R; q++) {
+    const long long i = i0 + q * RED_THREADS;
+    if (i >= n) break;
+    const double v = fma(sign, s[q], y[i]);
+    y[i] = v;
+    if (NORM) sq = fma(v, v, sq);
+  }
+  if (NORM) {
+    __shared__ double sh[W];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = sq;
+    __syncthreads();
+    if (threadIdx.x == 0) partial[blockIdx.x] = gm_pairs<W>(sh, 1);
+  }
 }
 
-// y[i] = alpha[0]^(power) * y[i] with power -1: divide by alpha; used to normalise.
-__global__ void scale_kernel(int n, const double *__restrict__ alpha, int invert, const double *__restrict__ x,
-                             double *__restrict__ y) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double a = *alpha;
-  y[i] = invert ? x[i] / a : x[i] * a;
+// y = x / alpha[0], the division once a thread (2.16M rows: 33 us with one a
+// row, which the FP64 pipe bounds; 11 us so)
+__global__ void __launch_bounds__(RED_THREADS) scale_kernel(int n, const double *__restrict__ alpha, const double *x,
+                                                            double *y) {
+  const double inv = 1.0 / *alpha;
+  for (long long i = (long long)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (long long)gridDim.x * RED_THREADS)
+    y[i] = x[i] * inv;
 }
 
 // v = dinv .* (b - A x)  fused: first residual then scale (two kernels for clarity)
@@ -145,8 +207,8 @@ int launch_jacobi_diag(cudaStream_t st, int n, const int *row_ptr, const int *co
 }
 
 int reduction_blocks(int n) {
-  int nb = (int)nblk(n, RED_THREADS * 8);
-  if (nb > 1216) nb = 1216;  // 8 x 152 SMs
+  int nb = (int)nblk(n, RED_THREADS * 2);
+  if (nb > 760) nb = 760;  // 5 x 152 SMs
   if (nb < 1) nb = 1;
   return nb;
 }
@@ -155,8 +217,7 @@ int reduction_blocks(int n) {
 int launch_multidot(cudaStream_t st, int n, int m, const double *base, long long ld, const double *w,
                     double *partial, double *out, int sqrt_out) {
   const int nb = reduction_blocks(n);
-  dim3 g1(nb, m);
-  multidot_stage1<<<g1, RED_THREADS, 0, st>>>(n, base, ld, w, partial);
+  multidot_stage1<<<dim3(nb, (m + 7) / 8), RED_THREADS, 0, st>>>(n, m, base, ld, w, partial);
   multidot_stage2<<<m, RED_THREADS, 0, st>>>(nb, partial, out, sqrt_out);
   GB_CUDA(cudaGetLastError());
   return 2;
@@ -165,13 +226,24 @@ int launch_multidot(cudaStream_t st, int n, int m, const double *base, long long
 int launch_multiaxpy(cudaStream_t st, int n, int m, const double *c, double sign, const double *base,
                      long long ld, double *y) {
   if (m <= 0) return 0;
-  multiaxpy_kernel<<<nblk(n, 256), 256, 0, st>>>(n, m, c, sign, base, ld, y);
+  multiaxpy_kernel<false><<<nblk(n, RED_THREADS * AXPY_ROWS), RED_THREADS, 0, st>>>(n, m, c, sign, base, ld, y, nullptr);
   GB_CUDA(cudaGetLastError());
   return 1;
 }
 
-int launch_scale(cudaStream_t st, int n, const double *alpha, int invert, const double *x, double *y) {
-  scale_kernel<<<nblk(n, 256), 256, 0, st>>>(n, alpha, invert, x, y);
+// w -= sum_{k<m} h[k] A_k, *norm = |w|; partial must hold n / 1024 + 1 doubles
+int launch_orthogonalize(cudaStream_t st, int n, int m, const double *h, const double *base, long long ld, double *w,
+                         double *partial, double *norm) {
+  const int nb = (int)nblk(n, RED_THREADS * AXPY_ROWS);
+  multiaxpy_kernel<true><<<nb, RED_THREADS, 0, st>>>(n, m, h, -1.0, base, ld, w, partial);
+  multidot_stage2<<<1, RED_THREADS, 0, st>>>(nb, partial, norm, 1);
+  GB_CUDA(cudaGetLastError());
+  return 2;
+}
+
+// y = x / alpha[0]
+int launch_normalize(cudaStream_t st, int n, const double *alpha, const double *x, double *y) {
+  scale_kernel<<<reduction_blocks(n), RED_THREADS, 0, st>>>(n, alpha, x, y);
   GB_CUDA(cudaGetLastError());
   return 1;
 }
