@@ -757,6 +757,11 @@ static int ensure_side(gbfem_ctx c) {
   }
   return 0;
 }
+static gbfem::StdFaceArgs face_args(gbfem_ctx c, int count, const int *ent_fa, const int *fa_map, int fa_map_len,
+                                    const int *ent_pos, const int *tab, int do_sm, int do_rhs) {
+  return {count,      ent_fa,     0,    fa_map,   fa_map_len, ent_pos, c->nfa,   c->fa_el.p, c->fa_side.p, c->el_nodes.p,
+          c->xyz.p,   c->penalty, c->g, tab,      c->val.p,   c->rhs.p, do_sm,   do_rhs,     c->err.p};
+}
 static int launch_faces_beside(gbfem_ctx c, int count, const int *ent_fa, const int *fa_map, int fa_map_len,
                                const int *ent_pos, const int *tab, int do_sm, int do_rhs, int *launches,
                                cudaStream_t after = nullptr, cudaEvent_t coords_ready = nullptr) {
@@ -764,9 +769,8 @@ static int launch_faces_beside(gbfem_ctx c, int count, const int *ent_fa, const 
   GB_CUDA(cudaEventRecord(c->side_ev[0], after ? after : c->stream));
   GB_CUDA(cudaStreamWaitEvent(c->side_stream, c->side_ev[0], 0));
   if (coords_ready) GB_CUDA(cudaStreamWaitEvent(c->side_stream, coords_ready, 0));
-  const int r = gbfem::launch_prism_faces(c->side_stream, true, count, ent_fa, 0, fa_map, fa_map_len,
-                                          ent_pos, c->nfa, c->fa_el.p, c->fa_side.p, c->el_nodes.p, c->xyz.p,
-                                          c->penalty, c->g, tab, c->val.p, c->rhs.p, do_sm, do_rhs, c->err.p);
+  const int r = gbfem::launch_prism_faces(
+      c->side_stream, true, face_args(c, count, ent_fa, fa_map, fa_map_len, ent_pos, tab, do_sm, do_rhs));
   GB_TRY(r);
   *launches += r;
   GB_CUDA(cudaEventRecord(c->side_ev[1], c->side_stream));
@@ -1216,9 +1220,8 @@ int gbfem_assemble(gbfem_ctx c, int scatter_mode) {
       // the colour permutation lists face indices: feed them as "ids" through an identity map
       for (size_t k = 0; k + 1 < c->h_fa_color_ptr.size(); k++) {
         const int lo = c->h_fa_color_ptr[k], hi = c->h_fa_color_ptr[k + 1];
-        r = gbfem::launch_prism_faces(c->stream, false, hi - lo, c->fa_perm.p + lo, 0, nullptr, -1, nullptr,
-                                      c->nfa, c->fa_el.p, c->fa_side.p, c->el_nodes.p, c->xyz.p, c->penalty,
-                                      c->g, c->el_table.p, c->val.p, c->rhs.p, 1, 1, c->err.p);
+        r = gbfem::launch_prism_faces(c->stream, false, face_args(c, hi - lo, c->fa_perm.p + lo, nullptr, -1, nullptr,
+                                                                  c->el_table.p, 1, 1));
         GB_TRY(r);
         launches += r;
       }

@@ -112,11 +112,22 @@ int launch_prism_elements(cudaStream_t st, bool atomic, bool aniso, int count, c
                           const double *xyz, const double *k_el, const double *D_el, double f,
                           const int *tab, double *val, double *rhs, int do_sm, int do_rhs, int *err,
                           bool dword = false);
-int launch_prism_faces(cudaStream_t st, bool atomic, int count, const int *ent_fa, int fa_base,
-                       const int *fa_map, int fa_map_len, const int *ent_pos, int nfa,
-                       const int *fa_el, const int *fa_side, const int *el_nodes,
-                       const double *xyz, double penalty, double g, const int *tab, double *val,
-                       double *rhs, int do_sm, int do_rhs, int *err);
+struct StdFaceArgs {
+  int count;
+  const int *ent_fa;  // null: faces 0 .. count - 1
+  int fa_base;
+  const int *fa_map;
+  int fa_map_len;
+  const int *ent_pos;
+  int nfa;
+  const int *fa_el, *fa_side, *el_nodes;
+  const double *xyz;
+  double penalty, g;
+  const int *tab;
+  double *val, *rhs;
+  int do_sm, do_rhs, *err;
+};
+int launch_prism_faces(cudaStream_t st, bool atomic, const StdFaceArgs &A);
 // Prism elements by the deterministic gather scatter: local matrices stored
 // to ek (nv nv + nv doubles an element), then a group of lanes a row over the incidence
 // (and the penalty faces through the elements' face lists; nv 6 prisms, 4

@@ -20,7 +20,10 @@
 //    (s = k w / |det|); the 21 matrix entries are then linear combinations of
 //    quadrature sums of those products with compile-time weights h_s(zeta),
 //    L_t(xi, eta);
-//  * the six determinants share one reciprocal (running products).
+//  * the six determinants share one reciprocal (running products);
+//  * what the shape functions have in common is summed once: L_t is the same
+//    at two of the three triangle points, and e_0 = -(e_1 + e_2) enters after
+//    the sums (about 50 of 510 operations: 315k prisms stored 310 -> 281 us).
 #pragma once
 
 #include <math.h>
@@ -150,25 +153,20 @@ GB_HD void prism_std_element_t(vec3<T> ea, vec3<T> eb, vec3<T> fa, vec3<T> fb, v
 
   // quadrature sums of the scaled adjugate products
   const T kw = T(0.5 * wq) * kk;
+  // L_t is B_t at two of the triangle points and B_t + 1/2 at its own, p = 0, 2,
+  // 1 for t = 0, 1, 2: 2 sum_p L_t(p) v_p = v_own + 2 B_t sum_p v_p
+  const double B[3] = {1.0 - GB_PRISM_T1 - GB_PRISM_T2, GB_PRISM_T1, GB_PRISM_T1};
+  const int own[3] = {0, 2, 1};
   T S11[2], S12[2], S22[2];  // sum over triangle points of s c1.c1, s c1.c2, s c2.c2
-  T M[2][2][3];              // M[z][a][t'] = sum_p L_t'(p) s c_a.c3   (a: c1, c2)
+  T M[2][2][3];              // M[z][a][t'] = 2 sum_p L_t'(p) s c_a.c3   (a: c1, c2)
   T F[3];                    // F[p] = sum_z s c3.c3
-  T RA[2][3];                // RA[z][t] = sum_p L_t(p) |det'|
-#pragma unroll
-  for (int p = 0; p < 3; p++) F[p] = T(0.0);
+  T RA[2][3];                // RA[z][t] = 2 sum_p L_t(p) |det'|
 #pragma unroll
   for (int z = 0; z < 2; z++) {
-    S11[z] = S12[z] = S22[z] = T(0.0);
-#pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-      for (int t = 0; t < 3; t++) M[z][a][t] = T(0.0);
-#pragma unroll
-    for (int t = 0; t < 3; t++) RA[z][t] = T(0.0);
+    T g13[3], g23[3];
 #pragma unroll
     for (int p = 0; p < 3; p++) {
       const int q = 3 * z + p;
-      const double L[3] = {1.0 - XI[p] - ETA[p], XI[p], ETA[p]};
       const T s = kw * inv[q];
       // Binet-Cauchy: c1 = j2 x j3, c2 = j3 x j1, c3 = j1 x j2
       const T c11 = t_fma(a22[z], a33[p], -a23[q] * a23[q]);
@@ -176,56 +174,49 @@ GB_HD void prism_std_element_t(vec3<T> ea, vec3<T> eb, vec3<T> fa, vec3<T> fb, v
       const T c22 = t_fma(a33[p], a11[z], -a13[q] * a13[q]);
       const T c13 = t_fma(a12[z], a23[q], -a22[z] * a13[q]);
       const T c23 = t_fma(a13[q], a12[z], -a23[q] * a11[z]);
-      S11[z] = t_fma(s, c11, S11[z]);
-      S12[z] = t_fma(s, c12, S12[z]);
-      S22[z] = t_fma(s, c22, S22[z]);
-      const T g13 = s * c13, g23 = s * c23;
+      S11[z] = p == 0 ? s * c11 : t_fma(s, c11, S11[z]);
+      S12[z] = p == 0 ? s * c12 : t_fma(s, c12, S12[z]);
+      S22[z] = p == 0 ? s * c22 : t_fma(s, c22, S22[z]);
+      g13[p] = s * c13;
+      g23[p] = s * c23;
+      F[p] = z == 0 ? s * c33[z] : t_fma(s, c33[z], F[p]);
+    }
+    const T G13 = g13[0] + g13[1] + g13[2], G23 = g23[0] + g23[1] + g23[2];
+    const T D = adet[3 * z] + adet[3 * z + 1] + adet[3 * z + 2];
 #pragma unroll
-      for (int t = 0; t < 3; t++) {
-        M[z][0][t] = t_fma(T(L[t]), g13, M[z][0][t]);
-        M[z][1][t] = t_fma(T(L[t]), g23, M[z][1][t]);
-        RA[z][t] = t_fma(T(L[t]), adet[q], RA[z][t]);
-      }
-      F[p] = t_fma(s, c33[z], F[p]);
+    for (int t = 0; t < 3; t++) {
+      M[z][0][t] = t_fma(T(2.0 * B[t]), G13, g13[own[t]]);
+      M[z][1][t] = t_fma(T(2.0 * B[t]), G23, g23[own[t]]);
+      RA[z][t] = t_fma(T(2.0 * B[t]), D, adet[3 * z + own[t]]);
     }
   }
 
   // A[ss'][tt'] = sum_z h_s h_s' E_tt'(z), E = sums of s e_t.e_t' with
-  // e = (-(c1+c2), c1, c2); N[s][t][t'] = 1/2 sum_z h_s(z) M_tt'(z)
-  T A[3][6];
+  // e = (-(c1+c2), c1, c2); N[s][t][t'] = 1/2 sum_z h_s(z) M_tt'(z): the entries of
+  // t = 0 from those of 1 and 2 after the sums over z
+  T A[3][6];  // packed symmetric 3x3: (00, 01, 02, 11, 12, 22)
   T N[2][3][3];
+  const double h0[2] = {(1.0 + GB_PRISM_G2) / 2.0, (1.0 - GB_PRISM_G2) / 2.0};  // h_0 at z = 0, 1
+  const double h[2][2] = {{h0[0], h0[1]}, {h0[1], h0[0]}};                        // h[s][z]
 #pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 6; j++) A[i][j] = T(0.0);
+  for (int i = 0; i < 3; i++) {
+    const int s = i == 2, sp = i > 0;
+    const double H0 = h[s][0] * h[sp][0], H1 = h[s][1] * h[sp][1];
+    A[i][3] = t_fma(T(H1), S11[1], T(H0) * S11[0]);
+    A[i][4] = t_fma(T(H1), S12[1], T(H0) * S12[0]);
+    A[i][5] = t_fma(T(H1), S22[1], T(H0) * S22[0]);
+    A[i][1] = -(A[i][3] + A[i][4]);
+    A[i][2] = -(A[i][4] + A[i][5]);
+    A[i][0] = -(A[i][1] + A[i][2]);
+  }
 #pragma unroll
   for (int s = 0; s < 2; s++)
 #pragma unroll
-    for (int t = 0; t < 3; t++)
-#pragma unroll
-      for (int u = 0; u < 3; u++) N[s][t][u] = T(0.0);
-#pragma unroll
-  for (int z = 0; z < 2; z++) {
-    const double zeta = z == 0 ? -GB_PRISM_G2 : GB_PRISM_G2;
-    const double h[2] = {(1.0 - zeta) / 2.0, (1.0 + zeta) / 2.0};
-    // packed symmetric 3x3: (00, 01, 02, 11, 12, 22)
-    const T e01 = -(S11[z] + S12[z]), e02 = -(S12[z] + S22[z]);
-    const T E[6] = {-(e01 + e02), e01, e02, S11[z], S12[z], S22[z]};
-    const double H[3] = {h[0] * h[0], h[0] * h[1], h[1] * h[1]};
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 6; j++) A[i][j] = t_fma(T(H[i]), E[j], A[i][j]);
-#pragma unroll
     for (int u = 0; u < 3; u++) {
-      const T m1t = M[z][0][u], m2t = M[z][1][u];
-      const T mt[3] = {-(m1t + m2t), m1t, m2t};
-#pragma unroll
-      for (int s = 0; s < 2; s++)
-#pragma unroll
-        for (int t = 0; t < 3; t++) N[s][t][u] = t_fma(T(0.5 * h[s]), mt[t], N[s][t][u]);
+      N[s][1][u] = t_fma(T(0.25 * h[s][1]), M[1][0][u], T(0.25 * h[s][0]) * M[0][0][u]);
+      N[s][2][u] = t_fma(T(0.25 * h[s][1]), M[1][1][u], T(0.25 * h[s][0]) * M[0][1][u]);
+      N[s][0][u] = -(N[s][1][u] + N[s][2][u]);
     }
-  }
   // fold P_tt' = 1/4 sum_p L_t L_t' F(p) into A with the sign sigma_s sigma_s'
   // (+ for ss' = 00 and 11, - for 01)
   {
@@ -259,12 +250,11 @@ GB_HD void prism_std_element_t(vec3<T> ea, vec3<T> eb, vec3<T> fa, vec3<T> fb, v
     }
   }
   // R_{t,s} = f w sum_z h_s(z) sum_p L_t(p) |det|,  |det| = |det'| / 8
-  const T fw = T(0.125 * wq) * f;
+  const T fw = T(0.0625 * wq) * f;
 #pragma unroll
   for (int t = 0; t < 3; t++) {
-    const double hlo0 = (1.0 + GB_PRISM_G2) / 2.0, hlo1 = (1.0 - GB_PRISM_G2) / 2.0;  // h_0 at z = 0, 1
-    R[t] = fw * t_fma(T(hlo0), RA[0][t], T(hlo1) * RA[1][t]);
-    R[t + 3] = fw * t_fma(T(hlo1), RA[0][t], T(hlo0) * RA[1][t]);
+    R[t] = fw * t_fma(T(h0[0]), RA[0][t], T(h0[1]) * RA[1][t]);
+    R[t + 3] = fw * t_fma(T(h0[1]), RA[0][t], T(h0[0]) * RA[1][t]);
   }
 }
 

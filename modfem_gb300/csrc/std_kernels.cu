@@ -157,11 +157,40 @@ __device__ __forceinline__ void prism_element_aniso(const d3 (&X)[6], const doub
 // Elements: for i in [0, count): element e = ent_el ? ent_el[i] - el_base : i,
 // table at tab + (ent_pos ? ent_pos[i] : 42*e).  Entity ids outside
 // [0, nel) set *err and are skipped.
-template <bool ATOMIC, bool ANISO, bool DWORD>
+// (isotropic)
+template <bool ATOMIC>
 __global__ void __launch_bounds__(128) prism_elements_kernel(
     int count, const int *__restrict__ ent_el, int el_base, const int *__restrict__ ent_pos, int nel,
-    const int *__restrict__ el_nodes, const double *__restrict__ xyz, const double *__restrict__ k_el,
-    const double *__restrict__ D_el, double f, const int *__restrict__ tab, double *__restrict__ val,
+    const int *__restrict__ el_nodes, const double *__restrict__ xyz, const double *__restrict__ k_el, double f,
+    const int *__restrict__ tab, double *__restrict__ val, double *__restrict__ rhs, int do_sm, int do_rhs,
+    int *__restrict__ err) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= count) return;
+  int e = ent_el ? __ldg(ent_el + i) - el_base : i;
+  if (e < 0 || e >= nel) {
+    atomicExch(err, 1);
+    return;
+  }
+  const int *tb = tab + (ent_pos ? (size_t)__ldg(ent_pos + i) : (size_t)42 * e);
+  const int2 *n2 = reinterpret_cast<const int2 *>(el_nodes + 6 * (size_t)e);
+  const int2 na = __ldg(n2), nb = __ldg(n2 + 1), nc = __ldg(n2 + 2);
+  const int nodes[6] = {na.x, na.y, nb.x, nb.y, nc.x, nc.y};
+  v3 X[6];
+#pragma unroll
+  for (int j = 0; j < 6; j++) {
+    const d3 x = load_node(xyz, nodes[j]);
+    X[j] = {x.x, x.y, x.z};
+  }
+  double R[6], K[21];
+  prism_std_element(X, k_el ? __ldg(k_el + e) : 1.0, f, K, R);
+  scatter6<ATOMIC>(tb, K, R, val, rhs, do_sm, do_rhs);
+}
+
+// (full tensor)
+template <bool ATOMIC>
+__global__ void __launch_bounds__(128) prism_elements_aniso_kernel(
+    int count, const int *__restrict__ ent_el, int el_base, const int *__restrict__ ent_pos, int nel,
+    const int *__restrict__ el_nodes, const double *__restrict__ xyz, const double *__restrict__ D_el, double f, const int *__restrict__ tab, double *__restrict__ val,
     double *__restrict__ rhs, int do_sm, int do_rhs, int *__restrict__ err) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
@@ -176,33 +205,25 @@ __global__ void __launch_bounds__(128) prism_elements_kernel(
   d3 X[6] = {load_node(xyz, na.x), load_node(xyz, na.y), load_node(xyz, nb.x),
              load_node(xyz, nb.y), load_node(xyz, nc.x), load_node(xyz, nc.y)};
   double R[6];
-  if (!ANISO) {
-    double K[21];
-    const v3 Xv[6] = {{X[0].x, X[0].y, X[0].z}, {X[1].x, X[1].y, X[1].z}, {X[2].x, X[2].y, X[2].z},
-                      {X[3].x, X[3].y, X[3].z}, {X[4].x, X[4].y, X[4].z}, {X[5].x, X[5].y, X[5].z}};
-    prism_std_element(Xv, k_el ? __ldg(k_el + e) : 1.0, f, K, R);
-    scatter6<ATOMIC>(tb, K, R, val, rhs, do_sm, do_rhs);
-  } else {
-    double K[36];
-    prism_element_aniso(X, D_el + 9 * (size_t)e, f, K, R);
-    int t[42];
-    const int2 *t2 = reinterpret_cast<const int2 *>(tb);
+  double K[36];
+  prism_element_aniso(X, D_el + 9 * (size_t)e, f, K, R);
+  int t[42];
+  const int2 *t2 = reinterpret_cast<const int2 *>(tb);
 #pragma unroll
-    for (int j = 0; j < 21; j++) {
-      int2 v = __ldg(t2 + j);
-      t[2 * j] = v.x;
-      t[2 * j + 1] = v.y;
-    }
-    if (do_sm) {
+  for (int j = 0; j < 21; j++) {
+    int2 v = __ldg(t2 + j);
+    t[2 * j] = v.x;
+    t[2 * j + 1] = v.y;
+  }
+  if (do_sm) {
 #pragma unroll
-      for (int u = 0; u < 6; u++)
+    for (int u = 0; u < 6; u++)
 #pragma unroll
-        for (int w = 0; w < 6; w++) add_val<ATOMIC>(val, t[w + 6 * u], K[u * 6 + w]);
-    }
-    if (do_rhs) {
+      for (int w = 0; w < 6; w++) add_val<ATOMIC>(val, t[w + 6 * u], K[u * 6 + w]);
+  }
+  if (do_rhs) {
 #pragma unroll
-      for (int w = 0; w < 6; w++) add_val<ATOMIC>(rhs, t[36 + w], R[w]);
-    }
+    for (int w = 0; w < 6; w++) add_val<ATOMIC>(rhs, t[36 + w], R[w]);
   }
 }
 
@@ -269,62 +290,69 @@ __global__ void __launch_bounds__(kDwThreads, 3) prism_elements_dw_kernel(
   }
 }
 
+// local vertex j of a prism side: the lower (side 0) or upper triangle, or lower
+// then upper ends of the sides 2..4 (edge 01, 12, 20)
+__device__ __forceinline__ int side_vertex(int side, int j) {
+  if (side <= 1) return 3 * side + j;
+  return ((j & 1) ? (side - 1) % 3 : side - 2) + 3 * (j >> 1);
+}
+
 // The penalty face integrals of one boundary face (side 0..4 of its prism,
-// vertices X): K over the face's own vertices loc[0..nloc) (upper triangle
-// of a 4x4 block packed row by row), R their load entries.
-__device__ __forceinline__ void prism_face_local(const d3 (&X)[6], int side, double penalty, double g,
-                                                 int (&loc)[4], int &nloc, double (&K)[10], double (&Rl)[4]) {
-  const d3 a0 = X[0], a1 = X[1], a2 = X[2], b0 = X[3], b1 = X[4], b2 = X[5];
-  const d3 ea = a1 - a0, eb = b1 - b0, fa_ = a2 - a0, fb = b2 - b0;
-  const d3 m1 = 0.5 * (ea + eb), d1 = 0.5 * (eb - ea);
-  const d3 m2 = 0.5 * (fa_ + fb), d2 = 0.5 * (fb - fa_);
-  const d3 c0 = 0.5 * (b0 - a0);
-  if (side == 0) { loc[0] = 0; loc[1] = 1; loc[2] = 2; nloc = 3; }
-  else if (side == 1) { loc[0] = 3; loc[1] = 4; loc[2] = 5; nloc = 3; }
-  else {
-    int a = side - 2, b = (side - 1) % 3;
-    loc[0] = a; loc[1] = b; loc[2] = a + 3; loc[3] = b + 3; nloc = 4;
-  }
+// nd: the prism's vertices): the upper entries over the face's own vertices in
+// side_vertex order, row by row of 4, and their load entries; returns the
+// vertices it has.  Works on the face alone: |dS| of a triangle is constant, a
+// quadrilateral is bilinear in its four corners, the values of the shape
+// functions at the points are constants (the sides by cases over the whole
+// prism, values through an index: 2,400 faces 20 us, 14 us so).
+__device__ __forceinline__ int prism_face_local(const double *__restrict__ xyz, const int *__restrict__ nd, int side,
+                                                double penalty, double g, double (&K)[10], double (&Rl)[4]) {
+  const bool tri = side <= 1;
+  d3 X[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) X[j] = load_node(xyz, __ldg(nd + side_vertex(side, tri && j == 3 ? 0 : j)));
 #pragma unroll
   for (int j = 0; j < 10; j++) K[j] = 0.0;
 #pragma unroll
   for (int j = 0; j < 4; j++) Rl[j] = 0.0;
-  const int nq = side <= 1 ? 3 : 4;
-  for (int q = 0; q < nq; q++) {
-    double xi, eta, zeta, w;
-    if (side <= 1) {
-      xi = q == 2 ? GB_T2 : GB_T1;
-      eta = q == 1 ? GB_T2 : GB_T1;
-      zeta = side == 0 ? -1.0 : 1.0;
-      w = 0.5 * GB_TW;
-    } else {
-      const double s = (q >> 1) == 0 ? -GB_G2 : GB_G2, t = (q & 1) == 0 ? -GB_G2 : GB_G2;
-      const double u = (s + 1.0) / 2.0;
-      if (side == 2) { xi = u; eta = 0.0; }
-      else if (side == 3) { xi = 1.0 - u; eta = u; }
-      else { xi = 0.0; eta = 1.0 - u; }
-      zeta = t;
-      w = 0.5;
+  if (tri) {
+    const d3 ds = cross(X[1] - X[0], X[2] - X[0]);
+    const double pa = penalty * (sqrt(dot(ds, ds)) * (0.5 * GB_TW));
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      double r = 0.0, k[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        const double xi = q == 2 ? GB_T2 : GB_T1, eta = q == 1 ? GB_T2 : GB_T1;
+        const double L[3] = {1.0 - xi - eta, xi, eta};
+        r += L[a];
+#pragma unroll
+        for (int b = a; b < 3; b++) k[b] += L[a] * L[b];
+      }
+#pragma unroll
+      for (int b = a; b < 3; b++) K[4 * a - a * (a - 1) / 2 + b - a] = pa * k[b];
+      Rl[a] = pa * g * r;
     }
-    const d3 j1 = fma3(zeta, d1, m1), j2 = fma3(zeta, d2, m2);
-    const d3 j3 = fma3(eta, d2, fma3(xi, d1, c0));
-    d3 ds;
-    if (side <= 1) ds = cross(j1, j2);
-    else if (side == 2) ds = cross(j1, j3);
-    else if (side == 3) ds = cross(j2 - j1, j3);
-    else ds = cross(j3, j2);
-    const double area = sqrt(dot(ds, ds)) * w;
-    const double hlo = (1.0 - zeta) / 2.0, hhi = (1.0 + zeta) / 2.0, L0 = 1.0 - xi - eta;
-    const double phi6[6] = {hlo * L0, hlo * xi, hlo * eta, hhi * L0, hhi * xi, hhi * eta};
-    double ph[4];
-    for (int j = 0; j < nloc; j++) ph[j] = phi6[loc[j]];
-    const double pa = penalty * area;
-    int k = 0;
-    for (int a = 0; a < 4; a++)
-      for (int b = a; b < 4; b++, k++)
-        if (a < nloc && b < nloc) K[k] = fma(pa * ph[a], ph[b], K[k]);
-    for (int a = 0; a < nloc; a++) Rl[a] = fma(pa * g, ph[a], Rl[a]);
+    return 3;
   }
+  // corners 0, 1 (zeta = -1), 2, 3 (zeta = 1); u from 0, 2 to 1, 3
+  const d3 elo = X[1] - X[0], ehi = X[3] - X[2], f0 = X[2] - X[0], f1 = X[3] - X[1];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const double u = (((q >> 1) == 0 ? -GB_G2 : GB_G2) + 1.0) / 2.0, zeta = (q & 1) == 0 ? -GB_G2 : GB_G2;
+    const double hlo = (1.0 - zeta) / 2.0, hhi = (1.0 + zeta) / 2.0;
+    const double ph[4] = {hlo * (1.0 - u), hlo * u, hhi * (1.0 - u), hhi * u};
+    // dx/du and 2 dx/dzeta
+    const d3 ds = cross(fma3(hhi, ehi, hlo * elo), fma3(u, f1, (1.0 - u) * f0));
+    const double pa = penalty * (sqrt(dot(ds, ds)) * 0.25);
+    int k = 0;
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+#pragma unroll
+      for (int b = a; b < 4; b++, k++) K[k] = fma(ph[a] * ph[b], pa, K[k]);
+      Rl[a] = fma(pa * g, ph[a], Rl[a]);
+    }
+  }
+  return 4;
 }
 
 // Boundary penalty faces of the std weak form (pdd_conv_diff/weak_formulation/
@@ -334,49 +362,39 @@ __device__ __forceinline__ void prism_face_local(const d3 (&X)[6], int side, dou
 // side cases of apr_elem_calc_3D_prism (aps_std_util.c:770-805).  Only the
 // face's own vertices get non-zero entries.
 template <bool ATOMIC>
-__global__ void __launch_bounds__(128) prism_faces_kernel(
-    int count, const int *__restrict__ ent_fa, int fa_base, const int *__restrict__ fa_map,
-    int fa_map_len, const int *__restrict__ ent_pos, int nfa, const int *__restrict__ fa_el,
-    const int *__restrict__ fa_side, const int *__restrict__ el_nodes, const double *__restrict__ xyz,
-    double penalty, double g, const int *__restrict__ tab, double *__restrict__ val,
-    double *__restrict__ rhs, int do_sm, int do_rhs, int *__restrict__ err) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
+__global__ void __launch_bounds__(128) prism_faces_kernel(StdFaceArgs A) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= A.count) return;
   // face index: i, or ent_fa[i] (a face index when fa_map is null, else a
   // mesh face id translated through fa_map)
   int fa = i;
-  if (ent_fa) {
-    int id = __ldg(ent_fa + i) - fa_base;
-    if (fa_map)
-      fa = (id >= 0 && id < fa_map_len) ? __ldg(fa_map + id) : -1;
+  if (A.ent_fa) {
+    int id = __ldg(A.ent_fa + i) - A.fa_base;
+    if (A.fa_map)
+      fa = (id >= 0 && id < A.fa_map_len) ? __ldg(A.fa_map + id) : -1;
     else
       fa = id;
   }
-  if (fa < 0 || fa >= nfa) {
-    atomicExch(err, 2);
+  if (fa < 0 || fa >= A.nfa) {
+    atomicExch(A.err, 2);
     return;
   }
-  const int e = __ldg(fa_el + fa), side = __ldg(fa_side + fa);
-  const int *tb = tab + (ent_pos ? (size_t)__ldg(ent_pos + i) : (size_t)42 * e);
-  const int *nd = el_nodes + 6 * (size_t)e;
-  d3 X[6];
-#pragma unroll
-  for (int j = 0; j < 6; j++) X[j] = load_node(xyz, __ldg(nd + j));
-  int loc[4], nloc;
+  const int e = __ldg(A.fa_el + fa), side = __ldg(A.fa_side + fa);
+  const int *tb = A.tab + (A.ent_pos ? (size_t)__ldg(A.ent_pos + i) : (size_t)42 * e);
   double K[10], Rl[4];
-  prism_face_local(X, side, penalty, g, loc, nloc, K, Rl);
-  if (do_sm) {
-    int k = 0;
-    for (int a = 0; a < 4; a++)
-      for (int b = a; b < 4; b++, k++) {
-        if (a >= nloc || b >= nloc) continue;
-        const int u = loc[a], wv = loc[b];
-        add_val<ATOMIC>(val, __ldg(tb + wv + 6 * u), K[k]);
-        if (a != b) add_val<ATOMIC>(val, __ldg(tb + u + 6 * wv), K[k]);
-      }
-  }
-  if (do_rhs && g != 0.0) {
-    for (int a = 0; a < nloc; a++) add_val<ATOMIC>(rhs, __ldg(tb + 36 + loc[a]), Rl[a]);
+  const int nloc = prism_face_local(A.xyz, A.el_nodes + 6 * (size_t)e, side, A.penalty, A.g, K, Rl);
+  int k = 0;
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    const int u = side_vertex(side, a);
+#pragma unroll
+    for (int b = a; b < 4; b++, k++) {
+      if (!A.do_sm || b >= nloc) continue;
+      const int w = side_vertex(side, b);
+      add_val<ATOMIC>(A.val, __ldg(tb + w + 6 * u), K[k]);
+      if (a != b) add_val<ATOMIC>(A.val, __ldg(tb + u + 6 * w), K[k]);
+    }
+    if (A.do_rhs && A.g != 0.0 && a < nloc) add_val<ATOMIC>(A.rhs, __ldg(tb + 36 + u), Rl[a]);
   }
 }
 
@@ -522,13 +540,8 @@ __global__ void __launch_bounds__(128) prism_faces_store_kernel(
     const double *__restrict__ xyz, double penalty, double g, double *__restrict__ fk) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nfa) return;
-  const int *nd = el_nodes + 6 * (size_t)__ldg(fa_el + f);
-  d3 X[6];
-#pragma unroll
-  for (int j = 0; j < 6; j++) X[j] = load_node(xyz, __ldg(nd + j));
-  int loc[4], nloc;
   double K[10], Rl[4];
-  prism_face_local(X, __ldg(fa_side + f), penalty, g, loc, nloc, K, Rl);
+  prism_face_local(xyz, el_nodes + 6 * (size_t)__ldg(fa_el + f), __ldg(fa_side + f), penalty, g, K, Rl);
 #pragma unroll
   for (int i = 0; i < 10; i++) fk[14 * (size_t)f + i] = K[i];
 #pragma unroll
@@ -541,7 +554,7 @@ __global__ void face_lists_kernel(int nfa, const int *__restrict__ fa_el, int *h
   if (f < nfa) next[f] = atomicExch(head + fa_el[f], f);
 }
 
-// place of local vertex v among the vertices of a prism side (prism_face_local's order), -1: not on it
+// place of local vertex v among the vertices of a prism side (side_vertex's order), -1: not on it
 __device__ __forceinline__ int side_place(int side, int v) {
   if (side <= 1) return v / 3 == side ? v % 3 : -1;
   const int a = side - 2, b = (side - 1) % 3, t = v % 3;
@@ -704,9 +717,8 @@ __global__ void __launch_bounds__(128) prism_constrained_kernel(
   // the local matrix, K[u * 6 + w] = (row w, column u), and load vector
   double K[36], R[6];
   if (FACE) {
-    int loc[4], nloc;
     double Kf[10], Rl[4];
-    prism_face_local(X, side, penalty, g, loc, nloc, Kf, Rl);
+    const int nloc = prism_face_local(xyz, el_nodes + 6 * (size_t)e, side, penalty, g, Kf, Rl);
 #pragma unroll
     for (int j = 0; j < 36; j++) K[j] = 0.0;
 #pragma unroll
@@ -714,11 +726,12 @@ __global__ void __launch_bounds__(128) prism_constrained_kernel(
     int k = 0;
     for (int a = 0; a < 4; a++)
       for (int b = a; b < 4; b++, k++) {
-        if (a >= nloc || b >= nloc) continue;
-        K[loc[a] * 6 + loc[b]] = Kf[k];
-        K[loc[b] * 6 + loc[a]] = Kf[k];
+        if (b >= nloc) continue;
+        const int u = side_vertex(side, a), w = side_vertex(side, b);
+        K[u * 6 + w] = Kf[k];
+        K[w * 6 + u] = Kf[k];
       }
-    for (int a = 0; a < nloc; a++) R[loc[a]] = Rl[a];
+    for (int a = 0; a < nloc; a++) R[side_vertex(side, a)] = Rl[a];
   } else if (ANISO) {
     prism_element_aniso(X, D_el + 9 * (size_t)e, f, K, R);
   } else {
@@ -766,13 +779,10 @@ int launch_prism_elements(cudaStream_t st, bool atomic, bool aniso, int count, c
                           bool dword) {
   if (count <= 0) return 0;
   const int T = 128;
-#define GB_LAUNCH(A, B, W)                                                                        \
-  prism_elements_kernel<A, B, W><<<nblk(count, T), T, 0, st>>>(count, ent_el, el_base, ent_pos, nel, \
-                                                               el_nodes, xyz, k_el, D_el, f, tab,   \
-                                                               val, rhs, do_sm, do_rhs, err)
   if (aniso) {
-    if (atomic) GB_LAUNCH(true, true, false);
-    else GB_LAUNCH(false, true, false);
+    auto k = atomic ? prism_elements_aniso_kernel<true> : prism_elements_aniso_kernel<false>;
+    k<<<nblk(count, T), T, 0, st>>>(count, ent_el, el_base, ent_pos, nel, el_nodes, xyz, D_el, f, tab, val, rhs,
+                                    do_sm, do_rhs, err);
   } else if (dword) {
     const size_t sm = (size_t)kPrismDwSlots * kDwThreads * sizeof(float2);
     if (atomic)
@@ -782,29 +792,19 @@ int launch_prism_elements(cudaStream_t st, bool atomic, bool aniso, int count, c
       prism_elements_dw_kernel<false><<<nblk(count, kDwThreads), kDwThreads, sm, st>>>(
           count, ent_el, el_base, ent_pos, nel, el_nodes, xyz, k_el, f, tab, val, rhs, do_sm, do_rhs, err);
   } else {
-    if (atomic) GB_LAUNCH(true, false, false);
-    else GB_LAUNCH(false, false, false);
+    auto k = atomic ? prism_elements_kernel<true> : prism_elements_kernel<false>;
+    k<<<nblk(count, T), T, 0, st>>>(count, ent_el, el_base, ent_pos, nel, el_nodes, xyz, k_el, f, tab, val, rhs,
+                                    do_sm, do_rhs, err);
   }
-#undef GB_LAUNCH
   GB_CUDA(cudaGetLastError());
   return 1;
 }
 
-int launch_prism_faces(cudaStream_t st, bool atomic, int count, const int *ent_fa, int fa_base,
-                       const int *fa_map, int fa_map_len, const int *ent_pos, int nfa,
-                       const int *fa_el, const int *fa_side, const int *el_nodes,
-                       const double *xyz, double penalty, double g, const int *tab, double *val,
-                       double *rhs, int do_sm, int do_rhs, int *err) {
-  if (count <= 0) return 0;
+int launch_prism_faces(cudaStream_t st, bool atomic, const StdFaceArgs &A) {
+  if (A.count <= 0) return 0;
   const int T = 128;
-  if (atomic)
-    prism_faces_kernel<true><<<nblk(count, T), T, 0, st>>>(count, ent_fa, fa_base, fa_map, fa_map_len,
-                                                           ent_pos, nfa, fa_el, fa_side, el_nodes, xyz,
-                                                           penalty, g, tab, val, rhs, do_sm, do_rhs, err);
-  else
-    prism_faces_kernel<false><<<nblk(count, T), T, 0, st>>>(count, ent_fa, fa_base, fa_map, fa_map_len,
-                                                            ent_pos, nfa, fa_el, fa_side, el_nodes, xyz,
-                                                            penalty, g, tab, val, rhs, do_sm, do_rhs, err);
+  auto k = atomic ? prism_faces_kernel<true> : prism_faces_kernel<false>;
+  k<<<nblk(A.count, T), T, 0, st>>>(A);
   GB_CUDA(cudaGetLastError());
   return 1;
 }
