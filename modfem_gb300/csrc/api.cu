@@ -821,26 +821,39 @@ static int build_pipe_plan(gbfem_ctx c, int e0, int e1) {
   GB_CUDA(cudaMemcpyAsync(last.data(), c->row_last.p, (size_t)nd * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   GB_CUDA(cudaStreamSynchronize(c->stream));
   for (int r = 1; r < nd; r++) last[r] = std::max(last[r], last[r - 1]);  // prefix maximum
-  // chunks of whole waves of resident element threads (128-thread blocks,
-  // five per SM for the FP64 kernel, three for the double-word one), at
-  // most eight
+  // Chunks of whole waves of resident element threads (128-thread blocks,
+  // five per SM for the FP64 kernel, three for the double-word one), an eighth
+  // of the elements each.  The double-word kernel outruns the download (2M
+  // prisms: 709 us of kernel, 930 us of host link), so its first chunks are one
+  // wave and grow by less than the download is slower, 1.4: the download
+  // starts a wave after the first coordinates and does not stop.  The FP64
+  // kernels take twice the download's time: their last chunks shrink to one wave,
+  // which is what is left to download after the last element.  (2M prisms, double word
+  // 1,274 us with even chunks, 1,238 us so; FP64 2,080 and 2,008 us)
   int nsm = 152;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-  const long long wave = (long long)nsm * (c->std_dword ? 3 : 5) * 128;
-  const long long chunk = std::max(wave, (count / 8 + wave) / wave * wave);
-  const int K = (int)((count + chunk - 1) / chunk);
+  const long long wave = (long long)nsm * (c->std_dword ? 3 : 5) * 128, waves = (count + wave - 1) / wave;
+  const long long most = count / (8 * wave) + 1;
+  std::vector<long long> size;
+  double ramp = 1.0;
+  for (long long left = waves; left > 0; left -= size.back(), ramp *= 1.4)
+    size.push_back(std::min({left, most, (long long)(ramp + 0.5)}));
+  if (!c->std_dword) std::reverse(size.begin(), size.end());
+  const int K = (int)size.size();
   c->pipe_el.assign(K + 1, 0);
   c->pipe_rows.assign(K, nd);
-  for (int k = 0; k <= K; k++) c->pipe_el[k] = (int)std::min<long long>(count, chunk * k);
+  for (int k = 0; k < K; k++) c->pipe_el[k + 1] = (int)std::min<long long>(count, c->pipe_el[k] + size[k] * wave);
   for (int k = 0; k + 1 < K; k++)
     c->pipe_rows[k] = (int)(std::upper_bound(last.begin(), last.end(), c->pipe_el[k + 1] - 1) - last.begin());
   // (the chunks' largest node and element indices are found when a call
   // first overlaps uploads with them: pipe_chunk_reach)
   c->pipe_maxnode.clear();
   c->pipe_maxel.clear();
-  if (!c->copy_stream) {
-    GB_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
-    for (auto &ev : c->pipe_ev) GB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  if (!c->copy_stream) GB_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
+  while ((int)c->pipe_ev.size() < K + 1) {
+    cudaEvent_t ev = nullptr;
+    GB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    c->pipe_ev.push_back(ev);
   }
   for (int i = 0; i < 3; i++) {
     c->pipe_key[i] = c->cache_key[i];

@@ -373,7 +373,7 @@ struct gbfem_ctx_s {
   // element chunks, and per chunk the rows no later element touches, copied
   // on copy_stream while the next chunk runs
   cudaStream_t copy_stream = nullptr;
-  cudaEvent_t pipe_ev[9] = {};
+  std::vector<cudaEvent_t> pipe_ev;
   gbfem::DevBuf<int> row_last;
   const void *pipe_key[3] = {nullptr, nullptr, nullptr};
   long long pipe_len[3] = {0, 0, 0};
