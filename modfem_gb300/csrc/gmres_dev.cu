@@ -430,11 +430,38 @@ __global__ void __launch_bounds__(32 * WARPS, DOTS ? 1 : 8) gm_arnoldi_spmv(GmAr
   }
 }
 
+// t[u] = this thread's share of <V_u, w> over the rows lo .. hi, u < K (exactly
+// K FMAs a row), two rows' loads in flight
+template <int K, int T>
+__device__ __forceinline__ void gm_dots_rows(const double *__restrict__ v, long long n, const double *__restrict__ w,
+                                             int lo, int hi, double (&t)[8]) {
+#pragma unroll
+  for (int u = 0; u < 8; u++) t[u] = 0.0;
+  int i = lo + threadIdx.x;
+  for (; i + T < hi; i += 2 * T) {
+    const double w0 = __ldg(w + i), w1 = __ldg(w + i + T);
+    double x[K], y[K];
+#pragma unroll
+    for (int u = 0; u < K; u++) {
+      x[u] = __ldg(v + u * n + i);
+      y[u] = __ldg(v + u * n + i + T);
+    }
+#pragma unroll
+    for (int u = 0; u < K; u++) t[u] = fma(y[u], w1, fma(x[u], w0, t[u]));
+  }
+  if (i < hi) {
+    const double w0 = __ldg(w + i);
+#pragma unroll
+    for (int u = 0; u < K; u++) t[u] = fma(__ldg(v + u * n + i), w0, t[u]);
+  }
+}
+
 // Block partials of <W_k, W_{j+1}>, k <= j: one block per SM takes an equal
-// share of the rows and all vectors, eight at a time (two rows' loads in
-// flight), so that a row costs one FMA a vector and the reductions are paid
-// once per thread and eight vectors.  W_{j+1} is read once per eight vectors
-// (L1 after the first).
+// share of the rows and all vectors, eight at a time, so that a row costs one
+// FMA a vector and the reductions are paid once per thread and eight vectors.
+// W_{j+1} is read once per eight vectors (L1 after the first).  1,030,301 rows, 1
+// to 30 vectors: 49.5 us on average with the FMAs of incomplete groups
+// predicated, 38.5 us with a body a count.
 constexpr int GM_DOT_BLOCKS = 152, GM_DOT_T = 768;
 __global__ void __launch_bounds__(GM_DOT_T) gm_dots(GmArgs a, int j) {
   if (!a.alive[j]) return;
@@ -445,21 +472,15 @@ __global__ void __launch_bounds__(GM_DOT_T) gm_dots(GmArgs a, int j) {
   for (int k0 = 0; k0 <= j; k0 += 8) {
     const double *v = a.V + (size_t)k0 * a.n;
     double t[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) t[u] = 0.0;
-    for (int i = lo + threadIdx.x; i < hi; i += 2 * GM_DOT_T) {
-      const bool two = i + GM_DOT_T < hi;
-      const double w0 = __ldg(w + i), w1 = two ? __ldg(w + i + GM_DOT_T) : 0.0;
-      double x[8], y[8];
-#pragma unroll
-      for (int u = 0; u < 8; u++)
-        if (k0 + u <= j) {
-          x[u] = __ldg(v + (size_t)u * a.n + i);
-          y[u] = two ? __ldg(v + (size_t)u * a.n + i + GM_DOT_T) : 0.0;
-        }
-#pragma unroll
-      for (int u = 0; u < 8; u++)
-        if (k0 + u <= j) t[u] = fma(y[u], w1, fma(x[u], w0, t[u]));
+    switch (j + 1 - k0) {
+      case 1: gm_dots_rows<1, GM_DOT_T>(v, a.n, w, lo, hi, t); break;
+      case 2: gm_dots_rows<2, GM_DOT_T>(v, a.n, w, lo, hi, t); break;
+      case 3: gm_dots_rows<3, GM_DOT_T>(v, a.n, w, lo, hi, t); break;
+      case 4: gm_dots_rows<4, GM_DOT_T>(v, a.n, w, lo, hi, t); break;
+      case 5: gm_dots_rows<5, GM_DOT_T>(v, a.n, w, lo, hi, t); break;
+      case 6: gm_dots_rows<6, GM_DOT_T>(v, a.n, w, lo, hi, t); break;
+      case 7: gm_dots_rows<7, GM_DOT_T>(v, a.n, w, lo, hi, t); break;
+      default: gm_dots_rows<8, GM_DOT_T>(v, a.n, w, lo, hi, t); break;
     }
     const double d = gm_warp_sums(t, threadIdx.x & 31);
     if ((threadIdx.x & 3) == 0) part[threadIdx.x / 32][k0 % KP + ((threadIdx.x & 31) >> 2)] = d;
@@ -486,8 +507,10 @@ __global__ void __launch_bounds__(GM_SUM_T) gm_column(GmArgs a, int j) {
 
 // W_{j+1} = sc_j W_{j+1} - sum_k h_k sc_k W_k, the block partials of its squared
 // norm and its double-word copy for the next SpMV.  SMALL: the column entries
-// first.  Otherwise (T = 256) five blocks fit an SM, and the grid is at most
-// that many (a second wave would leave most SMs idle).
+// first, a row a thread.  Otherwise (T = 256) five blocks fit an SM, the grid is at most
+// that many (a second wave would leave most SMs idle); beyond a row a thread a
+// block takes an equal share of the rows, four a thread at a time (1,030,301
+// rows, 1 to 30 vectors: 51 us on average with one, 43 us with four).
 template <int T, bool SMALL>
 __global__ void __launch_bounds__(T, SMALL ? 1 : 5) gm_orthogonalize(GmArgs a, int j) {
   if (!a.alive[j]) return;
@@ -502,7 +525,26 @@ __global__ void __launch_bounds__(T, SMALL ? 1 : 5) gm_orthogonalize(GmArgs a, i
   __syncthreads();
   double *w = a.V + (size_t)(j + 1) * a.n;
   double s = 0.0;
-  for (long long i = (long long)blockIdx.x * T + threadIdx.x; i < a.n; i += (long long)gridDim.x * T) {
+  long long i = (long long)blockIdx.x * T + threadIdx.x, end = a.n, step = (long long)gridDim.x * T;
+  if constexpr (!SMALL) {
+    if (a.n > step) {
+      i = (long long)a.n * blockIdx.x / gridDim.x + threadIdx.x;
+      end = (long long)a.n * (blockIdx.x + 1) / gridDim.x;
+      step = T;
+      for (; i + 3 * T < end; i += 4 * T) {
+        double t[4];
+        gm_combine_rows<4>(a.V, a.n, coef, j + 1, i, T, t);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const double wi = fma(scj, w[i + q * T], -t[q]);
+          w[i + q * T] = wi;
+          if (a.xdw) a.xdw[i + q * T] = dw_f2(wi);
+          s = fma(wi, wi, s);
+        }
+      }
+    }
+  }
+  for (; i < end; i += step) {
     const double wi = fma(scj, w[i], -gm_combine<SMALL ? 32 : 8>(a.V, a.n, coef, j + 1, i));
     w[i] = wi;
     if (a.xdw) a.xdw[i] = dw_f2(wi);
@@ -541,7 +583,7 @@ unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 // Up to here (slices of 32 rows; 38,912 rows) the dots run in the SpMV kernel:
 // below, an Arnoldi step is launches and memory latency (9,261 rows: 14 us a step
 // in two kernels; the three kernels with last-block tails before took 28).
-// 1,030,301 rows: 135 us a step on average over 30 (180 before).
+// 1,030,301 rows: 118 us a step on average over 30 (180 before).
 constexpr int GM_SMALL = 1216, GM_SMALL_WARPS = 4;
 
 // SELL-32 index arrays of the context's structure (once per structure)

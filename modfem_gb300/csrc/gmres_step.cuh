@@ -61,7 +61,9 @@ __device__ __forceinline__ void gm_sum_dots(const double *partial, int rows, int
 }
 
 // sum_k c[k] V_k[i], U vectors' loads in flight, two accumulators (an FP64 FMA
-// waits long for the one before it)
+// waits long for the one before it).  An incomplete group's FMAs are predicated:
+// in the small systems that take U = 32 (9,261 rows, a step 17.6 us) a branch
+// around every four of them costs 0.7 us a step more than it saves.
 template <int U>
 __device__ __forceinline__ double gm_combine(const double *V, long long n, const double *c, int nk, long long i) {
   double a0 = 0.0, a1 = 0.0;
@@ -81,6 +83,31 @@ __device__ __forceinline__ double gm_combine(const double *V, long long n, const
       }
   }
   return a0 + a1;
+}
+
+// out[q] = sum_k c[k] V_k[i + q T], q < R: R rows' chains of FMAs side by side and
+// 4 R loads in flight
+template <int R>
+__device__ __forceinline__ void gm_combine_rows(const double *V, long long n, const double *c, int nk, long long i,
+                                                int T, double (&out)[R]) {
+  const double *v = V + i;
+#pragma unroll
+  for (int q = 0; q < R; q++) out[q] = 0.0;
+  int k = 0;
+  for (; k + 4 <= nk; k += 4, v += 4 * n) {
+    double x[4][R];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int q = 0; q < R; q++) x[u][q] = __ldg(v + u * n + q * T);
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+      for (int q = 0; q < R; q++) out[q] = fma(c[k + u], x[u][q], out[q]);
+  }
+  for (; k < nk; k++, v += n)
+#pragma unroll
+    for (int q = 0; q < R; q++) out[q] = fma(c[k], __ldg(v + q * T), out[q]);
 }
 
 // The step's logic for step j (one block of T threads): |w| from the norm
