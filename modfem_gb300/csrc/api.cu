@@ -1682,18 +1682,6 @@ int gbfem_dg_get_structure(gbfem_ctx c, int *dof_off, int *bptr, int *bcol, long
 }
 
 // Point fields of every face of the moment form; returns the launches.
-static int launch_mom_fields(gbfem_ctx c) {
-  int n = 0;
-  for (int b = 0; b < 8; b++) {
-    const int r = gbfem::launch_dg_face_fields(c->stream, b % 4 + 1, b / 4, c->dg_fb_start[b + 1] - c->dg_fb_start[b],
-                                               c->dg_frec.p + c->dg_fb_start[b], c->el_nodes.p, c->xyz.p, c->k_el.p,
-                                               c->D_el.p, c->dg_pen, c->dg_ffield.p);
-    GB_TRY(r);
-    n += r;
-  }
-  return n;
-}
-
 int gbfem_dg_assemble(gbfem_ctx c) {
   GB_CHECK(c && c->dg_ready, "DG structure not built (gbfem_dg_build_structure)");
   GB_TRY(settle_uploads(c));
@@ -1805,7 +1793,8 @@ int gbfem_dg_assemble(gbfem_ctx c) {
     }
     if (mom) {
       GB_TRY(c->dg_ffield.alloc((size_t)c->dg_ffield_n));
-      const int rf = launch_mom_fields(c);
+      const int rf = gbfem::launch_dg_face_fields(c->stream, c->dg_fb_start, c->dg_frec.p, c->el_nodes.p, c->xyz.p,
+                                                  c->k_el.p, c->D_el.p, c->dg_pen, c->dg_ffield.p);
       GB_TRY(rf);
       launches += rf;
       for (int p = 1; p <= 4; p++) {
@@ -1942,7 +1931,8 @@ int gbfem_dg_autotune(gbfem_ctx c, int sample, int *vol_out, int *face_out, doub
   };
   if (c->dg_hf.p && c->dg_mom_ok) {
     GB_TRY(c->dg_ffield.alloc((size_t)c->dg_ffield_n));
-    GB_TRY(launch_mom_fields(c));
+    GB_TRY(gbfem::launch_dg_face_fields(c->stream, c->dg_fb_start, c->dg_frec.p, c->el_nodes.p, c->xyz.p,
+                                                  c->k_el.p, c->D_el.p, c->dg_pen, c->dg_ffield.p));
   }
   for (int p = 1; p <= 4; p++) {
     if (!c->dg_list[p].p) continue;

@@ -39,6 +39,7 @@
 #include "dg_face.cuh"
 #include "gbfem_internal.h"
 
+#include <algorithm>
 #include <mutex>
 
 namespace gbfem {
@@ -175,17 +176,32 @@ bool dg_face_moments_cover(const DgFaceRec &r) {
 }
 
 // ---------------------------------------------------------------- geometry
-// The point fields of `count` faces with the same rule (nq points, degree
-// pr, ti 0 triangles, 1 quadrilaterals): geo[f * nq + q] of face slot f.
-// NF faces per CTA: the vertex differences of both sides first, then one
-// thread a point.  FP64-bound (about 180 instructions a point).
+// The point fields of every face, by groups with the same rule (nq points,
+// degree pr, ti 0 triangles, 1 quadrilaterals), all in one launch: geo[f * nq + q]
+// of face slot f.  NF faces per CTA: the vertex differences of both sides
+// first, then one or two points a thread.  FP64-bound (about 180 instructions a point)
+// where there are many faces (162,000: 720 us); a launch a group, each
+// waiting for its loads and one long chain a thread, took 34 us at 2,000 prisms
+// of p = 2 (68 us for both groups, 31 us in one launch of one point a
+// thread) and 46 us each for the eight groups of 8,000 prisms of p = 1..4
+// (368 us, 135 us).
 constexpr int FG_THREADS = 128;
+struct DgFieldGroup {
+  int block, first, count, NF, nq, pr, ti;
+};
+struct DgFieldGroups {
+  DgFieldGroup g[8];
+};
 __global__ void __launch_bounds__(FG_THREADS) dg_face_fields_kernel(
-    int count, const DgFaceRec *__restrict__ rec, int NF, int nq, int pr, int ti, const int *__restrict__ el_nodes,
+    DgFieldGroups groups, int ngroups, const DgFaceRec *__restrict__ rec, const int *__restrict__ el_nodes,
     const double *__restrict__ xyz, const double *__restrict__ k_el, const double *__restrict__ D_el, double pen,
     double *__restrict__ geo) {
+  int gi = 0;
+  while (gi + 1 < ngroups && (int)blockIdx.x >= groups.g[gi + 1].block) gi++;
+  const int NF = groups.g[gi].NF, nq = groups.g[gi].nq, pr = groups.g[gi].pr, ti = groups.g[gi].ti;
   extern __shared__ double smem[];  // [NF][2][30] differences and tensor, [NF] penalty / sqrt(area)
-  const int first = blockIdx.x * NF, nf = count - first < NF ? count - first : NF, tid = threadIdx.x;
+  const int at = (blockIdx.x - groups.g[gi].block) * NF, nf = min(NF, groups.g[gi].count - at);
+  const int first = groups.g[gi].first + at, tid = threadIdx.x;
   double *sPen = smem + 60 * NF;
   for (int t = tid; t < nf * 60; t += FG_THREADS) {
     const DgFaceRec &R = rec[first + t / 60];
@@ -682,13 +698,27 @@ __global__ void __launch_bounds__(FmOff<PM, QUAD>::THR) dg_face_blocks_kernel(
 }
 
 // ------------------------------------------------------------------ launches
-int launch_dg_face_fields(cudaStream_t st, int pm, int ti, int count, const DgFaceRec *rec, const int *el_nodes,
+// start[b] .. start[b + 1]: the records of rule degree b % 4 + 1, triangles (b < 4) or quadrilaterals
+int launch_dg_face_fields(cudaStream_t st, const int *start, const DgFaceRec *rec, const int *el_nodes,
                           const double *xyz, const double *k_el, const double *D_el, double pen, double *geo) {
-  if (count <= 0) return 0;
-  const int nq = GB_DG_NQF[pm][ti];
-  const int NF = 2 * FG_THREADS / nq;  // about two points a thread
-  dg_face_fields_kernel<<<(count + NF - 1) / NF, FG_THREADS, 61 * NF * sizeof(double), st>>>(
-      count, rec, NF, nq, pm, ti, el_nodes, xyz, k_el, D_el, pen, geo);
+  // one point a thread up to eight blocks an SM (2,000 prisms of p = 2: 31 us, two points 44;
+  // 54,000 of p = 3: 729 and 696)
+  long long points = 0;
+  for (int b = 0; b < 8; b++) points += (long long)(start[b + 1] - start[b]) * GB_DG_NQF[b % 4 + 1][b / 4];
+  const int per = points <= 8LL * 152 * FG_THREADS ? 1 : 2;
+  DgFieldGroups G;
+  int n = 0, blocks = 0, most = 0;
+  for (int b = 7; b >= 0; b--) {  // the longest first
+    const int count = start[b + 1] - start[b], nq = GB_DG_NQF[b % 4 + 1][b / 4];
+    if (count <= 0) continue;
+    const int NF = std::max(1, per * FG_THREADS / nq);
+    G.g[n++] = {blocks, start[b], count, NF, nq, b % 4 + 1, b / 4};
+    blocks += (count + NF - 1) / NF;
+    most = std::max(most, NF);
+  }
+  if (blocks == 0) return 0;
+  dg_face_fields_kernel<<<blocks, FG_THREADS, 61 * most * sizeof(double), st>>>(G, n, rec, el_nodes, xyz, k_el, D_el,
+                                                                                pen, geo);
   GB_CUDA(cudaGetLastError());
   return 1;
 }

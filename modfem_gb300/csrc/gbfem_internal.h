@@ -204,7 +204,7 @@ struct DgFaceRec {
 bool dg_face_moments_cover(const DgFaceRec &r);
 // Point fields of `count` faces of one rule (degree pm, ti 0 triangles, 1
 // quadrilaterals): 7 x nq doubles a face at geo + rec.geo
-int launch_dg_face_fields(cudaStream_t st, int pm, int ti, int count, const DgFaceRec *rec, const int *el_nodes,
+int launch_dg_face_fields(cudaStream_t st, const int *start, const DgFaceRec *rec, const int *el_nodes,
                           const double *xyz, const double *k_el, const double *D_el, double pen, double *geo);
 // Diagonal shares and boundary loads of the owners of degree p; hrec[h] = 2
 // record + (1 if the owner is its second neighbour) of half-face h.  variant:
