@@ -1682,6 +1682,7 @@ int gbfem_dg_get_structure(gbfem_ctx c, int *dof_off, int *bptr, int *bcol, long
 }
 
 // Point fields of every face of the moment form; returns the launches.
+constexpr int DG_BESIDE_MAX = 16384;
 int gbfem_dg_assemble(gbfem_ctx c) {
   GB_CHECK(c && c->dg_ready, "DG structure not built (gbfem_dg_build_structure)");
   GB_TRY(settle_uploads(c));
@@ -1735,6 +1736,40 @@ int gbfem_dg_assemble(gbfem_ctx c) {
       GB_TRY(r);
       launches += r;
     }
+    GB_CUDA(cudaEventRecord(c->side_ev[1], c->side_stream));
+  }
+  // Prism faces from moments, few elements: the point fields and the
+  // off-diagonal blocks read nothing that the volume and tetrahedron kernels
+  // write, and none of these fills the chip: they run beside on the side
+  // stream (assembly and download: 2,000 prisms of p = 2 320 -> 299 us, 8,000 of
+  // p = 1..4 4.22 -> 4.05 ms, prisms and tetrahedra 4.10 -> 3.99 ms; 54,000 of p =
+  // 3: 8 ms either way, so there each kernel keeps its own time).
+  const bool beside = mom && c->dg_hf.p && c->nel <= DG_BESIDE_MAX;
+  auto fields = [&](cudaStream_t st) -> int {
+    return gbfem::launch_dg_face_fields(st, c->dg_fb_start, c->dg_frec.p, c->el_nodes.p, c->xyz.p, c->k_el.p, c->D_el.p,
+                                        c->dg_pen, c->dg_ffield.p);
+  };
+  auto face_blocks = [&](cudaStream_t st) -> int {
+    int n = 0;
+    for (int b = 7; b >= 0; b--) {
+      const int r = gbfem::launch_dg_face_blocks(st, c->device, b % 4 + 1, b / 4, c->dg_fb_inner[b],
+                                                 c->dg_frec.p + c->dg_fb_start[b], c->dg_ffield.p, c->dg_val.p);
+      GB_TRY(r);
+      n += r;
+    }
+    return n;
+  };
+  if (beside) {
+    GB_TRY(ensure_side(c));
+    GB_TRY(c->dg_ffield.alloc((size_t)c->dg_ffield_n));
+    GB_CUDA(cudaEventRecord(c->side_ev[0], c->stream));
+    GB_CUDA(cudaStreamWaitEvent(c->side_stream, c->side_ev[0], 0));
+    int r = fields(c->side_stream);
+    GB_TRY(r);
+    launches += r;
+    GB_CUDA(cudaEventRecord(c->side_ev[2], c->side_stream));
+    GB_TRY(r = face_blocks(c->side_stream));
+    launches += r;
     GB_CUDA(cudaEventRecord(c->side_ev[1], c->side_stream));
   }
   for (int cls = 5; cls <= 8; cls++) {
@@ -1792,11 +1827,14 @@ int gbfem_dg_assemble(gbfem_ctx c) {
       launches += r;
     }
     if (mom) {
-      GB_TRY(c->dg_ffield.alloc((size_t)c->dg_ffield_n));
-      const int rf = gbfem::launch_dg_face_fields(c->stream, c->dg_fb_start, c->dg_frec.p, c->el_nodes.p, c->xyz.p,
-                                                  c->k_el.p, c->D_el.p, c->dg_pen, c->dg_ffield.p);
-      GB_TRY(rf);
-      launches += rf;
+      if (beside) {
+        GB_CUDA(cudaStreamWaitEvent(c->stream, c->side_ev[2], 0));
+      } else {
+        GB_TRY(c->dg_ffield.alloc((size_t)c->dg_ffield_n));
+        const int rf = fields(c->stream);
+        GB_TRY(rf);
+        launches += rf;
+      }
       for (int p = 1; p <= 4; p++) {
         if (!c->dg_list[p].p) continue;
         const int r = gbfem::launch_dg_face_diag(c->stream, c->device, p, (int)c->dg_list[p].n, c->dg_list[p].p,
@@ -1806,9 +1844,10 @@ int gbfem_dg_assemble(gbfem_ctx c) {
         GB_TRY(r);
         launches += r;
       }
-      for (int b = 7; b >= 0; b--) {
-        const int r = gbfem::launch_dg_face_blocks(c->stream, c->device, b % 4 + 1, b / 4, c->dg_fb_inner[b],
-                                                   c->dg_frec.p + c->dg_fb_start[b], c->dg_ffield.p, c->dg_val.p);
+      if (beside) {
+        GB_TRY(join_side(c, c->stream));
+      } else {
+        const int r = face_blocks(c->stream);
         GB_TRY(r);
         launches += r;
       }

@@ -381,7 +381,7 @@ struct gbfem_ctx_s {
   bool pipe_dword = false;
   // the boundary-face kernel runs beside the element kernel (atomic scatter)
   cudaStream_t side_stream = nullptr;
-  cudaEvent_t side_ev[2] = {};
+  cudaEvent_t side_ev[3] = {};  // work before, side work done, DG: face point fields done
   std::vector<int> pipe_el, pipe_rows;
   std::vector<int> pipe_maxnode, pipe_maxel;  // largest node / element index an element chunk reads
   // node coordinates and coefficients set while the tables are cached go up
