@@ -280,6 +280,12 @@ int gbfem_destroy(gbfem_ctx c) {
   c->dg_tcface.release();
   c->dg_fgeo.release();
   c->dg_fshare.release();
+  DevBuf<double> *rest[] = {&c->ek, &c->fk};
+  for (auto *b : rest) b->release();
+  DevBuf<int> *irest[] = {&c->con_node, &c->con_par, &c->con_lists, &c->inc_ptr, &c->inc, &c->fa_head, &c->fa_next};
+  for (auto *b : irest) b->release();
+  c->dg_valdw.release();
+  c->dg_dinvdw.release();
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
   cudaEventDestroy(c->ev2);
