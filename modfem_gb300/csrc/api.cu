@@ -280,7 +280,7 @@ int gbfem_destroy(gbfem_ctx c) {
   c->dg_tcface.release();
   c->dg_fgeo.release();
   c->dg_fshare.release();
-  DevBuf<double> *rest[] = {&c->ek, &c->fk};
+  DevBuf<double> *rest[] = {&c->ek, &c->fk, &c->dg_tet_tab};
   for (auto *b : rest) b->release();
   DevBuf<int> *irest[] = {&c->con_node, &c->con_par, &c->con_lists, &c->inc_ptr, &c->inc, &c->fa_head, &c->fa_next};
   for (auto *b : irest) b->release();
@@ -312,7 +312,7 @@ long long gbfem_device_bytes(gbfem_ctx c) {
   for (int cls = 0; cls < 9; cls++) s += c->dg_list[cls].bytes() + c->dg_mlist[cls].bytes();
   for (int p = 0; p < 5; p++) s += c->dg_flist_tc[p].bytes() + c->dg_flist_64[p].bytes();
   s += c->dg_mhf_ptr.bytes() + c->dg_mhf.bytes() + c->el_nodes4.bytes();
-  s += c->dg_frec.bytes() + c->dg_hrec.bytes() + c->dg_ffield.bytes();
+  s += c->dg_frec.bytes() + c->dg_hrec.bytes() + c->dg_ffield.bytes() + c->dg_tet_tab.bytes();
   return s;
 }
 
@@ -1823,12 +1823,14 @@ int gbfem_dg_assemble(gbfem_ctx c) {
     if (tcf && !tc && !overlap) GB_CUDA(cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream));
     for (int cls = 5; cls <= 8; cls++) {
       if (!c->dg_list[cls].p) continue;
+      if (!c->dg_tet_tab.p) {  // once per context
+        GB_TRY(c->dg_tet_tab.alloc((size_t)gbfem::dg_tet_face_table_size()));
+        GB_TRY(gbfem::launch_dg_tet_face_table(c->stream, c->dg_tet_tab.p));
+      }
       const int r = gbfem::launch_dg_tet_faces(c->stream, cls - 4, (int)c->dg_list[cls].n, c->dg_list[cls].p,
                                                c->dg_hf_ptr.p, c->dg_hf.p, c->dg_p_d.p, tet_nodes(c), c->xyz.p,
-                                               c->k_el.p, c->D_el.p, c->dg_pen, c->g, c->dg_boff_diag_d.p,
-                                               c->dg_roff_d.p, c->dg_val.p, c->dg_rhs.p,
-                                               c->dg_face_mode == GBFEM_DG_FACE_DWORD ||
-                                                   c->dg_face_mode == GBFEM_DG_FACE_TC_DWORD);
+                                               c->k_el.p, c->D_el.p, c->dg_pen, c->g, c->dg_tet_tab.p,
+                                               c->dg_boff_diag_d.p, c->dg_roff_d.p, c->dg_val.p, c->dg_rhs.p);
       GB_TRY(r);
       launches += r;
     }

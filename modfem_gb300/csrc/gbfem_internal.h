@@ -221,8 +221,11 @@ int launch_dg_tet_elements(cudaStream_t st, int device, int p, int count, const 
                            const long long *boff, const int *roff, double *val, double *rhs);
 int launch_dg_tet_faces(cudaStream_t st, int p, int count, const int *ent_el, const int *hf_ptr,
                         const DgHalfFace *hf, const int *el_p, const int *el_nodes, const double *xyz,
-                        const double *k_el, const double *D_el, double pen, double g, const long long *boff_diag,
-                        const int *roff, double *val, double *rhs, bool dword = false);
+                        const double *k_el, const double *D_el, double pen, double g, const double *tab,
+                        const long long *boff_diag, const int *roff, double *val, double *rhs);
+// the face mass matrices it reads (values; a constant table)
+long long dg_tet_face_table_size();
+int launch_dg_tet_face_table(cudaStream_t st, double *tab);
 // Faces between a prism and a tetrahedron (dg_mixed_faces.cu): owners of
 // class cls (1..4 prisms of degree cls, 5..8 tetrahedra of degree cls - 4),
 // their mixed half-faces mhf[mhf_ptr[e] .. mhf_ptr[e + 1]); prism vertices
@@ -442,6 +445,7 @@ struct gbfem_ctx_s {
   gbfem::DevBuf<gbfem::DgFaceRec> dg_frec;
   gbfem::DevBuf<int> dg_hrec;
   gbfem::DevBuf<double> dg_ffield;
+  gbfem::DevBuf<double> dg_tet_tab;  // face mass matrices of tetrahedra
   int dg_fb_start[9] = {}, dg_fb_inner[8] = {};
   long long dg_ffield_n = 0;
   bool dg_mom_ok = false;
