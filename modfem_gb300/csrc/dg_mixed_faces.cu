@@ -23,7 +23,10 @@
 // adds each face's share to it directly; it writes the whole off-diagonal
 // block (owner, neighbour), which no other face touches.  These faces lie on
 // the interface between the two element regions only, so the kernel is
-// sized for simplicity: every table in shared memory, 128 threads.
+// sized for simplicity: every table in shared memory, 128 threads.  The row
+// factors L = a (f g + c Phi) and M = -f a Phi are tables too, so an entry costs
+// two FP64 operations a point (five when they were formed per entry: owners
+// of degree 4 279 us, prisms, and 140, tetrahedra; 139 and 72 so).
 
 #include "dg_face.cuh"
 #include "gbfem_internal.h"
@@ -50,9 +53,11 @@ __global__ void __launch_bounds__(MF_THREADS) dg_mixed_faces_kernel(
     const double *__restrict__ xyz, const double *__restrict__ k_el, const double *__restrict__ D_el, double pen,
     const long long *__restrict__ boff_diag, double *__restrict__ val, int *__restrict__ err) {
   constexpr int NS = mf_ns(OTET, P);
-  __shared__ double sPhi[MF_NQ][MF_NCOL], sGam[MF_NQ][MF_NCOL];
+  extern __shared__ double mf_smem[];
+  double(*sPhi)[MF_NCOL] = reinterpret_cast<double(*)[MF_NCOL]>(mf_smem), (*sGam)[MF_NCOL] = sPhi + MF_NQ;
+  double(*sL)[NS] = reinterpret_cast<double(*)[NS]>(mf_smem + 2 * MF_NQ * MF_NCOL), (*sM)[NS] = sL + MF_NQ;
   __shared__ double sFac[MF_NQ][2][30];  // monomial factors per point and side (dg_point_factors)
-  __shared__ double sX[2][18], sA[2][9], sAw[MF_NQ], sN[3], sC;
+  __shared__ double sX[2][18], sA[2][9], sAw[MF_NQ], sN[3], sC, sD;
   __shared__ unsigned char sTexp[MF_TET_NS][3];
   const int bi = blockIdx.x;
   if (bi >= count) return;
@@ -121,9 +126,10 @@ __global__ void __launch_bounds__(MF_THREADS) dg_mixed_faces_kernel(
       sN[1] = n.y;
       sN[2] = n.z;
       sC = pen * (p1 < p2 ? p1 : p2) / sqrt(0.5 * d);
-      for (int q = 0; q < nq; q++) sAw[q] = d * mf_fq[pr - 1][0][q][2];
+      sD = d;
     }
     __syncthreads();
+    for (int q = tid; q < nq; q += MF_THREADS) sAw[q] = sD * mf_fq[pr - 1][0][q][2];
     // per (point, side): the point in that side's local coordinates, v and
     // the factor table
     for (int t = tid; t < 2 * nq; t += MF_THREADS) {
@@ -140,6 +146,7 @@ __global__ void __launch_bounds__(MF_THREADS) dg_mixed_faces_kernel(
       dg_point_factors(ev, v, sFac[q][sd]);
     }
     __syncthreads();
+    const double fac = 0.5, cp = sC;
     for (int t = tid; t < nq * nsum; t += MF_THREADS) {
       const int q = t / nsum, j = t - q * nsum;
       const int side = j < ns1 ? 0 : 1, jj = side == 0 ? j : j - ns1;
@@ -148,28 +155,30 @@ __global__ void __launch_bounds__(MF_THREADS) dg_mixed_faces_kernel(
       const unsigned char *ex = tet ? sTexp[jj] : mf_pexp[ps - 1][jj];
       double phi, g;
       dg_basis_from_factors(sFac[q][side], ex[0], ex[1], ex[2], phi, g);
-      sPhi[q][j] = side == 1 ? -phi : phi;
+      const double Phi = side == 1 ? -phi : phi;
+      sPhi[q][j] = Phi;
       sGam[q][j] = g;
+      if (side == own2) {
+        sL[q][jj] = sAw[q] * fma(fac, g, cp * Phi);
+        sM[q][jj] = -fac * sAw[q] * Phi;
+      }
     }
     __syncthreads();
-    const double fac = 0.5, cp = sC;
     const int own_lo = own2 ? ns1 : 0;
     // the face's share of the diagonal block, entry i + NS j
     for (int k = tid; k < NS * NS; k += MF_THREADS) {
-      const int i = k % NS + own_lo, j = k / NS + own_lo;
+      const int i = k % NS, j = k / NS + own_lo;
       double s = 0.0;
-      for (int q = 0; q < nq; q++)
-        s = fma(sAw[q], fma(fma(fac, sGam[q][i], cp * sPhi[q][i]), sPhi[q][j], -fac * sPhi[q][i] * sGam[q][j]), s);
+      for (int q = 0; q < nq; q++) s = fma(sL[q][i], sPhi[q][j], fma(sM[q][i], sGam[q][j], s));
       dblk[k] += s;
     }
     // block (owner, neighbour): NS x ns_nb, column-major, leading dimension NS
     const int nb_lo = own2 ? 0 : ns1, ns_nb = own2 ? ns1 : ns2;
     double *blk = val + F.blk;
     for (int k = tid; k < NS * ns_nb; k += MF_THREADS) {
-      const int i = k % NS + own_lo, j = k / NS + nb_lo;
+      const int i = k % NS, j = k / NS + nb_lo;
       double s = 0.0;
-      for (int q = 0; q < nq; q++)
-        s = fma(sAw[q], fma(fma(fac, sGam[q][i], cp * sPhi[q][i]), sPhi[q][j], -fac * sPhi[q][i] * sGam[q][j]), s);
+      for (int q = 0; q < nq; q++) s = fma(sL[q][i], sPhi[q][j], fma(sM[q][i], sGam[q][j], s));
       blk[k] = s;
     }
   }
@@ -181,19 +190,24 @@ int launch_dg_mixed_faces(cudaStream_t st, int cls, int count, const int *ent_el
                           const long long *boff_diag, double *val, int *err) {
   if (count <= 0) return 0;
   GB_CHECK(cls >= 1 && cls <= 2 * GB_DG_PMAX, "DG element class must be 1..8");
-#define GB_MF_LAUNCH(PP, TT)                                                                                   \
-  dg_mixed_faces_kernel<PP, TT><<<count, MF_THREADS, 0, st>>>(count, ent_el, mhf_ptr, mhf, el_p, el_nodes6,  \
-                                                              el_nodes4, xyz, k_el, D_el, pen, boff_diag, val, \
-                                                              err)
+#define GB_MF_LAUNCH(PP, TT)                                                                                  \
+  {                                                                                                           \
+    constexpr int bytes = 8 * 2 * MF_NQ * (MF_NCOL + mf_ns(TT, PP));                                          \
+    GB_CUDA(cudaFuncSetAttribute(dg_mixed_faces_kernel<PP, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
+                                 bytes));                                                                     \
+    dg_mixed_faces_kernel<PP, TT><<<count, MF_THREADS, bytes, st>>>(count, ent_el, mhf_ptr, mhf, el_p,        \
+                                                                    el_nodes6, el_nodes4, xyz, k_el, D_el,    \
+                                                                    pen, boff_diag, val, err);                \
+  }
   switch (cls) {
-    case 1: GB_MF_LAUNCH(1, false); break;
-    case 2: GB_MF_LAUNCH(2, false); break;
-    case 3: GB_MF_LAUNCH(3, false); break;
-    case 4: GB_MF_LAUNCH(4, false); break;
-    case 5: GB_MF_LAUNCH(1, true); break;
-    case 6: GB_MF_LAUNCH(2, true); break;
-    case 7: GB_MF_LAUNCH(3, true); break;
-    default: GB_MF_LAUNCH(4, true); break;
+    case 1: GB_MF_LAUNCH(1, false) break;
+    case 2: GB_MF_LAUNCH(2, false) break;
+    case 3: GB_MF_LAUNCH(3, false) break;
+    case 4: GB_MF_LAUNCH(4, false) break;
+    case 5: GB_MF_LAUNCH(1, true) break;
+    case 6: GB_MF_LAUNCH(2, true) break;
+    case 7: GB_MF_LAUNCH(3, true) break;
+    default: GB_MF_LAUNCH(4, true) break;
   }
 #undef GB_MF_LAUNCH
   GB_CUDA(cudaGetLastError());
