@@ -40,16 +40,16 @@ N_HEX = 100
 JITTER, SEED = 0.2, 1
 # FP64 work per std prism.  Textbook count of the reference algorithm:
 # nq*(151 + 18*ns + 2*ns) + 2*3*nq*ns^2 with nq = ns = 6.  The kernel's
-# quadrature-aggregated formulation executes 289 DFMA + 213 other FP64
+# quadrature-aggregated formulation executes 199 DFMA + 256 other FP64
 # instructions per element (ncu instruction mix, profiles/std_prism_elements_2M.md),
-# i.e. 791 flop and 502 FP64-pipe issue slots.
+# i.e. 654 flop and 455 FP64-pipe issue slots.
 TEXTBOOK_FLOP_PER_ELEM = 6 * (151 + 18 * 6 + 2 * 6) + 2 * 3 * 6 * 36
 # Algorithmic DRAM bytes per element of the 100^3 x 2 workload: connectivity
 # 24 + k 8 + coordinates 24 nno/nel + CRS values written once 8 nnz/nel +
 # rhs 8 ndof/nel + the 42-entry int32 assembly table 168 (302 B in all)
 ALG_BYTES_PER_ELEM = 24 + 8 + 24 * 1030301 / 2e6 + 8 * 21250901 / 2e6 + 8 * 1030301 / 2e6 + 4 * 42
-FLOP_PER_ELEM = 2 * 289 + 213
-FP64_SLOTS_PER_ELEM = 289 + 213
+FLOP_PER_ELEM = 2 * 199 + 256
+FP64_SLOTS_PER_ELEM = 199 + 256
 
 
 def parse():
@@ -324,7 +324,9 @@ def cpu_assemble(m, k, nthreads, reps=1):
 
 
 def dg_fma_per_element(p):
-    """FP64 FMAs of the DG volume kernel per element: nq (9 ns + 3 ns (ns+1)/2)."""
+    """FP64 FMAs of the sums over the quadrature points per element: nq (9 ns +
+    3 ns (ns+1)/2).  The kernel takes the entries from moments of the geometry,
+    6 to 8 times fewer operations: its rate of these FMAs passes the FP64 peak."""
     ns = {1: 6, 2: 18, 3: 40, 4: 75}[p]
     nq = {1: 6, 2: 18, 3: 48, 4: 80}[p]
     return nq * (9 * ns + 3 * ns * (ns + 1) // 2)
@@ -334,8 +336,9 @@ DG_NQF = {1: (3, 4), 2: (6, 9), 3: (12, 16), 4: (16, 25)}  # face rule points (t
 
 
 def dg_face_fma(F, pdeg):
-    """FP64 FMAs of the face block products: every face contributes its full
-    (ns1+ns2)^2 matrix (both owners' rows) at 2 FMA per entry and point."""
+    """FP64 FMAs of the face sums over the points: every face contributes its
+    full (ns1+ns2)^2 matrix (both owners' rows) at 2 FMA per entry and point
+    (the kernels use moments here too)."""
     ns = np.array([0, 6, 18, 40, 75])
     p1 = pdeg[F.el1]
     p2 = np.where(F.el2 >= 0, pdeg[np.maximum(F.el2, 0)], 0)
@@ -456,8 +459,8 @@ def bench_dg(gb, local, steps, fp64_peak, gmres_iters=100):
             "elements": m.nel, "faces": int(F.n), "dofs": nd, "stored_values": nv,
             "autotuned_shapes": {"volume": tuned_vol[1:].tolist(), "face": tuned_face[1:].tolist()},
             "assemble_ms": tot, "elem_per_s": m.nel / (tot * 1e-3),
-            "volume_ms": vol, "volume_fp64_frac": 2 * vfma / (vol * 1e-3) / 1e12 / fp64_peak,
-            "face_ms": fa, "face_fp64_frac": 2 * ffma / (fa * 1e-3) / 1e12 / fp64_peak,
+            "volume_ms": vol, "volume_point_sum_rate_over_fp64_peak": 2 * vfma / (vol * 1e-3) / 1e12 / fp64_peak,
+            "face_ms": fa, "face_point_sum_rate_over_fp64_peak": 2 * ffma / (fa * 1e-3) / 1e12 / fp64_peak,
             "tensor_core_volume": {"volume_ms": vol_tc, "assemble_ms": tot_tc, "elem_per_s": m.nel / (tot_tc * 1e-3),
                                    "max_abs_diff_vs_fp64_rel_to_max": tc_dev,
                                    "note": "tcgen05 split-BF16 products (p <= 3; p = 4 stays FP64)"},
@@ -468,12 +471,12 @@ def bench_dg(gb, local, steps, fp64_peak, gmres_iters=100):
                                              "others stay FP64)"},
             "double_word_assembly": dict(
                 dwf["double_word_assembly"],
-                note="volume and face entries summed in double-word (float pair) arithmetic on the FP32 pipes, "
-                     "all degrees"),
+                note="the double-word modes: prism volume and faces from FP64 moments (faster than double-word "
+                     "sums over the points), as the FP64 assembly; double words elsewhere"),
             "fastest_assembly": dict(
                 dwf["fastest_assembly"],
-                note="double-word volume (all degrees); split-BF16 tensor-core faces (owners and neighbours p <= 3), "
-                     "double-word faces for the rest"),
+                note="the fastest modes (DG_VOLUME_DWORD, DG_FACE_TC_DWORD): FP64 moments wherever the faces have "
+                     "the regular orientation, as the FP64 assembly"),
             "tf32_volume": {"volume_ms": vol_tf, "assemble_ms": tot_tf, "elem_per_s": m.nel / (tot_tf * 1e-3),
                             "max_abs_diff_vs_fp64_rel_to_max": tf_dev,
                             "note": "tcgen05 kind::tf32, hi/lo operands, FP32 accumulation (p <= 3)"},
@@ -593,13 +596,13 @@ def bench_batch(gb, local, steps, fp64_peak):
         "elements": NP + NT, "stored_values": nval, "rhs": nrhs,
         "autotuned_variants": {"prism": pv[1:].tolist(), "tet_elements_per_tile": [8 << int(v) for v in tv[1:]]},
         "step_ms": step_ms, "elem_per_s": (NP + NT) / (step_ms * 1e-3),
-        "fp64_frac": 2 * (pfma + tfma) / (step_ms * 1e-3) / 1e12 / fp64_peak,
+        "point_sum_rate_over_fp64_peak": 2 * (pfma + tfma) / (step_ms * 1e-3) / 1e12 / fp64_peak,
         "output_gbs": out_bytes / (step_ms * 1e-3) / 1e9,
         "tets_alone_ms": tet_ms, "tets_alone_output_gbs": 8 * (tnv + tnr) / (tet_ms * 1e-3) / 1e9,
         "prisms_per_degree_kernels_ms": per_degree_ms,
         "double_word_prisms": {"step_ms": dw_ms, "elem_per_s": (NP + NT) / (dw_ms * 1e-3),
                                "speedup_vs_fp64": step_ms / dw_ms, "max_abs_diff_vs_fp64_rel_to_max": dw_dev,
-                               "note": "prism stiffness sums in double-word (float pair) arithmetic, tetrahedra FP64"},
+                               "note": "prisms from FP64 moments in either arithmetic, tetrahedra FP64"},
         "e2e_ms": e2e_s * 1e3, "e2e_elem_per_s": (NP + NT) / e2e_s,
         "e2e_note": "page-locked host arrays: upload of geometry and tensors, tile build, graph capture, run, "
                     "download of "
@@ -921,8 +924,9 @@ def compact_line(full):
         d = dg.get(name)
         if not d:
             continue
-        out[key] = {"fp64_assemble_ms": _r(d["assemble_ms"]), "fp64_volume_frac": _r(d["volume_fp64_frac"], 3),
-                    "fp64_face_frac": _r(d["face_fp64_frac"], 3)}
+        out[key] = {"fp64_assemble_ms": _r(d["assemble_ms"]),
+                    "volume_point_sum_rate_over_fp64_peak": _r(d["volume_point_sum_rate_over_fp64_peak"], 3),
+                    "face_point_sum_rate_over_fp64_peak": _r(d["face_point_sum_rate_over_fp64_peak"], 3)}
         for form in ("tensor_core_assembly", "double_word_assembly", "fastest_assembly"):
             f = d[form]
             out[key][form] = {"assemble_ms": _r(f["assemble_ms"]), "face_ms": _r(f["face_ms"]),
@@ -935,7 +939,7 @@ def compact_line(full):
         out["mixed_precision_solution"] = mps.get("summary", mps)
     b = full["batch_mixed"]
     out["batch_mixed"] = {"step_ms": _r(b["step_ms"]), "elem_per_s": _r(b["elem_per_s"]),
-                          "fp64_frac": _r(b["fp64_frac"], 3),
+                          "point_sum_rate_over_fp64_peak": _r(b["point_sum_rate_over_fp64_peak"], 3),
                           "double_word_step_ms": _r(b["double_word_prisms"]["step_ms"])}
     # the mixed prism + tetrahedron workload as a whole step: the mixed-degree prism DG system and
     # the tetrahedral DG system (volume and faces each, measured above in this

@@ -273,10 +273,10 @@ int gbfem_dg_set_volume_kernel(gbfem_ctx ctx, int mode);
  * 2^-48 of the summed magnitudes, GBFEM_DG_FACE_TC_DWORD for the tensor cores
  * where they apply (prisms) and that accuracy elsewhere: between prisms the
  * FP64 kernel (moments of the face geometry) meets both and is the fastest,
- * so it serves them; tetrahedra, and prism meshes in which a quadrilateral is
- * turned by 90 degrees between its neighbours (the moment form does not cover
- * those), take the point sums in double-word (float pair) arithmetic on the
- * FP32 pipes (or the tensor cores). */
+ * so it serves them; tetrahedra take face mass matrices in FP64 in every
+ * mode; prism meshes in which a quadrilateral is turned by 90 degrees between
+ * its neighbours (the moment form does not cover those) take the point sums in
+ * double-word (float pair) arithmetic on the FP32 pipes (or the tensor cores). */
 #define GBFEM_DG_FACE_FP64 0
 #define GBFEM_DG_FACE_TC 1
 #define GBFEM_DG_FACE_DWORD 2
@@ -503,7 +503,10 @@ int gbfem_batch_get(gbfem_batch batch, double *vals, double *rhs);
  * alone and together).  The numerics per request are those of
  * gbfem_assemble + gbfem_solve (std) and gbfem_dg_assemble + gbfem_dg_solve
  * (DG): same assembly, same GMRES(krylov) with (block) Jacobi, stopping on the
- * preconditioned residual relative to the initial one. */
+ * preconditioned residual relative to the initial one.  The contexts of
+ * finished requests are kept for later ones of the same kind (up to 8 each, an
+ * eighth of the budget in all) and given back when the budget needs them or
+ * with the server. */
 #define GBFEM_SERVE_STD 0
 #define GBFEM_SERVE_DG 1
 typedef struct gbfem_server_s *gbfem_server;

@@ -163,7 +163,6 @@ int launch_multiaxpy(cudaStream_t st, int n, int m, const double *c, double sign
 int launch_orthogonalize(cudaStream_t st, int n, int m, const double *h, const double *base, long long ld, double *w,
                          double *partial, double *norm);
 int launch_normalize(cudaStream_t st, int n, const double *alpha, const double *x, double *y);
-int launch_mul(cudaStream_t st, int n, const double *a, double *y);
 int measure_fp64_peak(cudaStream_t st, int device, double *tflops);
 // restarted GMRES with point Jacobi on the context's CRS matrix, all of it on
 // the device (gmres_dev.cu); returns the iteration count

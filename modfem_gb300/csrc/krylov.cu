@@ -177,13 +177,6 @@ __global__ void __launch_bounds__(RED_THREADS) scale_kernel(int n, const double 
     y[i] = x[i] * inv;
 }
 
-// v = dinv .* (b - A x)  fused: first residual then scale (two kernels for clarity)
-__global__ void mul_kernel(int n, const double *__restrict__ a, double *__restrict__ y) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  y[i] *= a[i];
-}
-
 static inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 int launch_spmv(cudaStream_t st, int mode, int n, const int *row_ptr, const int *col_ind, const double *val,
@@ -244,12 +237,6 @@ int launch_orthogonalize(cudaStream_t st, int n, int m, const double *h, const d
 // y = x / alpha[0]
 int launch_normalize(cudaStream_t st, int n, const double *alpha, const double *x, double *y) {
   scale_kernel<<<reduction_blocks(n), RED_THREADS, 0, st>>>(n, alpha, x, y);
-  GB_CUDA(cudaGetLastError());
-  return 1;
-}
-
-int launch_mul(cudaStream_t st, int n, const double *a, double *y) {
-  mul_kernel<<<nblk(n, 256), 256, 0, st>>>(n, a, y);
   GB_CUDA(cudaGetLastError());
   return 1;
 }
