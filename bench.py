@@ -634,7 +634,7 @@ def bench_tet_dg(gb, local, steps):
         tt += np.array(c.dg_last_timing()[:3])
     tot, vol, fa = tt / steps
     v64, _ = c.dg_get_matrix()
-    # the faces summed in double-word arithmetic
+    # the double-word face mode (tetrahedra: the same FP64 kernel)
     c.dg_set_face_kernel(gb.DG_FACE_DWORD)
     c.dg_assemble()
     tt = np.zeros(3)
@@ -666,8 +666,8 @@ def bench_mixed_dg_system(gb, local, steps, n=63, layers=50):
     regions joined by 7,938 prism-tetrahedron triangles; p uniform in 1..4
     (seeded), lognormal(0,1) k, interior-penalty faces into the
     variable-block storage.  Assembly (volume and all faces) in plain FP64
-    and in the fastest form (double-word volume sums, split-BF16 tensor-core
-    faces between prisms), then a fixed 100 GMRES(50) iterations with block
+    and in the modes DG_VOLUME_DWORD, DG_FACE_TC_DWORD (the same kernels on this
+    mesh), then a fixed 100 GMRES(50) iterations with block
     Jacobi."""
     from modfem_gb300.mesh import lognormal_k, mixed_faces, structured_mixed_mesh
     m = structured_mixed_mesh(n, layers, jitter=0.2, seed=SEED)
