@@ -140,7 +140,8 @@ static int dg_spmv(gbfem_ctx c, int mode, const double *x, const double *b, doub
     }
     const int r = gbfem::launch_dg_block_spmv(c->stream, mode, cls, (int)c->dg_list[cls].n, c->dg_list[cls].p,
                                               c->dg_roff_d.p, c->dg_row_val_d.p, c->dg_cx_off_d.p, c->dg_colx_d.p,
-                                              c->dg_val.p, c->dg_dinv_off_d.p, c->dg_dinv.p, x, b, out);
+                                              c->dg_val.p, c->dg_dinv_off_d.p, c->dg_dinv.p, x, b, out,
+                                              c->dg_longest[cls]);
     if (r < 0) return r;
     n += r;
   }
@@ -1622,6 +1623,7 @@ int gbfem_dg_build_structure(gbfem_ctx c, int *ndof, long long *nval) {
     std::stable_sort(lst.begin(), lst.end(), [&](int a, int b) {
       return cx_off[a + 1] - cx_off[a] > cx_off[b + 1] - cx_off[b];
     });
+    c->dg_longest[cls] = (int)(cx_off[lst[0] + 1] - cx_off[lst[0]]);
     GB_TRY(upload(c, c->dg_list[cls], lst.data(), lst.size()));
     if (!mlst.empty()) GB_TRY(upload(c, c->dg_mlist[cls], mlst.data(), mlst.size()));
   }

@@ -309,7 +309,7 @@ template <typename VT>
 static int launch_dg_block_spmv_t(cudaStream_t st, int mode, int p, int count, const int *ent_el, const int *roff,
                                   const long long *row_val, const long long *cx_off, const int *colx, const VT *val,
                                   const long long *dinv_off, const VT *dinv, const double *x, const double *b,
-                                  double *out) {
+                                  double *out, int longest = 0) {
   if (count <= 0) return 0;
   GB_CHECK(mode >= 0 && mode <= 2, "bad block SpMV mode");
   GB_CHECK(p >= 1 && p <= 2 * GB_DG_PMAX, "DG block class must be 1..8 (prisms 1..4, tetrahedra 5..8)");
@@ -317,7 +317,7 @@ static int launch_dg_block_spmv_t(cudaStream_t st, int mode, int p, int count, c
   const int grid = (count + DGS_ROWS - 1) / DGS_ROWS;
 #define GB_DGS_LAUNCH(PP)                                                                                      \
   if constexpr (std::is_same<VT, double>::value) {                                                             \
-    if (count <= dgs_wide_max(PP)) {                                                                            \
+    if (count <= dgs_wide_max(PP, longest)) {                                                                   \
       dg_block_spmv_wide_kernel<PP><<<count, DGS_THREADS, 0, st>>>(mode, ent_el, roff, row_val, cx_off, colx,  \
                                                                    val, dinv_off, dinv, x, b, out);            \
       break;                                                                                                   \
@@ -343,9 +343,9 @@ static int launch_dg_block_spmv_t(cudaStream_t st, int mode, int p, int count, c
 int launch_dg_block_spmv(cudaStream_t st, int mode, int p, int count, const int *ent_el, const int *roff,
                          const long long *row_val, const long long *cx_off, const int *colx, const double *val,
                          const long long *dinv_off, const double *dinv, const double *x, const double *b,
-                         double *out) {
+                         double *out, int longest) {
   return launch_dg_block_spmv_t<double>(st, mode, p, count, ent_el, roff, row_val, cx_off, colx, val, dinv_off,
-                                        dinv, x, b, out);
+                                        dinv, x, b, out, longest);
 }
 
 int launch_dg_block_spmv32(cudaStream_t st, int mode, int p, int count, const int *ent_el, const int *roff,

@@ -155,10 +155,17 @@ struct DgWide {
 //   tetrahedra p = 1: never;                              p = 2: 1,296 16 / 18, 2,058 21 / 18
 //           p = 3: 2,058 25 / 38, 6,000 61 / 64;          p = 4: 2,058 52 / 134, 10,368 211 / 197
 // (the groups' time stays flat until they fill the chip: they walk a row's
-// columns one or two at a time)
-__host__ __device__ constexpr int dgs_wide_max(int cls) {
-  return cls == 1 ? 512 : cls == 2 ? 6656 : cls == 3 ? 10000 : cls == 4 ? 13000
-       : cls == 6 ? 1536 : cls == 7 ? 6144 : cls == 8 ? 8192 : 0;
+// columns one or two at a time).  In meshes of mixed degrees the rows of the low
+// classes are longer and the groups' walk with them, so the limit grows with
+// the class's longest row over that of a uniform mesh (6 or 5 blocks of its own).
+// Degrees 1..4 mixed, rows a class: prisms p = 1 2,048 22 / 97, 6,912 55 / 100, 16,384
+// 124 / 103 (limit 6,400); p = 2..4 16,384 183 / 246, 335 / 419, 653 / 1,000; tetrahedra
+// p = 1 1,500 15 / 40, 6,144 46 / 38 (4,480); p = 2 6,144 38 / 68, 15,972 90 / 75 (5,376).
+__host__ __device__ constexpr int dgs_wide_max(int cls, int longest = 0) {
+  constexpr int base[9] = {0, 512, 6656, 10000, 13000, 512, 1536, 6144, 8192};
+  constexpr int own[9] = {1, 36, 108, 240, 450, 20, 50, 100, 175};
+  if (cls == 5 && longest < 2 * own[5]) return 0;
+  return longest <= own[cls] ? base[cls] : (int)((long long)base[cls] * longest / own[cls]);
 }
 template <int P>
 __device__ __forceinline__ double dg_wide_product(const double *__restrict__ A, int nct, const int *__restrict__ cx,

@@ -277,7 +277,7 @@ int dg_invert_diagonal(gbfem_ctx c);  // every class of a context (api.cu)
 int launch_dg_block_spmv(cudaStream_t st, int mode, int p, int count, const int *ent_el, const int *roff,
                          const long long *row_val, const long long *cx_off, const int *colx, const double *val,
                          const long long *dinv_off, const double *dinv, const double *x, const double *b,
-                         double *out);
+                         double *out, int longest /* columns of the class's longest row */);
 // The same with the matrix and the arithmetic in FP32 (inner solves of
 // iterative refinement); vectors stay FP64.
 int launch_dg_block_spmv32(cudaStream_t st, int mode, int p, int count, const int *ent_el, const int *roff,
@@ -445,6 +445,7 @@ struct gbfem_ctx_s {
   gbfem::DevBuf<int> dg_hrec;
   gbfem::DevBuf<double> dg_ffield;
   gbfem::DevBuf<double> dg_tet_tab;  // face mass matrices of tetrahedra
+  int dg_longest[9] = {};  // columns of each class's longest block row
   int dg_fb_start[9] = {}, dg_fb_inner[8] = {};
   long long dg_ffield_n = 0;
   bool dg_mom_ok = false;

@@ -68,3 +68,33 @@ def test_block_products(gb, kind, p, n):
     np.add.at(mag.reshape(-1, ns), rows, a)
     v = c.dg_compute_residual(x)
     assert np.all(np.abs(v - ref) <= 2 * 525 * 2.0**-53 * mag)
+
+
+@pytest.mark.parametrize("kind,n", [("prism", 6), ("prism", 13), ("tet", 5), ("tet", 12)])
+def test_block_products_of_mixed_degrees(gb, kind, n):
+    """The same with degrees 1..4 mixed (the forms' limits follow the longest
+    row): rows of at most 6 x 75 columns, 2 x 450 x 2^-53 = 1e-13."""
+    import scipy.sparse as sp
+    from modfem_gb300.mesh import prism_faces, structured_prism_mesh, structured_tet_mesh, tet_faces
+    m = structured_prism_mesh(n, jitter=0.1, seed=n) if kind == "prism" else structured_tet_mesh(n, jitter=0.1, seed=n)
+    c = gb.Context(0)
+    c.set_mesh(m)
+    c.set_coefficients(k=np.ones(m.nel), f=1.0, g=0.3)
+    c.dg_set_degrees(np.random.default_rng(n).integers(1, 5, m.nel))
+    c.dg_set_faces(prism_faces(m) if kind == "prism" else tet_faces(m), penalty=10.0)
+    c.dg_build_structure()
+    c.dg_assemble()
+    vals, rhs = c.dg_get_matrix()
+    off, bptr, bcol, boff = c.dg_get_structure()
+    I, J, V = [], [], []
+    for e in range(m.nel):
+        ns = off[e + 1] - off[e]
+        lo, hi = boff[bptr[e]], boff[bptr[e + 1]]
+        cols = np.concatenate([np.arange(off[f], off[f + 1]) for f in bcol[bptr[e]:bptr[e + 1]]])
+        I.append(np.tile(np.arange(off[e], off[e + 1]), cols.size))
+        J.append(np.repeat(cols, ns))
+        V.append(vals[lo:hi])
+    A = sp.csr_matrix((np.concatenate(V), (np.concatenate(I), np.concatenate(J))))
+    x = np.random.default_rng(n).standard_normal(c.dg_ndof)
+    v = c.dg_compute_residual(x)
+    assert np.all(np.abs(v - (rhs - A @ x)) <= 2 * 451 * 2.0**-53 * (np.abs(rhs) + abs(A) @ np.abs(x)))
