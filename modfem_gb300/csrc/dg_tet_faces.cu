@@ -27,7 +27,7 @@
 // ascending order: 4 x 24), and a lower degree's is the leading part: one table
 // of 96 x 35 x 35 values for all degrees.  An entry is 7 FP64 operations
 // instead of 4 nq (or 2 nq double-word products).  2,300 tetrahedra of each degree
-// p = 1..4: 51, 94, 173, 404 us; 191, 247, 335, 721 us in double words over the points.
+// p = 1..4: 52, 84, 150, 346 us; 191, 247, 335, 721 us in double words over the points.
 
 #include "dg_face.cuh"
 #include "gbfem_internal.h"
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(T) dg_tet_faces_kernel(
     const double *__restrict__ k_el, const double *__restrict__ D_el, double pen, double gval,
     const double *__restrict__ tab, const long long *__restrict__ boff_diag, const int *__restrict__ roff,
     double *__restrict__ val, double *__restrict__ rhs) {
-  constexpr int NS = tt_ns(P), PER = (NS * NS + T - 1) / T;
+  constexpr int NS = tt_ns(P), NP = NS * (NS + 1) / 2, PER = (NP + T - 1) / T;
   __shared__ double sO[NS * NS], sN[TT_NS * NS];      // S owner-owner and owner-neighbour, [j][i]
   __shared__ double sV[TT_NF][2][3], sC[TT_NF][2];    // v of both sides; |ds|, |ds| c
   __shared__ double sCo[3][NS], sCn[3][TT_NS];        // |ds| f v_k e_k of the owner's and the neighbour's functions
@@ -131,9 +131,20 @@ __global__ void __launch_bounds__(T) dg_tet_faces_kernel(
       sDec[d][k] = (signed char)(x[d] ? tt_index(x[0] - (d == 0), x[1] - (d == 1), x[2] - (d == 2)) : k);
     }
   }
-  double acc[PER];
+  // diagonal share: thread's pairs (i <= j) of functions, both entries of each.  With
+  // R_ij = sum_k v_k e_k(i) S_{i-k,j} entry (i, j) is so (R_ij - R_ji) + c S_ij: R_ij
+  // and R_ji serve both
+  double acc[PER], acd[PER];
+  int pair[PER];
 #pragma unroll
-  for (int m = 0; m < PER; m++) acc[m] = 0.0;
+  for (int m = 0; m < PER; m++) {
+    acc[m] = acd[m] = 0.0;
+    const int k = min(tid + m * T, NP - 1);
+    int j = (int)((sqrtf(8.0f * k + 1.0f) - 1.0f) * 0.5f);
+    j += (j + 1) * (j + 2) / 2 <= k;
+    j -= j * (j + 1) / 2 > k;
+    pair[m] = (k - j * (j + 1) / 2) | j << 8;
+  }
   double racc[(NS + T - 1) / T];
 #pragma unroll
   for (int m = 0; m < (NS + T - 1) / T; m++) racc[m] = 0.0;
@@ -197,19 +208,19 @@ __global__ void __launch_bounds__(T) dg_tet_faces_kernel(
         sCn[d][k - NS] = df * sV[slot][own ^ 1][d] * sExp[d][k - NS];
     }
     __syncthreads();
-    // the face's share of the diagonal block: entry k = i + NS j
 #pragma unroll
     for (int m = 0; m < PER; m++) {
-      const int k = tid + m * T;
-      if (k < NS * NS) {
-        const int i = k % NS, j = k / NS;
+      if (tid + m * T < NP) {
+        const int i = pair[m] & 255, j = pair[m] >> 8;
         double r = 0.0, c = 0.0;
 #pragma unroll
         for (int d = 0; d < 3; d++) {
           r = fma(sCo[d][i], sO[sDec[d][i] + NS * j], r);
-          c = fma(sCo[d][j], sO[i + NS * sDec[d][j]], c);
+          c = fma(sCo[d][j], sO[sDec[d][j] + NS * i], c);
         }
-        acc[m] += fma(so, r - c, pc * sO[k]);
+        const double q = so * (r - c), g = pc * sO[i + NS * j];
+        acc[m] += g + q;
+        acd[m] += g - q;
       }
     }
     if (interior) {
@@ -242,8 +253,10 @@ __global__ void __launch_bounds__(T) dg_tet_faces_kernel(
   double *dblk = val + boff_diag[e];
 #pragma unroll
   for (int m = 0; m < PER; m++) {
-    const int k = tid + m * T;
-    if (k < NS * NS) dblk[k] += acc[m];
+    if (tid + m * T >= NP) continue;
+    const int i = pair[m] & 255, j = pair[m] >> 8;
+    dblk[i + NS * j] += acc[m];
+    if (i != j) dblk[j + NS * i] += acd[m];
   }
 #pragma unroll
   for (int m = 0; m < (NS + T - 1) / T; m++) {
