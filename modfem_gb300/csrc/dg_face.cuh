@@ -154,6 +154,20 @@ GB_HD v3 tet_face_v(const double *X, const double *A, v3 n) {
   return {v3_dot(c1, an) * rdet, v3_dot(c2, an) * rdet, v3_dot(c3, an) * rdet};
 }
 
+// Configuration of a tetrahedron face, 0 .. 95: how it sits in its owner (local
+// vertices lo) and in the other element (ln), both in face order.  A face that
+// names a vertex twice sits in none of the 96 ways and has no area, which alone
+// decides its entries (NaN, or rounding of the area); it takes the nearest place.
+GB_HD int tet_face_config(const unsigned char *lo, const unsigned char *ln) {
+  int a = lo[0], b = lo[1], c = lo[2], x = ln[0], y = ln[1], z = ln[2], t;
+  if (a > b) { t = a; a = b; b = t; t = x; x = y; y = t; }
+  if (b > c) { t = b; b = c; c = t; t = y; y = z; z = t; }
+  if (a > b) { t = a; a = b; b = t; t = x; x = y; y = t; }
+  const int code = 6 * x + 2 * (y - (y > x)) + (z - (z > x) - (z > y));
+  const int cfg = 24 * (6 - a - b - c) + code;
+  return cfg < 0 ? 0 : cfg > 95 ? 95 : cfg;
+}
+
 // Per point and side, the monomial factors of the basis: powers
 // T[k][m] = x_k^m and the gradient factors T[3 + k][m] = m x_k^(m-1) v_k
 // (m = 0..4, k = xi, eta, zeta), so that for xi^a eta^b zeta^c

@@ -98,16 +98,6 @@ __global__ void dg_tet_face_table_kernel(double *__restrict__ tab) {
   }
 }
 
-// configuration of a face: the owner's local vertices lo and the other's ln, both in face order
-__device__ __forceinline__ int tt_config(const unsigned char *lo, const unsigned char *ln) {
-  int a = lo[0], b = lo[1], c = lo[2], x = ln[0], y = ln[1], z = ln[2], t;
-  if (a > b) { t = a; a = b; b = t; t = x; x = y; y = t; }
-  if (b > c) { t = b; b = c; c = t; t = y; y = z; z = t; }
-  if (a > b) { t = a; a = b; b = t; t = x; x = y; y = t; }
-  const int code = 6 * x + 2 * (y - (y > x)) + (z - (z > x) - (z > y));
-  return 24 * (6 - a - b - c) + code;
-}
-
 template <int P, int T = tt_threads(P)>
 __global__ void __launch_bounds__(T) dg_tet_faces_kernel(
     int count, const int *__restrict__ ent_el, const int *__restrict__ hf_ptr, const DgHalfFace *__restrict__ hf,
@@ -192,10 +182,10 @@ __global__ void __launch_bounds__(T) dg_tet_faces_kernel(
     const bool interior = F.el2 >= 0;
     const int own = F.owner_is_2, ns_nb = interior ? tt_ns(el_p[own ? F.el1 : F.el2]) : 0;
     const unsigned char *lo = own ? F.loc2 : F.loc1, *ln = own ? F.loc1 : F.loc2;
-    const double *to = tab + (size_t)tt_config(lo, lo) * TT_NS * TT_NS;
+    const double *to = tab + (size_t)tet_face_config(lo, lo) * TT_NS * TT_NS;
     for (int t = tid; t < NS * NS; t += T) sO[t] = to[t / NS * TT_NS + t % NS];
     if (interior) {
-      const double *tn = tab + (size_t)tt_config(lo, ln) * TT_NS * TT_NS;
+      const double *tn = tab + (size_t)tet_face_config(lo, ln) * TT_NS * TT_NS;
       for (int t = tid; t < NS * ns_nb; t += T) sN[t] = tn[t / NS * TT_NS + t % NS];
     }
     __syncthreads();

@@ -52,3 +52,42 @@ def test_tet_faces_in_all_positions_vs_oracle(gb, seed, dword):
     ref = dense[np.repeat(np.arange(nd), np.diff(rp)), ci]
     assert sparse_rel_err(rp, ci, v, ref) < REL_TOL
     assert vec_rel_err(rhs, np.concatenate(R)) < REL_TOL
+
+
+@pytest.mark.parametrize("p", [1, 2, 3, 4])
+@pytest.mark.parametrize("interior", [True, False])
+def test_face_with_a_vertex_twice(gb, p, interior):
+    """A face of no area (its first vertex named twice) has no normal: the
+    blocks and load of its owners are NaN, every other row is untouched."""
+    from modfem_gb300.mesh import structured_tet_mesh, tet_faces
+    m = structured_tet_mesh(2, jitter=0.1, seed=p)
+    F = tet_faces(m)
+    f = int(np.flatnonzero((F.el2 >= 0) == interior)[5])
+    owners = [int(e) for e in (F.el1[f], F.el2[f]) if e >= 0]
+
+    def system(nodes):
+        F.nodes[f, :3] = nodes
+        c = gb.Context(0)
+        c.set_mesh(m)
+        c.set_coefficients(k=np.ones(m.nel), f=1.0, g=0.3)
+        c.dg_set_degrees(np.full(m.nel, p))
+        c.dg_set_faces(F, penalty=10.0)
+        c.dg_build_structure()
+        c.dg_assemble()
+        out = c.dg_get_matrix() + tuple(c.dg_get_structure())
+        c.close()
+        return out
+
+    nodes = F.nodes[f, :3].copy()
+    v0, r0, off, bptr, bcol, boff = system(nodes)
+    v1, r1 = system(nodes[[0, 0, 2]])[:2]
+    for e in range(m.nel):
+        touched = e in owners
+        assert touched or np.array_equal(r0[off[e]:off[e + 1]], r1[off[e]:off[e + 1]])
+        assert not touched or interior or np.all(np.isnan(r1[off[e]:off[e + 1]]))
+        for b in range(bptr[e], bptr[e + 1]):
+            x, y = v0[boff[b]:boff[b + 1]], v1[boff[b]:boff[b + 1]]
+            if touched and bcol[b] in owners:
+                assert np.all(np.isnan(y))
+            else:
+                assert np.array_equal(x, y)
