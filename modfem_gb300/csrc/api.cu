@@ -218,75 +218,15 @@ int gbfem_destroy(gbfem_ctx c) {
     for (auto &ev : c->pipe_ev)
       if (ev) cudaEventDestroy(ev);
   }
-  c->row_last.release();
   if (c->gm_graph) cudaGraphExecDestroy(c->gm_graph);
   if (c->gm_host) cudaFreeHost(c->gm_host);
-  c->sell_off.release();
-  c->sell_col.release();
-  c->sell_col16.release();
-  c->sell_val.release();
-  c->sell_valdw.release();
-  c->gm_xdw.release();
-  c->gm_small.release();
-  c->gm_npart.release();
-  c->gm_alive.release();
   if (c->side_stream) {
     cudaStreamSynchronize(c->side_stream);
     cudaStreamDestroy(c->side_stream);
     for (auto &ev : c->side_ev)
       if (ev) cudaEventDestroy(ev);
   }
-  DevBuf<double> *dbufs[] = {&c->xyz, &c->k_el, &c->D_el, &c->val, &c->rhs, &c->dinv, &c->V,
-                             &c->w, &c->tmp, &c->x, &c->b, &c->partial, &c->hcol};
-  for (auto *b : dbufs) b->release();
-  DevBuf<int> *ibufs[] = {&c->el_nodes, &c->fa_el, &c->fa_side, &c->row_ptr, &c->col_ind, &c->dof_of_node,
-                          &c->el_table, &c->el_perm, &c->fa_perm, &c->fa_map, &c->err, &c->in_id,
-                          &c->in_pos, &c->in_table, &c->dg_roff_d};
-  for (auto *b : ibufs) b->release();
-  for (int cls = 0; cls < 9; cls++) {
-    c->dg_list[cls].release();
-    c->dg_mlist[cls].release();
-  }
-  for (int p = 0; p < 5; p++) {
-    c->dg_flist_tc[p].release();
-    c->dg_flist_64[p].release();
-  }
-  c->dg_mhf_ptr.release();
-  c->dg_mhf.release();
-  c->dg_frec.release();
-  c->dg_hrec.release();
-  c->dg_ffield.release();
-  c->el_nodes4.release();
-  c->dg_boff_diag_d.release();
-  c->dg_val.release();
-  c->dg_rhs.release();
-  c->dg_hf_ptr.release();
-  c->dg_p_d.release();
-  c->dg_hf.release();
-  c->dg_dinv.release();
-  c->dg_dinv_off_d.release();
-  c->dg_bptr_d.release();
-  c->dg_bcol_d.release();
-  c->dg_boff_d.release();
-  c->dg_val32.release();
-  c->dg_dinv32.release();
-  c->ir_x.release();
-  c->ir_r.release();
-  c->dg_colx_d.release();
-  c->dg_row_val_d.release();
-  c->dg_cx_off_d.release();
-  c->dg_fcfg.release();
-  c->dg_ftab_off.release();
-  c->dg_ftab.release();
-  c->dg_tcface.release();
-  c->dg_fgeo.release();
-  c->dg_fshare.release();
-  DevBuf<double> *rest[] = {&c->ek, &c->fk, &c->dg_tet_tab};
-  for (auto *b : rest) b->release();
-  DevBuf<int> *irest[] = {&c->con_node, &c->con_par, &c->con_lists, &c->inc_ptr, &c->inc, &c->fa_head, &c->fa_next};
-  for (auto *b : irest) b->release();
-  c->dg_valdw.release();
-  c->dg_dinvdw.release();
+  c->each_buffer([](auto &b) { b.release(); });
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
   cudaEventDestroy(c->ev2);
@@ -299,21 +239,7 @@ int gbfem_destroy(gbfem_ctx c) {
 long long gbfem_device_bytes(gbfem_ctx c) {
   if (!c) return 0;
   long long s = 0;
-  const DevBuf<double> *dbufs[] = {&c->xyz, &c->k_el, &c->D_el, &c->val, &c->rhs, &c->dinv, &c->V,
-                                   &c->w, &c->tmp, &c->x, &c->b, &c->partial, &c->hcol};
-  for (auto *b : dbufs) s += b->bytes();
-  const DevBuf<int> *ibufs[] = {&c->el_nodes, &c->fa_el, &c->fa_side, &c->row_ptr, &c->col_ind,
-                                &c->dof_of_node, &c->el_table, &c->el_perm, &c->fa_perm, &c->fa_map,
-                                &c->err, &c->in_id, &c->in_pos, &c->in_table};
-  for (auto *b : ibufs) s += b->bytes();
-  s += c->dg_val.bytes() + c->dg_rhs.bytes() + c->dg_dinv.bytes() + c->dg_hf.bytes() + c->dg_boff_d.bytes() +
-       c->dg_boff_diag_d.bytes() + c->dg_dinv_off_d.bytes() + c->dg_bptr_d.bytes() + c->dg_bcol_d.bytes() +
-       c->dg_hf_ptr.bytes() + c->dg_p_d.bytes() + c->dg_roff_d.bytes() + c->dg_colx_d.bytes() +
-       c->dg_row_val_d.bytes() + c->dg_cx_off_d.bytes();
-  for (int cls = 0; cls < 9; cls++) s += c->dg_list[cls].bytes() + c->dg_mlist[cls].bytes();
-  for (int p = 0; p < 5; p++) s += c->dg_flist_tc[p].bytes() + c->dg_flist_64[p].bytes();
-  s += c->dg_mhf_ptr.bytes() + c->dg_mhf.bytes() + c->el_nodes4.bytes();
-  s += c->dg_frec.bytes() + c->dg_hrec.bytes() + c->dg_ffield.bytes() + c->dg_tet_tab.bytes();
+  c->each_buffer([&](const auto &b) { s += (long long)b.bytes(); });
   return s;
 }
 

@@ -471,4 +471,24 @@ struct gbfem_ctx_s {
   float last_ms = 0.f, last_el_ms = 0.f, last_fa_ms = 0.f, last_solve_ms = 0.f, last_spmv_ms = 0.f;
   int last_spmv_count = 0, last_solve_kernels = 0;
   int last_launches = 0;
+
+  // f(buffer) for every device buffer above: what the context holds
+  // (gbfem_device_bytes) and gives back (gbfem_destroy)
+  template <class F>
+  void each_buffer(F f) {
+    auto all = [&](auto &...b) { (f(b), ...); };
+    all(xyz, el_nodes, el_nodes4, fa_el, fa_side, con_node, con_par, con_lists, k_el, D_el);
+    all(row_ptr, col_ind, dof_of_node, el_table, el_perm, fa_perm, fa_map);
+    all(inc_ptr, inc, fa_head, fa_next, ek, fk, val, rhs, dinv, err, in_id, in_pos, in_table, row_last);
+    all(V, w, tmp, x, b, partial, hcol);
+    all(sell_off, sell_col, sell_val, gm_small, gm_npart, gm_alive, sell_valdw, gm_xdw, sell_col16);
+    for (auto &l : dg_list) f(l);
+    for (auto &l : dg_mlist) f(l);
+    for (auto &l : dg_flist_tc) f(l);
+    for (auto &l : dg_flist_64) f(l);
+    all(dg_roff_d, dg_mhf_ptr, dg_mhf, dg_boff_diag_d, dg_val, dg_rhs, dg_hf_ptr, dg_p_d, dg_hf);
+    all(dg_frec, dg_hrec, dg_ffield, dg_tet_tab, dg_fcfg, dg_ftab_off, dg_ftab, dg_fgeo, dg_fshare, dg_tcface);
+    all(dg_dinv, dg_val32, dg_dinv32, dg_valdw, dg_dinvdw, ir_x, ir_r);
+    all(dg_dinv_off_d, dg_bptr_d, dg_bcol_d, dg_colx_d, dg_boff_d, dg_row_val_d, dg_cx_off_d);
+  }
 };
