@@ -62,6 +62,7 @@
 #include <vector>
 
 #include "dg_spmv.cuh"
+#include "dg_tables.h"
 #include "gbfem_internal.h"
 #include "gmres_step.cuh"
 
@@ -336,17 +337,24 @@ using ReqPtr = std::shared_ptr<SrvRequest>;
 
 }  // namespace
 
-long long gbfem_serve_footprint_impl(int kind, int p, int nno, int nel, int nbf, int nfa, int krylov) {
+// What a request's context and Krylov space will hold (a std request's sliced-ELL
+// copy only when it is solved alone); the rounded part covers the small arrays
+// and the basis tables of the face configurations.  ntri of the nfa faces are triangles.
+long long gbfem_serve_footprint_impl(int kind, int p, int nno, int nel, int nbf, int nfa, int ntri, int krylov) {
   const long long m1 = krylov + 1;
-  long long b = 24LL * nno + 24LL * nel + 8LL * nel + 16LL * nbf + (1LL << 20);
+  long long b = 24LL * nno + 24LL * nel + 8LL * nel + 16LL * nbf + (3LL << 18);
   if (kind == 0) {
     const long long n = nno, nnz = 27LL * nno;  // prism meshes hold about 21 entries per row
-    b += 12LL * nnz + 4LL * (n + 1) + 4LL * nno + 168LL * nel + 8LL * nel + 16LL * nbf;  // CRS, tables, colours
-    b += 336LL * nel + 24LL * nel + 4LL * (n + 1);  // gather scatter: local matrices, incidence
-    b += 8LL * n * (m1 + 4) + 8LL * m1 * m1;                                           // Krylov
+    b += 12LL * nnz + 4LL * (n + 1) + 4LL * nno + 168LL * nel;                // CRS, tables
+    b += 336LL * nel + 28LL * nel + 4LL * (n + 2) + (112LL + 4) * nbf;        // gather scatter: local matrices, incidence, face lists
+    b += 8LL * n * (m1 + 4) + 8LL * m1 * m1 + 8LL * 152 * (m1 + 8);           // Krylov
+    b += 12LL * nnz + 4LL * n;                                                // sliced-ELL copy
   } else {
     const long long ns = kNs[p], n = ns * nel, blocks = nel + 2LL * nfa;
-    b += 8LL * ns * ns * blocks + 8LL * ns * ns * nel + 4LL * ns * blocks + 64LL * nel + 48LL * 2 * nfa;
+    b += 8LL * ns * ns * blocks + 8LL * ns * ns * nel + (4LL * ns + 12) * blocks + 64LL * nel;
+    // half-faces, face records, point fields (7 doubles a point)
+    b += (96 + 8 + (long long)sizeof(gbfem::DgFaceRec)) * nfa;
+    b += 56LL * (GB_DG_NQF[p][0] * (long long)ntri + GB_DG_NQF[p][1] * (long long)(nfa - ntri));
     b += 8LL * n * (m1 + 4) + 8LL * m1 * m1;
   }
   return b;
@@ -1046,7 +1054,9 @@ extern "C" {
 
 long long gbfem_serve_footprint(const gbfem_serve_request *q) {
   if (!q) return -2;
-  return gbfem_serve_footprint_impl(q->kind, q->dg_p, q->nno, q->nel, q->nbf, q->nfa, q->krylov);
+  int ntri = 0;
+  for (int f = 0; q->kind == GBFEM_SERVE_DG && q->fa_type && f < q->nfa; f++) ntri += q->fa_type[f] == 3;
+  return gbfem_serve_footprint_impl(q->kind, q->dg_p, q->nno, q->nel, q->nbf, q->nfa, ntri, q->krylov);
 }
 
 int gbfem_server_create(gbfem_server *out, int device, long long hbm_budget, int max_active, int prep_threads) {

@@ -1,0 +1,61 @@
+"""The serving engine's memory accounting (GPU): what a request is admitted
+with against what it then holds."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gb():
+    import modfem_gb300 as g
+    g.load_library()
+    return g
+
+
+def _krylov_bytes(n, m):
+    """A lane's Krylov space: x, tmp, m + 1 vectors, Hessenberg matrix, six rows."""
+    m1 = m + 1
+    return 8 * (n * (m1 + 2) + m1 * m1 + 6 * (m1 + 1))
+
+
+@pytest.mark.parametrize("krylov", [10, 60])
+@pytest.mark.parametrize("n", [1, 5, 20, 40])
+def test_std_footprint_covers_what_is_held(gb, n, krylov):
+    """In a lane (CRS rows, a Krylov space of its own) and alone (sliced-ELL
+    copy and the context's vectors)."""
+    from modfem_gb300.mesh import structured_prism_mesh
+    from modfem_gb300.serve import STD, Problem
+    m = structured_prism_mesh(n, jitter=0.1, seed=n)
+    pr = Problem(m, np.ones(m.nel), kind=STD, krylov=krylov)
+    c = gb.Context(0)
+    c.set_mesh(m)
+    c.set_coefficients(k=pr.k, f=1.0)
+    c.build_structure_device()
+    c.assemble(gb.SCATTER_GATHER)
+    lane = c.device_bytes() + 8 * m.nno + _krylov_bytes(m.nno, krylov)
+    c.solve(krylov, krylov, 1e-12)
+    alone = c.device_bytes()
+    c.close()
+    assert max(lane, alone) <= pr.footprint(), (lane, alone, pr.footprint())
+
+
+@pytest.mark.parametrize("p", [1, 2, 3, 4])
+@pytest.mark.parametrize("n", [1, 4, 12])
+def test_dg_footprint_covers_what_is_held(gb, n, p):
+    from modfem_gb300.mesh import prism_faces, structured_prism_mesh
+    from modfem_gb300.serve import DG, Problem
+    m = structured_prism_mesh(n, jitter=0.1, seed=n)
+    F = prism_faces(m)
+    pr = Problem(m, np.ones(m.nel), kind=DG, p=p, faces=F, krylov=30)
+    c = gb.Context(0)
+    c.set_mesh(m)
+    c.set_coefficients(k=pr.k, f=1.0)
+    c.dg_set_degrees(np.full(m.nel, p))
+    c.dg_set_faces(F, penalty=10.0)
+    c.dg_build_structure()
+    c.dg_assemble()
+    ns = c.dg_ndof // m.nel
+    held = c.device_bytes() + 8 * ns * ns * m.nel + _krylov_bytes(c.dg_ndof, 30)
+    c.close()
+    assert held <= pr.footprint(), (held, pr.footprint())
