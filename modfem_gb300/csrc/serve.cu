@@ -480,7 +480,8 @@ void reap(gbfem_server s, SrvRequest &r, bool reusable = true) {
       drop_oldest_idle(s);
       same--;
     }
-    if (s->idle_bytes + i.bytes <= s->budget / 8 && s->in_use + s->idle_bytes + i.bytes <= s->budget) {
+    if (s->idle_bytes + i.bytes <= s->budget / 8 &&
+        s->in_use - r.charged + s->idle_bytes + i.bytes <= s->budget) {  // (its charge ends with it)
       s->idle_bytes += i.bytes;
       s->idle.push_back(i);
       return;
@@ -491,7 +492,10 @@ void reap(gbfem_server s, SrvRequest &r, bool reusable = true) {
 }
 
 // An idle context for the request, of its own mesh size if there is one (its
-// buffers then fit as they are)
+// buffers then fit as they are).  What it holds is charged beside the estimate
+// (buffers only grow, so the two together bound what it will hold) until the
+// preparation puts the measured footprint in their place, or, for a request solved
+// alone, until it is done.
 bool take_idle(gbfem_server s, SrvRequest &r) {
   std::lock_guard<std::mutex> lk(s->mu);
   const int key = idle_key(r);
@@ -505,6 +509,9 @@ bool take_idle(gbfem_server s, SrvRequest &r) {
   r.ctx = best->ctx;
   r.kry = best->kry;
   s->idle_bytes -= best->bytes;
+  s->in_use += best->bytes;
+  r.charged += best->bytes;
+  s->peak_in_use = std::max(s->peak_in_use, s->in_use);
   s->idle.erase(best);
   return true;
 }
@@ -721,7 +728,7 @@ void prep_worker(gbfem_server s) {
 
 // Solo requests (large std): gbfem_solve's device GMRES on the request's own
 // stream and restart-cycle graph, beside the engine's batched lanes; the
-// estimate (which includes the Krylov space) stays charged until done.
+// estimate (which includes the Krylov space and the sliced-ELL copy) stays charged until done.
 void solo_worker(gbfem_server s) {
   cudaSetDevice(s->device);
   for (;;) {

@@ -59,3 +59,29 @@ def test_dg_footprint_covers_what_is_held(gb, n, p):
     held = c.device_bytes() + 8 * ns * ns * m.nel + _krylov_bytes(c.dg_ndof, 30)
     c.close()
     assert held <= pr.footprint(), (held, pr.footprint())
+
+
+def test_small_request_in_a_large_context_is_charged_for_it(gb):
+    """A solo request of 2,197 unknowns in the context that one of 68,921 has
+    left: while it is solved, the charge covers what the larger context holds
+    (at least its local matrices, 336 B a prism, and its 31 Krylov vectors)."""
+    import time
+    from modfem_gb300.mesh import lognormal_k, structured_prism_mesh
+    from modfem_gb300.serve import STD, Problem, Server
+    big, small = structured_prism_mesh(40), structured_prism_mesh(12)
+    held = 336 * big.nel + 8 * 31 * big.nno
+    srv = Server(0, prep_threads=1)
+    try:
+        srv.set_solo_dofs(1000)
+        rid = srv.submit(Problem(big, np.ones(big.nel), kind=STD, krylov=30, max_iter=5, tol=1e-10))
+        assert srv.wait(rid, 120.0) == 1
+        # (20,000 restarts of one vector: some 0.5 s)
+        rid = srv.submit(Problem(small, lognormal_k(small.nel, seed=1), kind=STD, krylov=1, max_iter=20000, tol=1e-12))
+        end = time.time() + 60.0
+        while srv.stats()["active"] == 0 and time.time() < end:
+            time.sleep(1e-3)
+        st = srv.stats()
+        assert srv.wait(rid, 120.0) == 1
+    finally:
+        srv.close()
+    assert st["active"] == 1 and held <= st["bytes"] <= st["budget"]
