@@ -449,9 +449,11 @@ void drop_oldest_idle(gbfem_server s) {  // caller holds s->mu
   s->cv_reap.notify_one();
 }
 
-// Whether `bytes` more fit in the HBM budget (idle contexts give way); a
-// request larger than the budget runs alone.
+// Whether `bytes` more fit in the HBM budget (idle contexts give way, but not
+// for a request that would have to wait all the same); a request larger than the
+// budget runs alone.
 bool fits(gbfem_server s, long long bytes) {  // caller holds s->mu
+  if (s->in_use > 0 && s->in_use + bytes > s->budget) return false;
   while (!s->idle.empty() && s->in_use + s->idle_bytes + bytes > s->budget) drop_oldest_idle(s);
   return s->in_use + bytes <= s->budget || s->in_use == 0;
 }

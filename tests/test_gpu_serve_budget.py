@@ -85,3 +85,42 @@ def test_small_request_in_a_large_context_is_charged_for_it(gb):
     finally:
         srv.close()
     assert st["active"] == 1 and held <= st["bytes"] <= st["budget"]
+
+
+def _free():
+    import ctypes
+    cu = ctypes.CDLL("libcuda.so.1")
+    free, total = ctypes.c_size_t(), ctypes.c_size_t()
+    assert cu.cuMemGetInfo_v2(ctypes.byref(free), ctypes.byref(total)) == 0
+    return free.value
+
+
+def test_a_request_that_must_wait_drops_no_kept_context(gb):
+    """A kept DG context (16 MB of matrix and more), a request in flight and one
+    that does not fit beside it: the kept context stays while that one waits."""
+    import time
+    from modfem_gb300.mesh import lognormal_k, prism_faces, structured_prism_mesh
+    from modfem_gb300.serve import DG, STD, Problem, Server
+    d, m = structured_prism_mesh(8), structured_prism_mesh(48)
+    kept = Problem(d, np.ones(d.nel), kind=DG, p=2, faces=prism_faces(d), krylov=10, max_iter=5)
+    large = Problem(m, lognormal_k(m.nel, seed=1), kind=STD, krylov=1, max_iter=15000, tol=1e-12)  # over a second
+    budget = max(int(1.5 * large.footprint()), 8 * kept.footprint())
+    assert 2 * large.footprint() > budget
+    srv = Server(0, hbm_budget=budget, prep_threads=1)
+    try:
+        rid = srv.submit(kept)
+        assert srv.wait(rid, 120.0) == 1
+        first = srv.submit(large)
+        end = time.time() + 60.0
+        while srv.stats()["active"] == 0 and time.time() < end:
+            time.sleep(1e-3)
+        time.sleep(0.2)  # its buffers are there
+        before = _free()
+        second = srv.submit(large)
+        time.sleep(0.2)
+        after, st = _free(), srv.stats()
+        assert srv.wait(first, 120.0) == 1 and srv.wait(second, 120.0) == 1
+    finally:
+        srv.close()
+    assert st["active"] == 1 and st["queued"] == 1
+    assert after - before <= 8 * 2**20
