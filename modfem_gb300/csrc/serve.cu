@@ -411,7 +411,13 @@ struct gbfem_server_s {
   long long idle_bytes = 0;
   // the others are freed by the reaper thread (a cudaFree on the engine
   // thread would hold every lane until all GPU work drained)
-  std::deque<std::pair<gbfem_ctx, double *>> reapq;
+  struct Reaped {
+    gbfem_ctx ctx;
+    double *kry;
+    long long bytes;
+  };
+  std::deque<Reaped> reapq;
+  long long reap_bytes = 0;  // held until the reaper has freed them
   std::condition_variable cv_reap;
   bool reap_stop = false;
   std::thread reaper;
@@ -441,21 +447,26 @@ constexpr int SRV_CAPTURE_POLLS = 16;  // polls of one set before its step is ca
 
 int idle_key(const SrvRequest &r) { return r.kind == 0 && r.solo_admit ? 2 : r.kind; }
 
-void drop_oldest_idle(gbfem_server s) {  // caller holds s->mu
-  gbfem_server_s::Idle &i = s->idle.front();
-  s->idle_bytes -= i.bytes;
-  s->reapq.emplace_back(i.ctx, i.kry.p);
-  s->idle.pop_front();
+void queue_reap(gbfem_server s, const gbfem_server_s::Idle &i) {  // caller holds s->mu
+  s->reapq.push_back({i.ctx, i.kry.p, i.bytes});
+  s->reap_bytes += i.bytes;
   s->cv_reap.notify_one();
+}
+
+void drop_oldest_idle(gbfem_server s) {  // caller holds s->mu
+  s->idle_bytes -= s->idle.front().bytes;
+  queue_reap(s, s->idle.front());
+  s->idle.pop_front();
 }
 
 // Whether `bytes` more fit in the HBM budget (idle contexts give way, but not
 // for a request that would have to wait all the same); a request larger than the
-// budget runs alone.
+// budget runs alone.  What the reaper has still to free counts: it admits again
+// afterwards.
 bool fits(gbfem_server s, long long bytes) {  // caller holds s->mu
   if (s->in_use > 0 && s->in_use + bytes > s->budget) return false;
   while (!s->idle.empty() && s->in_use + s->idle_bytes + bytes > s->budget) drop_oldest_idle(s);
-  return s->in_use + bytes <= s->budget || s->in_use == 0;
+  return s->in_use + s->reap_bytes + bytes <= s->budget || s->in_use + s->reap_bytes == 0;
 }
 
 // A finished request's context and Krylov space (no device work of it may be
@@ -471,8 +482,8 @@ void reap(gbfem_server s, SrvRequest &r, bool reusable = true) {
   r.kry = DevBuf<double>();  // ownership has passed
   if (!i.ctx && !i.kry.p) return;
   std::lock_guard<std::mutex> lk(s->mu);
+  i.bytes = gbfem_device_bytes(i.ctx) + (long long)i.kry.bytes();
   if (i.ctx && reusable && !s->stop) {
-    i.bytes = gbfem_device_bytes(i.ctx) + (long long)i.kry.bytes();
     int same = 0;
     for (const auto &o : s->idle) same += o.key == i.key;
     while (!s->idle.empty() && same >= SRV_IDLE) {
@@ -483,14 +494,13 @@ void reap(gbfem_server s, SrvRequest &r, bool reusable = true) {
       same--;
     }
     if (s->idle_bytes + i.bytes <= s->budget / 8 &&
-        s->in_use - r.charged + s->idle_bytes + i.bytes <= s->budget) {  // (its charge ends with it)
+        s->in_use - r.charged + s->reap_bytes + s->idle_bytes + i.bytes <= s->budget) {  // (its charge ends with it)
       s->idle_bytes += i.bytes;
       s->idle.push_back(i);
       return;
     }
   }
-  s->reapq.emplace_back(i.ctx, i.kry.p);
-  s->cv_reap.notify_one();
+  queue_reap(s, i);
 }
 
 // An idle context for the request, of its own mesh size if there is one (its
@@ -516,21 +526,6 @@ bool take_idle(gbfem_server s, SrvRequest &r) {
   s->peak_in_use = std::max(s->peak_in_use, s->in_use);
   s->idle.erase(best);
   return true;
-}
-
-void reaper_loop(gbfem_server s) {
-  cudaSetDevice(s->device);
-  std::unique_lock<std::mutex> lk(s->mu);
-  for (;;) {
-    s->cv_reap.wait(lk, [&] { return s->reap_stop || !s->reapq.empty(); });
-    if (s->reapq.empty()) return;  // stop, and nothing left
-    const auto item = s->reapq.front();
-    s->reapq.pop_front();
-    lk.unlock();
-    if (item.first) gbfem_destroy(item.first);
-    if (item.second) cudaFree(item.second);
-    lk.lock();
-  }
 }
 
 // A lane may hold half of max_active requests, or more while the other lane
@@ -580,6 +575,23 @@ void try_admit(gbfem_server s) {  // caller holds s->mu
       s->prepq.push_back(r);
       s->cv_prep.notify_one();
     }
+  }
+}
+
+void reaper_loop(gbfem_server s) {
+  cudaSetDevice(s->device);
+  std::unique_lock<std::mutex> lk(s->mu);
+  for (;;) {
+    s->cv_reap.wait(lk, [&] { return s->reap_stop || !s->reapq.empty(); });
+    if (s->reapq.empty()) return;  // stop, and nothing left
+    const auto item = s->reapq.front();
+    s->reapq.pop_front();
+    lk.unlock();
+    if (item.ctx) gbfem_destroy(item.ctx);
+    if (item.kry) cudaFree(item.kry);
+    lk.lock();
+    s->reap_bytes -= item.bytes;
+    try_admit(s);
   }
 }
 

@@ -124,3 +124,28 @@ def test_a_request_that_must_wait_drops_no_kept_context(gb):
         srv.close()
     assert st["active"] == 1 and st["queued"] == 1
     assert after - before <= 8 * 2**20
+
+
+def test_requests_that_need_the_kept_contexts_room_are_served(gb):
+    """Std and DG requests of nearly the whole budget in turn, small ones between
+    them: each large one waits until the contexts kept from the small ones have been
+    freed, is admitted then, and nothing stays charged."""
+    from modfem_gb300.mesh import prism_faces, structured_prism_mesh
+    from modfem_gb300.serve import DG, STD, Problem, Server
+    s, d = structured_prism_mesh(24), structured_prism_mesh(12)
+    large = [Problem(s, np.ones(s.nel), kind=STD, krylov=30, max_iter=20, tol=1e-10),
+             Problem(d, np.ones(d.nel), kind=DG, p=1, faces=prism_faces(d), krylov=30, max_iter=20, tol=1e-10)]
+    t = structured_prism_mesh(6)
+    small = [Problem(t, np.ones(t.nel), kind=STD, max_iter=20),
+             Problem(t, np.ones(t.nel), kind=DG, p=1, faces=prism_faces(t), max_iter=20)]
+    budget = max(p.footprint() for p in large) + min(p.footprint() for p in small)
+    srv = Server(0, hbm_budget=budget, prep_threads=2)
+    try:
+        for _ in range(5):
+            ids = [srv.submit(p) for p in small + large]
+            for rid in ids:
+                assert srv.wait(rid, 60.0) == 1
+        st = srv.stats()
+    finally:
+        srv.close()
+    assert st["bytes"] == 0 and st["queued"] == 0 and st["peak_bytes"] <= budget
