@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "dg_tables.h"
@@ -247,9 +248,11 @@ static void tet_tables(int p, std::vector<double> &T, std::vector<double> &MOM) 
 
 static DgBatchTables g_bt[64];
 static bool g_bt_ready[64];
+static std::mutex g_bt_lock;  // batches and contexts are made and used from several threads
 
 static int dg_batch_tables(int device, DgBatchTables *out) {
   GB_CHECK(device >= 0 && device < 64, "device index out of range");
+  std::lock_guard<std::mutex> hold(g_bt_lock);
   if (!g_bt_ready[device]) {
     DgDeviceTables *pt = nullptr;
     const int r = dg_tables_for_device(device, &pt);
