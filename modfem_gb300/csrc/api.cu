@@ -562,7 +562,8 @@ int gbfem_build_structure(gbfem_ctx c, int *ndof, long long *nnz, int *nr_colors
   GB_TRY(upload(c, c->col_ind, c->hs.col_ind.data(), c->hs.col_ind.size()));
   GB_TRY(upload(c, c->dof_of_node, c->hs.dof_of_node.data(), c->hs.dof_of_node.size()));
   GB_TRY(upload(c, c->el_table, c->hs.el_table.data(), c->hs.el_table.size()));
-  GB_TRY(upload(c, c->el_perm, c->hs.el_perm.data(), c->hs.el_perm.size()));
+  // (tetrahedra scatter without colours; theirs are counted for the caller only)
+  if (c->nv == GBFEM_PRISM) GB_TRY(upload(c, c->el_perm, c->hs.el_perm.data(), c->hs.el_perm.size()));
   GB_TRY(upload(c, c->fa_perm, c->hs.fa_perm.data(), c->hs.fa_perm.size()));
   c->h_el_color_ptr = c->hs.el_color_ptr;
   c->h_fa_color_ptr = c->hs.fa_color_ptr;
@@ -640,9 +641,8 @@ static int check_err_flag(gbfem_ctx c) {
   GB_CUDA(cudaStreamSynchronize(c->stream));
   if (h) {
     cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream);
-    set_error(h == 1   ? "integration entity list names an element outside the mesh"
-              : h == 9 ? "the element incidence does not match the element tables"
-                       : "integration entity list names a face that is not a boundary face of the mesh");
+    set_error(h == 1 ? "integration entity list names an element outside the mesh"
+                     : "integration entity list names a face that is not a boundary face of the mesh");
     return -3;
   }
   return 0;
@@ -1014,7 +1014,7 @@ int gbfem_create_assemble_stiff_mat(gbfem_ctx c, int Level_id, int Comp_type, co
       return gbfem::launch_prism_elements(est, true, c->aniso, b - a, fe_id + a, 1, fe_pos + a, c->nel,
                                           c->el_nodes.p, c->xyz.p, c->k_el.p, c->D_el.p, c->f, c->in_table.p,
                                           c->val.p, c->rhs.p, do_sm, do_rhs, c->err.p, c->std_dword);
-    return gbfem::launch_tet_elements(est, true, b - a, fe_id + a, 1, fe_pos + a, c->nel, c->el_nodes.p,
+    return gbfem::launch_tet_elements(est, b - a, fe_id + a, 1, fe_pos + a, c->nel, c->el_nodes.p,
                                       c->xyz.p, c->k_el.p, c->f, c->in_table.p, c->val.p, c->rhs.p, do_sm, do_rhs,
                                       c->err.p);
   };
@@ -1180,9 +1180,8 @@ int gbfem_assemble(gbfem_ctx c, int scatter_mode) {
                                        c->el_nodes.p, c->xyz.p, c->k_el.p, c->D_el.p, c->f, c->el_table.p,
                                        c->val.p, c->rhs.p, 1, 1, c->err.p, c->std_dword);
     else
-      r = gbfem::launch_tet_elements(c->stream, true, c->nel, nullptr, 0, nullptr, c->nel, c->el_nodes.p,
-                                     c->xyz.p, c->k_el.p, c->f, c->el_table.p, c->val.p, c->rhs.p, 1, 1,
-                                     c->err.p);
+      r = gbfem::launch_tet_elements(c->stream, c->nel, nullptr, 0, nullptr, c->nel, c->el_nodes.p, c->xyz.p,
+                                     c->k_el.p, c->f, c->el_table.p, c->val.p, c->rhs.p, 1, 1, c->err.p);
     GB_TRY(r);
     launches += r;
   } else if (gather) {
@@ -1195,14 +1194,9 @@ int gbfem_assemble(gbfem_ctx c, int scatter_mode) {
   } else {
     for (size_t k = 0; k + 1 < c->h_el_color_ptr.size(); k++) {
       const int lo = c->h_el_color_ptr[k], hi = c->h_el_color_ptr[k + 1];
-      if (c->nv == GBFEM_PRISM)
-        r = gbfem::launch_prism_elements(c->stream, false, c->aniso, hi - lo, c->el_perm.p + lo, 0, nullptr,
-                                         c->nel, c->el_nodes.p, c->xyz.p, c->k_el.p, c->D_el.p, c->f,
-                                         c->el_table.p, c->val.p, c->rhs.p, 1, 1, c->err.p, c->std_dword);
-      else
-        r = gbfem::launch_tet_elements(c->stream, false, hi - lo, c->el_perm.p + lo, 0, nullptr, c->nel,
-                                       c->el_nodes.p, c->xyz.p, c->k_el.p, c->f, c->el_table.p, c->val.p,
-                                       c->rhs.p, 1, 1, c->err.p);
+      r = gbfem::launch_prism_elements(c->stream, false, c->aniso, hi - lo, c->el_perm.p + lo, 0, nullptr,
+                                       c->nel, c->el_nodes.p, c->xyz.p, c->k_el.p, c->D_el.p, c->f,
+                                       c->el_table.p, c->val.p, c->rhs.p, 1, 1, c->err.p, c->std_dword);
       GB_TRY(r);
       launches += r;
     }

@@ -147,7 +147,7 @@ int launch_prism_constrained(cudaStream_t st, bool faces, bool aniso, int count,
                              const double *k_el, const double *D_el, double f, double penalty, double g,
                              const int *con_node, const int *con_par, const int *tab, double *val, double *rhs,
                              int do_sm, int do_rhs, int *err);
-int launch_tet_elements(cudaStream_t st, bool atomic, int count, const int *ent_el, int el_base,
+int launch_tet_elements(cudaStream_t st, int count, const int *ent_el, int el_base,
                         const int *ent_pos, int nel, const int *el_nodes, const double *xyz,
                         const double *k_el, double f, const int *tab, double *val, double *rhs,
                         int do_sm, int do_rhs, int *err);

@@ -296,12 +296,11 @@ __global__ void __launch_bounds__(GM_T) gm_restart_residual(GmArgs a) {
   if (valid && lane == 0) a.tmp[r] = (a.b[r] - s) * a.dinv[r];
 }
 
-// partial[b] = sum over block b's entries of v^2 (v = tmp, or V[j+1])
-template <int WHICH>
-__global__ void __launch_bounds__(GM_T) gm_norm_partial(GmArgs a, int j) {
+// partial[b] = sum over block b's entries of tmp^2
+__global__ void __launch_bounds__(GM_T) gm_norm_partial(GmArgs a) {
   const GmState &S = *a.st;
-  if (WHICH == 0 ? (S.phase != GM_RESTART || S.final_flag) : (S.phase != GM_ARNOLDI || S.j != j)) return;
-  const double *v = WHICH == 0 ? a.tmp : a.V + (size_t)(j + 1) * a.n;
+  if (S.phase != GM_RESTART || S.final_flag) return;
+  const double *v = a.tmp;
   double s = 0.0;
   for (long long i = (long long)blockIdx.x * GM_T + threadIdx.x; i < a.n; i += (long long)gridDim.x * GM_T)
     s = fma(v[i], v[i], s);
@@ -660,7 +659,7 @@ int capture_cycle(gbfem_ctx c, const GmArgs &a, int m, bool dword, int *kernels)
   cudaGraph_t graph = nullptr;
   GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   gbfem::gm_restart_residual<<<a.sell_val64 ? gs : gcrs, gbfem::GM_T, 0, st>>>(a);
-  gbfem::gm_norm_partial<0><<<gv, gbfem::GM_T, 0, st>>>(a, 0);
+  gbfem::gm_norm_partial<<<gv, gbfem::GM_T, 0, st>>>(a);
   gbfem::gm_logic_restart<<<1, gbfem::GM_T, 0, st>>>(a);
   gbfem::gm_start_cycle<<<gv, gbfem::GM_T, 0, st>>>(a);
   k += 4;

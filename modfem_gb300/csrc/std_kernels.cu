@@ -437,7 +437,6 @@ __device__ __forceinline__ void tet_local(int e, const int *__restrict__ el_node
   }
 }
 
-template <bool ATOMIC>
 __global__ void __launch_bounds__(128) tet_elements_kernel(
     int count, const int *__restrict__ ent_el, int el_base, const int *__restrict__ ent_pos, int nel,
     const int *__restrict__ el_nodes, const double *__restrict__ xyz, const double *__restrict__ k_el,
@@ -459,13 +458,13 @@ __global__ void __launch_bounds__(128) tet_elements_kernel(
     for (int u = 0; u < 4; u++)
 #pragma unroll
       for (int w = u; w < 4; w++, k++) {
-        add_val<ATOMIC>(val, __ldg(tb + w + 4 * u), K[k]);
-        if (w != u) add_val<ATOMIC>(val, __ldg(tb + u + 4 * w), K[k]);
+        add_val<true>(val, __ldg(tb + w + 4 * u), K[k]);
+        if (w != u) add_val<true>(val, __ldg(tb + u + 4 * w), K[k]);
       }
   }
   if (do_rhs) {
 #pragma unroll
-    for (int w = 0; w < 4; w++) add_val<ATOMIC>(rhs, __ldg(tb + 16 + w), R[w]);
+    for (int w = 0; w < 4; w++) add_val<true>(rhs, __ldg(tb + 16 + w), R[w]);
   }
 }
 
@@ -864,18 +863,14 @@ int launch_prism_constrained(cudaStream_t st, bool faces, bool aniso, int count,
   return 1;
 }
 
-int launch_tet_elements(cudaStream_t st, bool atomic, int count, const int *ent_el, int el_base,
+int launch_tet_elements(cudaStream_t st, int count, const int *ent_el, int el_base,
                         const int *ent_pos, int nel, const int *el_nodes, const double *xyz,
                         const double *k_el, double f, const int *tab, double *val, double *rhs,
                         int do_sm, int do_rhs, int *err) {
   if (count <= 0) return 0;
   const int T = 128;
-  if (atomic)
-    tet_elements_kernel<true><<<nblk(count, T), T, 0, st>>>(count, ent_el, el_base, ent_pos, nel, el_nodes,
-                                                            xyz, k_el, f, tab, val, rhs, do_sm, do_rhs, err);
-  else
-    tet_elements_kernel<false><<<nblk(count, T), T, 0, st>>>(count, ent_el, el_base, ent_pos, nel, el_nodes,
-                                                             xyz, k_el, f, tab, val, rhs, do_sm, do_rhs, err);
+  tet_elements_kernel<<<nblk(count, T), T, 0, st>>>(count, ent_el, el_base, ent_pos, nel, el_nodes, xyz, k_el, f,
+                                                    tab, val, rhs, do_sm, do_rhs, err);
   GB_CUDA(cudaGetLastError());
   return 1;
 }
