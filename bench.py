@@ -414,26 +414,15 @@ def bench_dg(gb, local, steps, fp64_peak, gmres_iters=100):
         vta, _ = c.dg_get_matrix()
         ta_dev = float(np.max(np.abs(vta - v64)) / np.max(np.abs(v64)))
         del vta
-        # double-word sums on the FP32 pipes for volume and faces (all
-        # degrees), and the tensor cores where they apply with double words
-        # for the rest
-        dwf = {}
-        for key, vmode, fmode in (("double_word_assembly", gb.DG_VOLUME_DWORD, gb.DG_FACE_DWORD),
-                                  ("fastest_assembly", gb.DG_VOLUME_DWORD, gb.DG_FACE_TC_DWORD)):
+        # the double-word modes run the FP64 kernels on a mesh without turned
+        # quadrilaterals: the same matrix
+        same_bits = {}
+        for key, vmode, fmode in (("DG_VOLUME_DWORD, DG_FACE_DWORD", gb.DG_VOLUME_DWORD, gb.DG_FACE_DWORD),
+                                  ("DG_VOLUME_DWORD, DG_FACE_TC_DWORD", gb.DG_VOLUME_DWORD, gb.DG_FACE_TC_DWORD)):
             c.dg_set_volume_kernel(vmode)
             c.dg_set_face_kernel(fmode)
             c.dg_assemble()
-            tt = np.zeros(3)
-            for _ in range(steps):
-                c.dg_assemble()
-                tt += np.array(c.dg_last_timing()[:3])
-            tot_tw, vol_tw, fa_tw = tt / steps
-            vtw, _ = c.dg_get_matrix()
-            dwf[key] = {"volume_ms": vol_tw, "face_ms": fa_tw, "assemble_ms": tot_tw,
-                        "elem_per_s": m.nel / (tot_tw * 1e-3), "speedup_vs_fp64": tot / tot_tw,
-                        "face_speedup_vs_fp64": fa / fa_tw,
-                        "max_abs_diff_vs_fp64_rel_to_max": float(np.max(np.abs(vtw - v64)) / np.max(np.abs(v64)))}
-            del vtw
+            same_bits[key] = bool(np.array_equal(c.dg_get_matrix()[0], v64))
         del v64
         c.dg_set_face_kernel(gb.DG_FACE_FP64)
         c.dg_set_volume_kernel(gb.DG_VOLUME_FP64)
@@ -469,14 +458,7 @@ def bench_dg(gb, local, steps, fp64_peak, gmres_iters=100):
                                      "max_abs_diff_vs_fp64_rel_to_max": ta_dev,
                                      "note": "tcgen05 split-BF16 volume and faces (owners and neighbours p <= 3; "
                                              "others stay FP64)"},
-            "double_word_assembly": dict(
-                dwf["double_word_assembly"],
-                note="the double-word modes: prism volume and faces from FP64 moments (faster than double-word "
-                     "sums over the points), as the FP64 assembly; double words elsewhere"),
-            "fastest_assembly": dict(
-                dwf["fastest_assembly"],
-                note="the fastest modes (DG_VOLUME_DWORD, DG_FACE_TC_DWORD): FP64 moments wherever the faces have "
-                     "the regular orientation, as the FP64 assembly"),
+            "modes_with_the_same_bits": same_bits,
             "tf32_volume": {"volume_ms": vol_tf, "assemble_ms": tot_tf, "elem_per_s": m.nel / (tot_tf * 1e-3),
                             "max_abs_diff_vs_fp64_rel_to_max": tf_dev,
                             "note": "tcgen05 kind::tf32, hi/lo operands, FP32 accumulation (p <= 3)"},
@@ -533,14 +515,11 @@ def bench_batch(gb, local, steps, fp64_peak):
     ms = [b.run() for _ in range(steps)]
     step_ms = float(np.mean(ms))
     v64, _ = b.get()
-    # the same launch with the prism stiffness sums in double-word arithmetic
+    # (the double-word choice runs the same kernel)
     b.set_arith(True)
-    for _ in range(2):
-        b.run()
-    dw_ms = float(np.mean([b.run() for _ in range(steps)]))
-    vdw, _ = b.get()
-    dw_dev = float(np.max(np.abs(vdw - v64)) / np.max(np.abs(v64)))
-    del v64, vdw
+    b.run()
+    dw_same = bool(np.array_equal(b.get()[0], v64))
+    del v64
     b.set_arith(False)
     pfma = sum(dg_fma_per_element(q) * int(np.sum(pp == q)) for q in range(1, 5))
     tfma = sum(tet_fma_per_element(q) * int(np.sum(tp == q)) for q in range(1, 5))
@@ -600,9 +579,7 @@ def bench_batch(gb, local, steps, fp64_peak):
         "output_gbs": out_bytes / (step_ms * 1e-3) / 1e9,
         "tets_alone_ms": tet_ms, "tets_alone_output_gbs": 8 * (tnv + tnr) / (tet_ms * 1e-3) / 1e9,
         "prisms_per_degree_kernels_ms": per_degree_ms,
-        "double_word_prisms": {"step_ms": dw_ms, "elem_per_s": (NP + NT) / (dw_ms * 1e-3),
-                               "speedup_vs_fp64": step_ms / dw_ms, "max_abs_diff_vs_fp64_rel_to_max": dw_dev,
-                               "note": "prisms from FP64 moments in either arithmetic, tetrahedra FP64"},
+        "double_word_arithmetic_same_bits": dw_same,  # (one FP64 kernel serves both choices)
         "e2e_ms": e2e_s * 1e3, "e2e_elem_per_s": (NP + NT) / e2e_s,
         "e2e_note": "page-locked host arrays: upload of geometry and tensors, tile build, graph capture, run, "
                     "download of "
@@ -633,26 +610,10 @@ def bench_tet_dg(gb, local, steps):
         c.dg_assemble()
         tt += np.array(c.dg_last_timing()[:3])
     tot, vol, fa = tt / steps
-    v64, _ = c.dg_get_matrix()
-    # the double-word face mode (tetrahedra: the same FP64 kernel)
-    c.dg_set_face_kernel(gb.DG_FACE_DWORD)
-    c.dg_assemble()
-    tt = np.zeros(3)
-    for _ in range(steps):
-        c.dg_assemble()
-        tt += np.array(c.dg_last_timing()[:3])
-    tot_dw, _, fa_dw = tt / steps
-    vdw, _ = c.dg_get_matrix()
-    dw_dev = float(np.max(np.abs(vdw - v64)) / np.max(np.abs(v64)))
-    del v64, vdw
-    c.dg_set_face_kernel(gb.DG_FACE_FP64)
-    c.dg_assemble()
     x, it, res, rel = c.dg_solve(krylov=50, max_iter=100, tol_rel=1e-10)
     st = c.last_solve_timing()
     out = {"elements": t.nel, "faces": int(F.n), "dofs": nd, "stored_values": nv,
            "assemble_ms": tot, "volume_ms": vol, "face_ms": fa, "elem_per_s": t.nel / (tot * 1e-3),
-           "double_word_faces": {"face_ms": fa_dw, "assemble_ms": tot_dw, "face_speedup_vs_fp64": fa / fa_dw,
-                                 "max_abs_diff_vs_fp64_rel_to_max": dw_dev},
            "gmres_iterations": it, "gmres_ms_per_iteration": st[0] / max(it, 1),
            "spmv_ms": st[1] / max(st[2], 1)}
     c.close()
@@ -665,10 +626,8 @@ def bench_mixed_dg_system(gb, local, steps, n=63, layers=50):
     upper 13 into 6 tetrahedra each (309,582 affine tetrahedra), the two
     regions joined by 7,938 prism-tetrahedron triangles; p uniform in 1..4
     (seeded), lognormal(0,1) k, interior-penalty faces into the
-    variable-block storage.  Assembly (volume and all faces) in plain FP64
-    and in the modes DG_VOLUME_DWORD, DG_FACE_TC_DWORD (the same kernels on this
-    mesh), then a fixed 100 GMRES(50) iterations with block
-    Jacobi."""
+    variable-block storage.  Assembly (volume and all faces) in plain FP64,
+    then a fixed 100 GMRES(50) iterations with block Jacobi."""
     from modfem_gb300.mesh import lognormal_k, mixed_faces, structured_mixed_mesh
     m = structured_mixed_mesh(n, layers, jitter=0.2, seed=SEED)
     F = mixed_faces(m)
@@ -682,35 +641,16 @@ def bench_mixed_dg_system(gb, local, steps, n=63, layers=50):
     out = {"prisms": int((m.el_nv == 6).sum()), "tetrahedra": int((m.el_nv == 4).sum()), "faces": int(F.n),
            "prism_tetrahedron_faces": int(((F.el2 >= 0) & (m.el_nv[F.el1] != m.el_nv[np.maximum(F.el2, 0)])).sum()),
            "dofs": nd, "stored_values": nv}
-    v64 = None
-    for key, vol, face in (("fp64", gb.DG_VOLUME_FP64, gb.DG_FACE_FP64),
-                           ("fastest", gb.DG_VOLUME_DWORD, gb.DG_FACE_TC_DWORD)):
-        c.dg_set_volume_kernel(vol)
-        c.dg_set_face_kernel(face)
-        for _ in range(2):
-            c.dg_assemble()
-        tt = np.zeros(3)
-        launches = 0
-        for _ in range(steps):
-            c.dg_assemble()
-            t = c.dg_last_timing()
-            tt += np.array(t[:3])
-            launches = t[3]
-        tot, vol_ms, fa = tt / steps
-        r = {"assemble_ms": tot, "volume_ms": vol_ms, "face_ms": fa, "elem_per_s": m.nel / (tot * 1e-3),
-             "launches": launches}
-        vals, _ = c.dg_get_matrix()
-        if v64 is None:
-            v64 = vals
-        else:
-            r["max_abs_diff_vs_fp64_rel_to_max"] = float(np.max(np.abs(vals - v64)) / np.max(np.abs(v64)))
-            r["speedup_vs_fp64"] = out["fp64"]["assemble_ms"] / tot
-        del vals
-        out[key] = r
-    del v64
-    c.dg_set_volume_kernel(gb.DG_VOLUME_FP64)
-    c.dg_set_face_kernel(gb.DG_FACE_FP64)
-    c.dg_assemble()
+    for _ in range(2):
+        c.dg_assemble()
+    tt = np.zeros(3)
+    for _ in range(steps):
+        c.dg_assemble()
+        t = c.dg_last_timing()
+        tt += np.array(t[:3])
+    tot, vol_ms, fa = tt / steps
+    out["fp64"] = {"assemble_ms": tot, "volume_ms": vol_ms, "face_ms": fa, "elem_per_s": m.nel / (tot * 1e-3),
+                   "launches": t[3]}
     x, it, res, rel = c.dg_solve(krylov=50, max_iter=100, tol_rel=1e-10)
     st = c.last_solve_timing()
     out.update({"elements": m.nel, "gmres_iterations": it, "gmres_ms_per_iteration": st[0] / max(it, 1),
@@ -722,8 +662,8 @@ def bench_mixed_dg_system(gb, local, steps, n=63, layers=50):
 def mixed_precision_solution_check(gb, local, sizes=(10, 16)):
     """Config-4 form at sizes GMRES(50) converges on in a bench run: p = 3
     prisms, the anisotropic tensor, Dirichlet value 0.3.  Every assembly
-    (plain FP64; split-BF16 tensor-core volume and faces; double-word volume
-    with tensor-core faces; double-word volume and faces) is solved by FP64
+    (plain FP64; split-BF16 tensor-core volume and faces; FP64 volume with
+    tensor-core faces) is solved by FP64
     iterative refinement around FP32-operator GMRES(50) with compensated
     residuals until the corrections reach FP64 rounding, so each solution is
     its matrix's to ~1e-15 and the differences are the matrices' effect on
@@ -732,8 +672,7 @@ def mixed_precision_solution_check(gb, local, sizes=(10, 16)):
     GMRES (stopped at 1e-12 preconditioned) against the same."""
     from modfem_gb300.mesh import anisotropic_tensors, prism_faces, structured_prism_mesh
     forms = {"fp64": (gb.DG_VOLUME_FP64, gb.DG_FACE_FP64), "tc_volume_tc_faces": (gb.DG_VOLUME_TC, gb.DG_FACE_TC),
-             "dword_volume_tc_faces": (gb.DG_VOLUME_DWORD, gb.DG_FACE_TC),
-             "dword_volume_dword_faces": (gb.DG_VOLUME_DWORD, gb.DG_FACE_DWORD)}
+             "fp64_volume_tc_faces": (gb.DG_VOLUME_FP64, gb.DG_FACE_TC)}
     out, summary = {}, {}
     for n in sizes:
         m = structured_prism_mesh(n, jitter=0.2, seed=44)
@@ -927,11 +866,10 @@ def compact_line(full):
         out[key] = {"fp64_assemble_ms": _r(d["assemble_ms"]),
                     "volume_point_sum_rate_over_fp64_peak": _r(d["volume_point_sum_rate_over_fp64_peak"], 3),
                     "face_point_sum_rate_over_fp64_peak": _r(d["face_point_sum_rate_over_fp64_peak"], 3)}
-        for form in ("tensor_core_assembly", "double_word_assembly", "fastest_assembly"):
-            f = d[form]
-            out[key][form] = {"assemble_ms": _r(f["assemble_ms"]), "face_ms": _r(f["face_ms"]),
-                              "speedup_vs_fp64": _r(f["speedup_vs_fp64"], 3),
-                              "max_dev_rel_to_max": _r(f["max_abs_diff_vs_fp64_rel_to_max"], 2)}
+        f = d["tensor_core_assembly"]
+        out[key]["tensor_core_assembly"] = {"assemble_ms": _r(f["assemble_ms"]), "face_ms": _r(f["face_ms"]),
+                                            "speedup_vs_fp64": _r(f["speedup_vs_fp64"], 3),
+                                            "max_dev_rel_to_max": _r(f["max_abs_diff_vs_fp64_rel_to_max"], 2)}
         out[key]["spmv_hbm_frac_of_measured"] = _r(d.get("spmv_hbm_frac_of_measured"), 3)
         out[key]["gmres_ms_per_iteration"] = _r(d["gmres_ms_per_iteration"])
     mps = dg.get("mixed_precision_solution")
@@ -939,25 +877,21 @@ def compact_line(full):
         out["mixed_precision_solution"] = mps.get("summary", mps)
     b = full["batch_mixed"]
     out["batch_mixed"] = {"step_ms": _r(b["step_ms"]), "elem_per_s": _r(b["elem_per_s"]),
-                          "point_sum_rate_over_fp64_peak": _r(b["point_sum_rate_over_fp64_peak"], 3),
-                          "double_word_step_ms": _r(b["double_word_prisms"]["step_ms"])}
+                          "point_sum_rate_over_fp64_peak": _r(b["point_sum_rate_over_fp64_peak"], 3)}
     # the mixed prism + tetrahedron workload as a whole step: the mixed-degree prism DG system and
     # the tetrahedral DG system (volume and faces each, measured above in this
     # run; the two element types form separate systems, no prism-tetrahedron
     # faces)
     mx, tet = dg.get("mixed_p1to4_390k"), b.get("tet_dg_system")
     if mx and tet:
-        out["batch_mixed"]["config3_whole_step_ms"] = {
-            "fp64": _r(mx["assemble_ms"] + tet["assemble_ms"]),
-            "double_word": _r(mx["double_word_assembly"]["assemble_ms"] + tet["double_word_faces"]["assemble_ms"]),
-            "elements": mx["elements"] + tet["elements"]}
+        out["batch_mixed"]["config3_whole_step_ms"] = {"fp64": _r(mx["assemble_ms"] + tet["assemble_ms"]),
+                                                       "elements": mx["elements"] + tet["elements"]}
     # the same workload as one system on one connected prism + tetrahedron mesh
     ms = b.get("mixed_dg_system")
     if ms:
         out["batch_mixed"]["config3_one_system"] = {
             "elements": ms["elements"], "prism_tetrahedron_faces": ms["prism_tetrahedron_faces"],
-            "fp64_assemble_ms": _r(ms["fp64"]["assemble_ms"]), "fastest_assemble_ms": _r(ms["fastest"]["assemble_ms"]),
-            "fastest_max_dev_rel_to_max": _r(ms["fastest"]["max_abs_diff_vs_fp64_rel_to_max"], 2),
+            "fp64_assemble_ms": _r(ms["fp64"]["assemble_ms"]),
             "gmres_ms_per_iteration": _r(ms["gmres_ms_per_iteration"])}
     sv = full.get("serving")
     if sv:
