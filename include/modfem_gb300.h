@@ -39,7 +39,9 @@ typedef struct gbfem_ctx_s *gbfem_ctx;
 #define GBFEM_TETRA 4
 /* scatter modes of gbfem_assemble */
 #define GBFEM_SCATTER_ATOMIC 0 /* one launch, FP64 atomics (summation order varies) */
-#define GBFEM_SCATTER_COLOR 1  /* one launch per colour, plain adds (deterministic); tetrahedra: as GATHER */
+#define GBFEM_SCATTER_COLOR 1  /* one launch per colour, plain adds (deterministic); tetrahedra: local
+                                  matrices stored and summed a row, as GATHER does for prisms, which
+                                  takes 180 B of device memory an element beside the structure */
 #define GBFEM_SCATTER_GATHER 2 /* local matrices stored, then a group of lanes a row sums them over
                                   the incident elements in element order (deterministic, no
                                   colouring; std prisms, FP64 element arithmetic) */
@@ -506,7 +508,7 @@ int gbfem_batch_get(gbfem_batch batch, double *vals, double *rhs);
  * preconditioned residual relative to the initial one.  The contexts of
  * finished requests are kept for later ones of the same kind (up to 8 each, an
  * eighth of the budget in all) and given back when the budget needs them or
- * with the server. */
+ * with the server; a request that takes one is charged for what it holds. */
 #define GBFEM_SERVE_STD 0
 #define GBFEM_SERVE_DG 1
 typedef struct gbfem_server_s *gbfem_server;

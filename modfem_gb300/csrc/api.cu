@@ -762,7 +762,7 @@ static int build_pipe_plan(gbfem_ctx c, int e0, int e1) {
   // starts a wave after the first coordinates and does not stop.  The FP64
   // kernels take twice the download's time: their last chunks shrink to one wave,
   // which is what is left to download after the last element.  (2M prisms, double word
-  // 1,274 us with even chunks, 1,238 us so; FP64 2,080 and 2,008 us)
+  // 1,294 us with eight even chunks, 1,238 us so; FP64 2,080 and 2,008 us)
   int nsm = 152;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
   const long long wave = (long long)nsm * (c->std_dword ? 3 : 5) * 128, waves = (count + wave - 1) / wave;
@@ -1609,7 +1609,12 @@ int gbfem_dg_get_structure(gbfem_ctx c, int *dof_off, int *bptr, int *bcol, long
   return (int)c->dg_bcol.size();
 }
 
-// Point fields of every face of the moment form; returns the launches.
+// Elements up to which the DG face kernels from moments run beside the volume
+// kernels.  What that saves is the kernels' starts and tails, 30 to 200 us at any size (one
+// after the other / beside, us: degree 1, 2,000 prisms 93 / 63, 16,000 287 / 245,
+// 43,904 696 / 634; degree 4, 2,000 1,011 / 918, 16,000 7,096 / 6,969, 27,648 12,148 / 12,023), so
+// the line lies where it falls below a few percent of most meshes; beyond it the
+// volume and face times of gbfem_dg_last_timing are each kernel's own.
 constexpr int DG_BESIDE_MAX = 16384;
 int gbfem_dg_assemble(gbfem_ctx c) {
   GB_CHECK(c && c->dg_ready, "DG structure not built (gbfem_dg_build_structure)");
@@ -1668,10 +1673,7 @@ int gbfem_dg_assemble(gbfem_ctx c) {
   }
   // Prism faces from moments, few elements: the point fields and the
   // off-diagonal blocks read nothing that the volume and tetrahedron kernels
-  // write, and none of these fills the chip: they run beside on the side
-  // stream (assembly and download: 2,000 prisms of p = 2 320 -> 299 us, 8,000 of
-  // p = 1..4 4.22 -> 4.05 ms, prisms and tetrahedra 4.10 -> 3.99 ms; 54,000 of p =
-  // 3: 8 ms either way, so there each kernel keeps its own time).
+  // write: they run beside on the side stream.
   const bool beside = mom && c->dg_hf.p && c->nel <= DG_BESIDE_MAX;
   auto fields = [&](cudaStream_t st) -> int {
     return gbfem::launch_dg_face_fields(st, c->dg_fb_start, c->dg_frec.p, c->el_nodes.p, c->xyz.p, c->k_el.p, c->D_el.p,

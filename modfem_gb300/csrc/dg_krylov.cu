@@ -28,9 +28,9 @@ namespace gbfem {
 // inverse[k][r_j] = entry (r_k, j).  The pivot column (f) and row (p) pass
 // through shared memory and leave zeros behind; with g_i = f_i / pivot,
 // g_r = -1 / pivot and p_k = 1 the whole step is entry (i, j) -= g_i p_j.  n^3 FMA
-// a block bound it by the FP64 pipe (p = 3: 2,000 of 2,500 FP64 warp
-// instructions, 54,000 blocks 6.9 ms); held in shared memory, three loads and a store an
-// FMA, the pipe stood half idle: 13.8 ms, 6.7 ms so.  (21,296 prisms of p = 1..4
+// a block bound it by the FP64 pipe (p = 3: 2,000 of some 2,330 FP64 warp
+// instructions, which hold it for 6.4 ms of 54,000 blocks' 6.7); held in shared memory, three
+// loads and a store an FMA, the pipe stood half idle: 13.8 ms.  (21,296 prisms of p = 1..4
 // 52, 504, 2,695, 19,765 us, 20,250 tetrahedra 33, 106, 530, 2,042 us; one CTA a
 // block in shared memory 581, 1,886, 6,317, 25,931 and 384, 919, 2,030, 4,798 us.)
 template <int P>

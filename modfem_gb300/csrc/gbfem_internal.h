@@ -201,8 +201,9 @@ struct DgFaceRec {
 // Whether the moment form covers the face: the edge direction of a
 // quadrilateral is the same in both neighbours, a triangle is a bottom or top
 bool dg_face_moments_cover(const DgFaceRec &r);
-// Point fields of `count` faces of one rule (degree pm, ti 0 triangles, 1
-// quadrilaterals): 7 x nq doubles a face at geo + rec.geo
+// Point fields of every face, 7 x nq doubles a face at geo + rec.geo, all rules in
+// one launch: records start[b] .. start[b + 1] are those of bucket b (degree
+// b % 4 + 1, triangles b < 4, quadrilaterals after them)
 int launch_dg_face_fields(cudaStream_t st, const int *start, const DgFaceRec *rec, const int *el_nodes,
                           const double *xyz, const double *k_el, const double *D_el, double pen, double *geo);
 // Diagonal shares and boundary loads of the owners of degree p; hrec[h] = 2

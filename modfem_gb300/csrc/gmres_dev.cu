@@ -12,9 +12,10 @@
 // Arnoldi steps, update of x) reads a state word and returns at once when the
 // cycle has already ended.  An Arnoldi step is the SpMV, the Gram-Schmidt dot
 // products and the orthogonalisation; small systems, where the step is a chain
-// of latencies, form the dots in the SpMV kernel.  No kernel has a serial
-// tail: the block partials of the dots are summed at the start of the
-// orthogonalisation (by every block, in the same order), and the step's logic
+// of latencies, form the dots in the SpMV kernel, and the block partials of the
+// dots are summed at the start of the orthogonalisation (by every block, in the
+// same order); in larger ones a kernel of one block sums them (gm_column, 8 us
+// a step: 760 blocks reading the same lines took 9 us more).  The step's logic
 // (norm, rotations, test, at the end of a cycle the triangular solve) runs in
 // one extra block of the next step's SpMV, which therefore starts before the
 // test of the step before it is known; a step that turns out not to be wanted
@@ -580,9 +581,10 @@ namespace {
 unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 // Up to here (slices of 32 rows; 38,912 rows) the dots run in the SpMV kernel:
-// below, an Arnoldi step is launches and memory latency (9,261 rows: 14 us a step
-// in two kernels; the three kernels with last-block tails before took 28).
-// 1,030,301 rows: 118 us a step on average over 30 (180 before).
+// its CTAs of four slices are then at most two an SM, all resident, and an Arnoldi
+// step is launches and memory latency.  60 steps of GMRES(30), two kernels a step
+// against four: 9,261 rows 938 / 1,653 us, 35,937 1,354 / 1,747, 39,304 1,796 / 1,873,
+// 50,653 2,103 / 1,871, 85,184 4,078 / 2,147.  1,030,301 rows: 118 us a step on average over 30.
 constexpr int GM_SMALL = 1216, GM_SMALL_WARPS = 4;
 
 // SELL-32 index arrays of the context's structure (once per structure)

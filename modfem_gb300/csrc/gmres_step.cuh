@@ -62,8 +62,8 @@ __device__ __forceinline__ void gm_sum_dots(const double *partial, int rows, int
 
 // sum_k c[k] V_k[i], U vectors' loads in flight, two accumulators (an FP64 FMA
 // waits long for the one before it).  An incomplete group's FMAs are predicated:
-// in the small systems that take U = 32 (9,261 rows, a step 17.6 us) a branch
-// around every four of them costs 0.7 us a step more than it saves.
+// in the small systems that take U = 32 a branch around every four of them costs
+// more than it saves (9,261 rows: 0.7 us a step).
 template <int U>
 __device__ __forceinline__ double gm_combine(const double *V, long long n, const double *c, int nk, long long i) {
   double a0 = 0.0, a1 = 0.0;
