@@ -299,6 +299,12 @@ __device__ __forceinline__ double flip(double v, int neg) {  // the sign on the 
   return __longlong_as_double(__double_as_longlong(v) ^ ((long long)(neg & 1) << 63));
 }
 
+// (NaN or infinity, on the integer side.)  Where a derivative of a function is
+// identically zero its moment is left out, and a field that is not finite, as a
+// coefficient that is not makes it, would leave no trace in the entry; the sums over the
+// points multiply it by zero, which is NaN.  So it is looked for.
+__device__ __forceinline__ int fm_nonfinite(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
+
 // How a quadrilateral lies in one of its elements: triangle vertices A, B of
 // its edge (x_A = 1 - s, x_B = s), whether zeta runs against the rule.
 struct FmQuad {
@@ -361,6 +367,7 @@ __global__ void __launch_bounds__(THR) dg_face_diag_kernel(
     for (; t < 2; t++) sTri[t] = -1;
   }
   // fields of the owner's side with its sign
+  int bad = 0;  // of a Dirichlet face
   for (int f = 0; f < nf; f++) {
     const DgFaceRec &R = sR[f];
     const int pm = R.el2 >= 0 && R.p2 > R.p1 ? R.p2 : R.p1;
@@ -371,9 +378,10 @@ __global__ void __launch_bounds__(THR) dg_face_diag_kernel(
       const int c = t / nq, q = t - c * nq;
       const double v = g[(size_t)(c == 0 ? 0 : c + 3 * o) * nq + q];
       sF[f][t] = c == 0 ? v : flip(v, o);
+      bad |= R.el2 < 0 && fm_nonfinite(v);
     }
   }
-  __syncthreads();
+  bad = __syncthreads_or(bad);
   for (int t = tid; t < 3 * NZ; t += THR) {
     const int qi = t / NZ, f = sQuad[qi];
     if (f < 0) break;  // (the quadrilaterals come first)
@@ -488,7 +496,7 @@ __global__ void __launch_bounds__(THR) dg_face_diag_kernel(
     }
     if (any) {
       double *r = rhs + roff[e] + i;
-      *r = fma(gval, s, *r);
+      *r = bad ? nan("") : fma(gval, s, *r);
     }
   }
   __syncthreads();
@@ -550,15 +558,19 @@ __global__ void __launch_bounds__(FmOff<PM, QUAD>::THR) dg_face_blocks_kernel(
     sFn[sd][u][0] = (unsigned char)fm_mono(x[0], x[1]);
     sFn[sd][u][1] = x[2];
   }
-  for (int t = tid; t < D::F; t += THR) sF[t] = geo[R.geo + t];
+  int bad = 0;
+  for (int t = tid; t < D::F; t += THR) {
+    const double v = geo[R.geo + t];
+    sF[t] = v;
+    if (QUAD) bad |= fm_nonfinite(v);
+  }
   const int neg1 = QUAD ? R.loc1[0] >= 3 : R.loc1[0] < 3, neg2 = QUAD ? R.loc2[0] >= 3 : R.loc2[0] < 3;
-  // QUAD: row offsets of the moments in sW (the last K doubles stay zero)
+  // QUAD: row offsets of the moments in sW (the last K doubles: no moment, zero)
   const int TD = fm_tri(DD), TD1 = fm_tri(DD - 1);
   const int o1 = TD * K, o2 = o1 + TD1 * K, o4 = o2 + TD1 * K, o5 = o4 + TD1 * K, o3 = o5 + TD1 * K, o6 = o3 + TD * (K - 1),
             oz = o6 + TD * (K - 1);
   if (QUAD) {
     const FmQuad A(R.loc1), B(R.loc2);
-    for (int t = tid; t < K; t += THR) sW[oz + t] = 0.0;
     // per pair of triangle monomials: the moment rows of its five products
     for (int t = tid; t < npair; t += THR) {
       const int x = t / nt2, y = t - x * nt2;
@@ -573,7 +585,8 @@ __global__ void __launch_bounds__(FmOff<PM, QUAD>::THR) dg_face_blocks_kernel(
       I[3] = (unsigned short)(a2 && v1 && B.trace(a2 - 1, b2, gA, gB) ? o4 + fm_mono(eA + gA, eB + gB) * K : oz);
       I[4] = (unsigned short)(b2 && v1 && B.trace(a2, b2 - 1, gA, gB) ? o5 + fm_mono(eA + gA, eB + gB) * K : oz);
     }
-    __syncthreads();
+    bad = __syncthreads_or(bad);
+    for (int t = tid; t < K; t += THR) sW[oz + t] = bad ? nan("") : 0.0;
     // line sums S[c][k][m]
     constexpr int ZS = Q1 | 1;
     const double *Z = tb.Z + (size_t)(PM - 1) * FM_Q1 * FM_ZP;

@@ -121,3 +121,42 @@ def test_turned_quadrilateral_vs_oracle(gb, p1, p2):
     Ao, ro = _oracle_system(m, F, p, D)
     for mode in (gb.DG_FACE_FP64, gb.DG_FACE_DWORD):
         _check(*_system(gb, m, F, p, D, mode), Ao, ro)
+
+
+@pytest.mark.parametrize("p", [1, 2, 3, 4])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_a_coefficient_that_is_not_finite_shows(gb, p, bad):
+    """One prism's coefficient NaN or infinite: nothing finite is left in its
+    own block, its neighbours' blocks with it and, on the boundary, its load; all else
+    is what it is beside a prism of coefficient 1."""
+    from modfem_gb300.mesh import prism_faces, structured_prism_mesh
+    m = structured_prism_mesh(3, jitter=0.2, seed=p)
+    F = prism_faces(m)
+
+    def system(e, k):
+        c = gb.Context(0)
+        c.set_mesh(m)
+        kk = np.ones(m.nel)
+        kk[e] = k
+        c.set_coefficients(k=kk, f=1.0, g=0.4)
+        c.dg_set_degrees(np.full(m.nel, p))
+        c.dg_set_faces(F, penalty=10.0)
+        c.dg_build_structure()
+        c.dg_assemble()
+        out = [np.array(a) for a in c.dg_get_matrix()], c.dg_get_structure()
+        c.close()
+        return out
+
+    inner = int(np.flatnonzero(~np.isin(np.arange(m.nel), F.el1[F.el2 < 0]))[0])
+    for e, boundary in ((inner, False), (int(F.el1[F.el2 < 0][0]), True)):
+        (v1, r1), (off, bptr, bcol, boff) = system(e, 1.0)
+        (v, r), _ = system(e, bad)
+        for i in range(m.nel):
+            assert np.array_equal(r[off[i]:off[i + 1]], r1[off[i]:off[i + 1]]) or (i == e and boundary)
+            for b in range(bptr[i], bptr[i + 1]):
+                x, x1 = v[boff[b]:boff[b + 1]], v1[boff[b]:boff[b + 1]]
+                if e in (i, bcol[b]):
+                    assert not np.any(np.isfinite(x)), (i, bcol[b])
+                else:
+                    assert np.array_equal(x, x1)
+        assert not boundary or not np.any(np.isfinite(r[off[e]:off[e + 1]]))
