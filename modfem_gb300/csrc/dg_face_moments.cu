@@ -300,9 +300,10 @@ __device__ __forceinline__ double flip(double v, int neg) {  // the sign on the 
 }
 
 // (NaN or infinity, on the integer side.)  Where a derivative of a function is
-// identically zero its moment is left out, and a field that is not finite, as a
-// coefficient that is not makes it, would leave no trace in the entry; the sums over the
-// points multiply it by zero, which is NaN.  So it is looked for.
+// identically zero, or the function on the face, its moment is left out, and a field
+// that is not finite (a coefficient that is not, a face without an area) would leave
+// no trace in the entry; the sums over the points multiply it by zero, which is NaN.
+// So it is looked for.
 __device__ __forceinline__ int fm_nonfinite(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
 
 // How a quadrilateral lies in one of its elements: triangle vertices A, B of
@@ -345,11 +346,12 @@ __global__ void __launch_bounds__(THR) dg_face_diag_kernel(
   __shared__ double sM[D::NM];
   __shared__ double sC[9];              // the doubles -4 .. 4
   __shared__ DgFaceRec sR[5];
-  __shared__ int sOwn[5], sQuad[3], sTri[2];
+  __shared__ int sOwn[5], sQuad[3], sTri[2], sBad;
   const int tid = threadIdx.x, e = ent_el[blockIdx.x];
   const int h0 = hf_ptr[e], nf = hf_ptr[e + 1] - h0;
   if (nf == 0) return;
   if (tid < 9) sC[tid] = (double)(tid - 4);
+  if (tid == 0) sBad = 0;
   if (tid < nf) {
     const int h = hrec[h0 + tid];
     sR[tid] = rec[h >> 1];
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(THR) dg_face_diag_kernel(
     for (; t < 2; t++) sTri[t] = -1;
   }
   // fields of the owner's side with its sign
-  int bad = 0;  // of a Dirichlet face
+  int bad = 0;  // 1: a field of any face is not finite, 3: of a Dirichlet face
   for (int f = 0; f < nf; f++) {
     const DgFaceRec &R = sR[f];
     const int pm = R.el2 >= 0 && R.p2 > R.p1 ? R.p2 : R.p1;
@@ -378,10 +380,12 @@ __global__ void __launch_bounds__(THR) dg_face_diag_kernel(
       const int c = t / nq, q = t - c * nq;
       const double v = g[(size_t)(c == 0 ? 0 : c + 3 * o) * nq + q];
       sF[f][t] = c == 0 ? v : flip(v, o);
-      bad |= R.el2 < 0 && fm_nonfinite(v);
+      if (fm_nonfinite(v)) bad |= R.el2 < 0 ? 3 : 1;
     }
   }
-  bad = __syncthreads_or(bad);
+  if (bad) atomicOr(&sBad, bad);
+  __syncthreads();
+  bad = sBad;
   for (int t = tid; t < 3 * NZ; t += THR) {
     const int qi = t / NZ, f = sQuad[qi];
     if (f < 0) break;  // (the quadrilaterals come first)
@@ -496,7 +500,7 @@ __global__ void __launch_bounds__(THR) dg_face_diag_kernel(
     }
     if (any) {
       double *r = rhs + roff[e] + i;
-      *r = bad ? nan("") : fma(gval, s, *r);
+      *r = bad & 2 ? nan("") : fma(gval, s, *r);
     }
   }
   __syncthreads();
@@ -504,7 +508,7 @@ __global__ void __launch_bounds__(THR) dg_face_diag_kernel(
   double *blk = val + boff_diag[e];
   for (int t = tid; t < NS * (NS + 1) / 2; t += THR) {
     const DgFaceEntry E = tb.ENT[P][t];
-    const double S = sM[E.off[0]];
+    const double S = bad ? nan("") : sM[E.off[0]];
     const double N = fma(sC[E.coef[0]], sM[E.off[1]], fma(sC[E.coef[1]], sM[E.off[2]], sC[E.coef[2]] * sM[E.off[3]]));
     double *lo = blk + E.w + NS * E.u, *up = blk + E.u + NS * E.w;
     if (lo == up) {

@@ -160,3 +160,33 @@ def test_a_coefficient_that_is_not_finite_shows(gb, p, bad):
                 else:
                     assert np.array_equal(x, x1)
         assert not boundary or not np.any(np.isfinite(r[off[e]:off[e + 1]]))
+
+
+@pytest.mark.parametrize("p", [1, 2, 3, 4])
+def test_a_face_without_a_normal_shows(gb, p):
+    """A corner of the mesh moved onto another vertex of its boundary triangle (no
+    area, no normal; the element itself keeps a volume): nothing finite in
+    that element's own block and load, as from the sums over the points."""
+    from modfem_gb300.mesh import prism_faces, structured_prism_mesh
+    m = structured_prism_mesh(3)
+    F = prism_faces(m)
+    m.coords = m.coords.copy()
+    m.coords[1] = m.coords[0]
+    c = gb.Context(0)
+    c.set_mesh(m)
+    c.set_coefficients(k=np.ones(m.nel), f=1.0, g=0.4)
+    c.dg_set_degrees(np.full(m.nel, p))
+    c.dg_set_faces(F, penalty=10.0)
+    c.dg_build_structure()
+    c.dg_assemble()
+    v, r = c.dg_get_matrix()
+    off, bptr, bcol, boff = c.dg_get_structure()
+    c.close()
+    flat = [f for f in range(F.n) if F.type[f] == 3 and {0, 1} <= set(F.nodes[f, :3].tolist())]
+    assert len(flat) == 1 and F.el2[flat[0]] < 0
+    e = int(F.el1[flat[0]])
+    d = bptr[e] + int(np.flatnonzero(bcol[bptr[e]:bptr[e + 1]] == e)[0])
+    assert not np.any(np.isfinite(v[boff[d]:boff[d + 1]])) and not np.any(np.isfinite(r[off[e]:off[e + 1]]))
+    others = np.ones(len(v), bool)
+    others[boff[bptr[e]]:boff[bptr[e + 1]]] = False
+    assert np.all(np.isfinite(v[others]))
