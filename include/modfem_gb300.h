@@ -41,7 +41,7 @@ typedef struct gbfem_ctx_s *gbfem_ctx;
 #define GBFEM_SCATTER_ATOMIC 0 /* one launch, FP64 atomics (summation order varies) */
 #define GBFEM_SCATTER_COLOR 1  /* one launch per colour, plain adds (deterministic); tetrahedra: local
                                   matrices stored and summed a row, as GATHER does for prisms, which
-                                  takes 180 B of device memory an element beside the structure */
+                                  takes 176 B of device memory an element beside the structure */
 #define GBFEM_SCATTER_GATHER 2 /* local matrices stored, then a group of lanes a row sums them over
                                   the incident elements in element order (deterministic, no
                                   colouring; std prisms, FP64 element arithmetic) */

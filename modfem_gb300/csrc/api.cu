@@ -1133,9 +1133,11 @@ int gbfem_assemble(gbfem_ctx c, int scatter_mode) {
   const bool gather = scatter_mode == GBFEM_SCATTER_GATHER || (!atomic && c->nv == GBFEM_TETRA);
   if (!atomic && !c->have_inc && (gather || c->el_colour_pending)) {
     GB_TRY(gbfem::build_device_incidence(c->stream, c->nel, c->nv, c->el_table.p, c->ndof, c->inc_ptr, c->inc));
-    GB_TRY(c->fa_head.alloc(c->nel));
-    GB_TRY(c->fa_next.alloc(std::max(c->nfa, 1)));
-    GB_TRY(gbfem::launch_face_lists(c->stream, c->nel, c->nfa, c->fa_el.p, c->fa_head.p, c->fa_next.p));
+    if (c->nfa > 0) {  // (without faces the gather reads no lists)
+      GB_TRY(c->fa_head.alloc(c->nel));
+      GB_TRY(c->fa_next.alloc(c->nfa));
+      GB_TRY(gbfem::launch_face_lists(c->stream, c->nel, c->nfa, c->fa_el.p, c->fa_head.p, c->fa_next.p));
+    }
     c->have_inc = true;
   }
   if (!gather && scatter_mode == GBFEM_SCATTER_COLOR && c->el_colour_pending) {
@@ -1147,7 +1149,7 @@ int gbfem_assemble(gbfem_ctx c, int scatter_mode) {
   }
   if (gather) {
     GB_TRY(c->ek.alloc((size_t)c->nel * (c->nv * c->nv + c->nv)));
-    GB_TRY(c->fk.alloc((size_t)std::max(c->nfa, 1) * 14));
+    GB_TRY(c->fk.alloc((size_t)c->nfa * 14));
   }
   cudaEventRecord(c->ev0, c->stream);
   if (!gather) {
